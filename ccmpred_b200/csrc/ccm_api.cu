@@ -240,13 +240,14 @@ int ensure_configured(int device) {
 int alloc_tc(ccm_context *c) {
   const bool sp = c->path == CCM_PATH_TC_I8SP;
   if (sp) {
-    // sparse integer path: forward tiles are 192-slot groups (9 columns); the
-    // slot space is padded to the backward's 256-slot pair tiles; K of the
-    // forward is 21 L in the order l * 21 + q, padded to 256
+    // sparse integer path: forward tiles are 192-slot groups (9 columns); K of the
+    // forward is 21 L in the order l * 21 + q, padded to 256; the backward has 21 L + 1
+    // natural slots, padded to its 256-slot pair tiles
     c->T = Groups192::groups(c->L);
     c->SW = c->T * Groups192::kSlots;
     c->S = ((c->SW + 255) / 256) * 256;
     c->KP = ((kQ * c->L + 255) / 256) * 256;
+    c->SB = ((kQ * c->L + 1 + 255) / 256) * 256;
   } else {
     c->T = n_groups(c->L);
     c->S = c->T * kGroupSlots;
@@ -258,13 +259,22 @@ int alloc_tc(ccm_context *c) {
   if (i8) {
     // integer path: one-hot x1 / x128 bytes, three digit matrices of W and of R
     const size_t wbytes = sp ? (size_t)c->KP * c->SW : S * S;
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_o1, Np * S));
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_o128, Np * S));
     for (int i = 0; i < 3; ++i) {
       CCM_CUDA_TRY(dev_alloc(c, &c->d_wdig[i], wbytes));
       CCM_CUDA_TRY(cudaMemsetAsync(c->d_wdig[i], 0, wbytes, c->stream));
-      CCM_CUDA_TRY(dev_alloc(c, &c->d_rdig[i], Np * S));
-      CCM_CUDA_TRY(cudaMemsetAsync(c->d_rdig[i], 0, Np * S, c->stream));
+    }
+    if (sp) {
+      CCM_CUDA_TRY(dev_alloc(c, &c->d_onat, 2 * Np * c->SB));
+      CCM_CUDA_TRY(dev_alloc(c, &c->d_rnat, 3 * Np * c->SB));
+      // the forward writes real slots only
+      CCM_CUDA_TRY(cudaMemsetAsync(c->d_rnat, 0, 3 * Np * c->SB, c->stream));
+    } else {
+      CCM_CUDA_TRY(dev_alloc(c, &c->d_o1, Np * S));
+      CCM_CUDA_TRY(dev_alloc(c, &c->d_o128, Np * S));
+      for (int i = 0; i < 3; ++i) {
+        CCM_CUDA_TRY(dev_alloc(c, &c->d_rdig[i], Np * S));
+        CCM_CUDA_TRY(cudaMemsetAsync(c->d_rdig[i], 0, Np * S, c->stream));
+      }
     }
     if (sp) {
       CCM_CUDA_TRY(dev_alloc(c, &c->d_ac1, Np * c->KP / 2));
@@ -292,7 +302,7 @@ int alloc_tc(ccm_context *c) {
   std::vector<int2> tiles;
   // P and Q in 256-slot blocks (rows, columns of C); the symmetric gradient
   // needs only the tiles that hold some s1 <= s2
-  const int blocks = c->S / 256;
+  const int blocks = (sp ? c->SB : c->S) / 256;
   for (int Q = 0; Q < blocks; ++Q)
     for (int P = 0; P < blocks; ++P)
       if (c->gradient == CCM_GRADIENT_PARTIAL || P <= Q) tiles.push_back(make_int2(P, Q));
@@ -306,24 +316,24 @@ int alloc_tc(ccm_context *c) {
     CCM_CUDA_TRY(i8_build_onehot(c));
     std::memset(&c->i8fwd_maps, 0, sizeof(c->i8fwd_maps));
     std::memset(&c->i8bwd_maps, 0, sizeof(c->i8bwd_maps));
-    if ((rc = make_map_u8(&c->i8fwd_maps.a1, c->d_o1, Np, S, 64, 128)) != CCM_OK) return rc;
-    if ((rc = make_map_u8(&c->i8fwd_maps.a128, c->d_o128, Np, S, 64, 128)) != CCM_OK) return rc;
-    // backward operands: the dense path reads 128-slot x 32-row boxes of the
-    // row-major matrices (128-byte swizzle); the sparse path stores them tiled
-    // (4 KB shared-memory images, swizzle applied) and reads 16 rows of 256 bytes
-    const long long trows = (long long)Np * S / 256;
     const int none = CU_TENSOR_MAP_SWIZZLE_NONE;
-    auto bwd_map = [&](CUtensorMap *m, void *p) {
-      return sp ? make_map_u8(m, p, trows, 256, 256, 16, none) : make_map_u8(m, p, Np, S, 128, 32);
-    };
-    if ((rc = bwd_map(&c->i8bwd_maps.o1, c->d_o1)) != CCM_OK) return rc;
-    if ((rc = bwd_map(&c->i8bwd_maps.o128, c->d_o128)) != CCM_OK) return rc;
-    for (int i = 0; i < 3; ++i) {
-      if (!sp && (rc = make_map_u8(&c->i8fwd_maps.b[i], c->d_wdig[i], S, S, 128, 64)) != CCM_OK)
+    if (!sp) {
+      if ((rc = make_map_u8(&c->i8fwd_maps.a1, c->d_o1, Np, S, 64, 128)) != CCM_OK) return rc;
+      if ((rc = make_map_u8(&c->i8fwd_maps.a128, c->d_o128, Np, S, 64, 128)) != CCM_OK) return rc;
+      // backward operands: 128-slot x 32-row boxes of the row-major matrices
+      if ((rc = make_map_u8(&c->i8bwd_maps.o1, c->d_o1, Np, S, 128, 32)) != CCM_OK) return rc;
+      if ((rc = make_map_u8(&c->i8bwd_maps.o128, c->d_o128, Np, S, 128, 32)) != CCM_OK) return rc;
+      for (int i = 0; i < 3; ++i) {
+        if ((rc = make_map_u8(&c->i8fwd_maps.b[i], c->d_wdig[i], S, S, 128, 64)) != CCM_OK) return rc;
+        if ((rc = make_map_u8(&c->i8bwd_maps.r[i], c->d_rdig[i], Np, S, 128, 32)) != CCM_OK) return rc;
+      }
+    } else {
+      // tiled shared-memory images viewed as rows of 256 bytes: 32 rows for the two
+      // one-hot tiles of a stage's side, 48 for the three digit tiles
+      const long long trows = (long long)Np * c->SB / 256;
+      if ((rc = make_map_u8(&c->i8bwd_maps.o1, c->d_onat, 2 * trows, 256, 256, 32, none)) != CCM_OK ||
+          (rc = make_map_u8(&c->i8bwd_maps.r[0], c->d_rnat, 3 * trows, 256, 256, 48, none)) != CCM_OK)
         return rc;
-      if ((rc = bwd_map(&c->i8bwd_maps.r[i], c->d_rdig[i])) != CCM_OK) return rc;
-    }
-    if (sp) {
       std::memset(&c->i8sp_maps, 0, sizeof(c->i8sp_maps));
       // tiled operand storage viewed as rows of 256 bytes; one box = one stage tile
       const long long KP = c->KP;
@@ -372,6 +382,7 @@ void free_all(ccm_context *c) {
   f(c->d_msa); f(c->d_w); f(c->d_out); f(c->d_onehot);
   for (int i = 0; i < 3; ++i) { f(c->d_wperm[i]); f(c->d_r[i]); f(c->d_wdig[i]); f(c->d_rdig[i]); }
   f(c->d_o1); f(c->d_o128); f(c->d_colmax); f(c->d_ac1); f(c->d_ac128); f(c->d_meta);
+  f(c->d_onat); f(c->d_rnat);
   f(c->d_part_f); f(c->d_part_reg); f(c->d_fin_part); f(c->d_fin_done); f(c->d_g1d); f(c->d_bwd_tiles);
   f(c->d_simt_pc); f(c->d_simt_g2); f(c->d_simt_part); f(c->d_simt_g1);
   f(c->d_xh); f(c->d_gh);
@@ -855,6 +866,20 @@ long long ccm_debug_copy(ccm_context *c, int which, void *dst, long long bytes) 
     // path: W digits are KP x SW, 9 compressed one-hot x1 (Npad x KP/2),
     // 10 its metadata (Npad x KP/8)
     const bool sp = c->path == CCM_PATH_TC_I8SP;
+    if (sp && (which == 0 || (which >= 4 && which <= 6))) {
+      // kept in the backward's natural storage: handed out as Npad x S bytes of the
+      // forward's slot groups
+      size = (long long)c->Npad * slots;
+      if (!dst) return size;
+      if (bytes < size) return set_error(CCM_ERR_INVALID, "ccm_debug_copy: need %lld bytes", size);
+      const int mats = which == 0 ? 2 : 3, mat = which == 0 ? 0 : which - 4;
+      std::vector<uint8_t> nat((size_t)mats * c->Npad * c->SB);
+      CCM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+      CCM_CUDA_TRY(cudaMemcpy(nat.data(), which == 0 ? c->d_onat : c->d_rnat, nat.size(),
+                              cudaMemcpyDeviceToHost));
+      i8nat_to_groups(c, nat.data(), mats, mat, static_cast<uint8_t *>(dst));
+      return CCM_OK;
+    }
     if (which == 0) { src = c->d_o1; size = (long long)c->Npad * slots; }
     else if (which >= 1 && which <= 3) {
       src = c->d_wdig[which - 1];

@@ -51,8 +51,12 @@ struct I8FwdMaps {
 };
 
 struct I8BwdMaps {
-  CUtensorMap o1, o128;  // one-hot O x1 / x128 [Npad][S] u8, box 128 (slots) x 32 (rows), 128B swizzle
-  CUtensorMap r[3];      // digits of R [Npad][S] s8, same box
+  // dense path: one-hot x1 / x128 [Npad][S] u8, box 128 (slots) x 32 (rows), 128B swizzle;
+  // sparse path: o1 alone, the tiles x1 | x128 of natural slots, box 256 x 32 bytes
+  CUtensorMap o1, o128;
+  // dense path: R_i [Npad][S] s8, box as the one-hot; sparse path: r[0] alone, the tiles
+  // of the three digits, box 256 x 48 bytes
+  CUtensorMap r[3];
 };
 
 // Sparse integer forward (CCM_PATH_TC_I8SP): compressed one-hot A and its
@@ -84,6 +88,7 @@ struct I8FwdArgs {
   const float *x1;
   const uint32_t *colmax;
   int8_t *r[3];
+  uint8_t *rnat;  // sparse path: digits of R in the backward's natural storage
   double *part_f;
   int *status;
   int L, N, S, T, Npad, m_tiles;
@@ -182,6 +187,7 @@ cudaError_t i8_configure_kernels();
 cudaError_t i8_forward_max_pairs(int *pairs);
 cudaError_t i8_backward_max_pairs(int *pairs);
 cudaError_t i8_build_onehot(ccm_context *c);
+void i8nat_to_groups(const ccm_context *c, const uint8_t *nat, int mats, int mat, uint8_t *dst);
 cudaError_t i8sp_forward_max_pairs(int *pairs);
 // tc_finalize over the loss partials of n_fwd_tiles 128-row forward tiles.
 cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles);
@@ -296,6 +302,10 @@ struct ccm_context {
   // sparse integer forward: W digits are KP x SW (K rows l * 21 + q, 192-slot
   // groups as columns); compressed one-hot Npad x KP/2 and metadata Npad x KP/8
   int KP = 0, SW = 0;
+  // its backward: SB natural slots q L + l (ones slot 21 L, padded to 256); one-hot
+  // x1 | x128 (2 x Npad x SB bytes) and digits of R (3 x Npad x SB), tiled
+  int SB = 0;
+  uint8_t *d_onat = nullptr, *d_rnat = nullptr;
   uint8_t *d_ac1 = nullptr, *d_ac128 = nullptr, *d_meta = nullptr;
   ccm::I8SpMaps i8sp_maps;
 

@@ -218,6 +218,36 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
   return r != 0;
 }
 
+// Add v to *p if pred: a predicated reduction, without a branch (a branch per add
+// costs a reconvergence, ~40 cycles of a warp's issue).
+__device__ __forceinline__ void red_add_if(float *p, float v, bool pred) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %2, 0;\n\t"
+      "@p red.global.add.f32 [%0], %1;\n\t}\n" ::"l"(p),
+      "f"(v), "r"((uint32_t)pred)
+      : "memory");
+}
+
+// Four consecutive adds; p is 16-byte aligned.
+__device__ __forceinline__ void red_add4_if(float *p, float4 v, bool pred) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %5, 0;\n\t"
+      "@p red.global.add.v4.f32 [%0], {%1,%2,%3,%4};\n\t}\n" ::"l"(p),
+      "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((uint32_t)pred)
+      : "memory");
+}
+
+// Register split between the warpgroups of a block (all four warps of a warpgroup
+// execute one of these; the shares must add up to at most the launch's total).
+template <int R> __device__ __forceinline__ void reg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R> __device__ __forceinline__ void reg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+
 // 32-byte global store (one full sector); `p` must be 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(void *p, const uint32_t (&r)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]),
@@ -407,6 +437,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+
+// 32 lanes x 4 columns of 32-bit.
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
 }
 
 __device__ __forceinline__ void tmem_wait_st() {

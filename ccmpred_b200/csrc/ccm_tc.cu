@@ -16,6 +16,7 @@
 // line-by-line restatement used as the checker).
 #include <cuda_bf16.h>
 
+#include "ccm_bwd_out.cuh"
 #include "ccm_internal.cuh"
 #include "ccm_layout.cuh"
 #include "ccm_ptx.cuh"
@@ -522,7 +523,6 @@ constexpr int kBwdBufs = 512 / kBwdBN;  // TMEM accumulators of kBwdBN columns
 constexpr int kBwdChunkKB = 40;
 // warp 0 TMA, warp 1 MMA (leader CTA), warps 2-9 epilogue (two warps per TMEM
 // lane quarter, one per half of the 256 columns)
-constexpr int kBwdThreads = 320;
 
 template <int NSPLIT>
 struct BwdSmem {
@@ -538,7 +538,7 @@ struct BwdSmem {
   static constexpr int kStage = kOffRQ + NSPLIT * kB;
   static constexpr int kBarOff = kStages * kStage;
   static constexpr int kTOff = kBarOff + 256;                    // epilogue transpose buffers
-  static constexpr int kTBytes = 8 * 32 * 9 * 4;                 // 8 warps x 32 rows x 8(+1) cols
+  static constexpr int kTBytes = 8 * kBwdOutWarpBytes;
   static constexpr int kTotal = kTOff + kTBytes + 1024;
 };
 
@@ -547,7 +547,7 @@ struct BwdSmem {
 // G = O^T R on all tiles, written directly only, self blocks included (the
 // true partial derivatives, for gradient checks and autograd).
 template <int NSPLIT, bool SYM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBwdThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     tc_backward_kernel(const __grid_constant__ BwdMaps maps, BwdArgs args) {
   using SM = BwdSmem<NSPLIT>;
   constexpr int kStages = SM::kStages;
@@ -585,6 +585,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBwdThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (warp < 4) reg_dec<kWgRegsLoad>();
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;
@@ -690,23 +691,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBwdThreads, 1)
       umma_commit_pair(drain, 0x1);
       if (!mbar_wait(drain, 0)) record_error(args.status, kErrBwdTimeout, abort_flag);
     }
-  } else {
+  } else if (warp >= 4) {
+    reg_inc<kWgRegsEpi>();
     // Epilogue.  Each thread owns one row s1 of the tile (TMEM lane) and one
     // half of its 256 columns; it sums the tile's K chunks in FP32 registers,
-    // then writes every element (s1, s2), s1 <= s2, of the symmetric C to
-    //   direct      g2 row (b,k) = s1, column (a,j) = s2
-    //   transposed  g2 row (a,j) = s2, column (b,k) = s1   (s1 != s2)
-    // (SYM = false: direct only, all elements).  Transposed writes are issued
-    // thread-major (consecutive lanes = consecutive k: contiguous runs); direct
-    // writes go through a per-warp shared-memory transpose so that one warp
-    // instruction covers 4 rows x 8 columns (runs of consecutive j).  g2 already
-    // holds the regulariser term (tc_prep) and every element receives exactly one
-    // atomic add, so the result does not depend on the order of the adds.
+    // then adds them to the gradient (bwd_output).
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int L = args.L;
-    float *__restrict__ g2 = args.g2;
-    float *Tb = reinterpret_cast<float *>(smem + SM::kTOff) + (warp - 2) * 32 * 9;
+    const int half = (warp - 4) >> 2;
+    float *Tb = reinterpret_cast<float *>(smem + SM::kTOff + (warp - 4) * kBwdOutWarpBytes);
     uint32_t chunk = 0;
     bool ok = true;
     for (int tile = pair; tile < n_tiles && ok; tile += npairs) {
@@ -741,62 +733,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBwdThreads, 1)
       if (!ok) break;
 
       const int2 pq = args.tiles[tile];
-      const int rowbase = pq.x * kBwdPairM + (int)rank * kBwdBM + q * 32;
-      const int s1 = rowbase + lane;
-      const int t1 = s1 / kGroupSlots, r1 = s1 % kGroupSlots;
-      const int b = r1 / kGroupCols, k = t1 * kGroupCols + r1 % kGroupCols;
-      const bool valid1 = r1 < kGroupUsed && k < L;
-      const long long colt = (long long)b * L + k;  // transposed: + ((a*L+j)*32)*L
-      // columns: Q block pq.y of kBwdBN slots, inside slot group tQ from slot rQ
-      const int tQ = pq.y * kBwdBN / kGroupSlots;
-      const int rQ = pq.y * kBwdBN % kGroupSlots + half * kBwdHalfN;
-      const int sQ = tQ * kGroupSlots + rQ;
-      // 8 rounds of 8 columns through the transpose buffer Tb[row][col]
-#pragma unroll
-      for (int cb = 0; cb < kBwdHalfN / 8; ++cb) {
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) Tb[lane * 9 + e] = accv[cb * 8 + e];
-        __syncwarp();
-        // (A) transposed writes and the ones-slot column: thread = row s1
-        if (SYM) {
-#pragma unroll 1
-          for (int col = 0; col < 8; ++col) {
-            const int r2 = rQ + cb * 8 + col;
-            const int s2 = sQ + cb * 8 + col;
-            const int a = r2 / kGroupCols, j = tQ * kGroupCols + r2 % kGroupCols;
-            const bool valid2 = r2 < kGroupUsed && j < L;
-            if (s1 < s2) {
-              const float val = Tb[lane * 9 + col];
-              if (valid1 && valid2) {
-                if (k != j) atomicAdd(g2 + ((long long)a * L + j) * kQPad * L + colt, val);
-              } else if (s2 == kOnesSlot && valid1 && b < kQ - 1) {
-                args.g1d[b * L + k] = val;
-              }
-            }
-          }
-        }
-        // (B) direct writes and the ones-slot row: lanes = 4 rows x 8 columns
-        const int col = lane & 7;
-        const int r2 = rQ + cb * 8 + col;
-        const int s2 = sQ + cb * 8 + col;
-        const int a = r2 / kGroupCols, j = tQ * kGroupCols + r2 % kGroupCols;
-        const bool valid2 = r2 < kGroupUsed && j < L;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int row = 4 * it + (lane >> 3);
-          const int s1r = rowbase + row;
-          if (SYM && s1r > s2) continue;
-          const float val = Tb[row * 9 + col];
-          const int tr = s1r / kGroupSlots, rr = s1r % kGroupSlots;
-          const int br = rr / kGroupCols, kr = tr * kGroupCols + rr % kGroupCols;
-          if (rr < kGroupUsed && kr < L) {
-            if (valid2 && (!SYM || kr != j)) atomicAdd(g2 + x2_index(br, kr, a, j, L), val);
-          } else if (s1r == kOnesSlot && valid2 && a < kQ - 1) {
-            args.g1d[a * L + j] = val;
-          }
-        }
-      }
+      bwd_output<Groups256, SYM>(accv, Tb, args.g2, args.g1d, args.L, lane,
+                                 pq.x * kBwdPairM + (int)rank * kBwdBM + q * 32,
+                                 pq.y * kBwdBN + half * kBwdHalfN);
     }
   }
 
@@ -913,10 +852,10 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   const int bwd_pairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
   if (c->gradient == CCM_GRADIENT_PARTIAL)
     tc_backward_kernel<NSPLIT, false>
-        <<<2 * bwd_pairs, kBwdThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
+        <<<2 * bwd_pairs, kWgThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
   else
     tc_backward_kernel<NSPLIT, true>
-        <<<2 * bwd_pairs, kBwdThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
+        <<<2 * bwd_pairs, kWgThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
   prof_mark(c);
 
   launch_tc_finalize(c, x1, d_g, fwd_tiles);
@@ -938,7 +877,7 @@ cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long
 cudaError_t tc_backward_max_pairs(int nsplit, int *pairs) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2, 1, 1);
-  cfg.blockDim = dim3(kBwdThreads, 1, 1);
+  cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = nsplit == 3 ? BwdSmem<3>::kTotal : BwdSmem<2>::kTotal;
   int n = 0;
   cudaError_t e = nsplit == 3

@@ -19,9 +19,11 @@
 // One evaluation = colmax (+ the fused CG step), prep (digits of W, g2 <- 2 l2 x,
 // sum x^2), forward, backward, finalize (shared with ccm_tc.cu).
 #include <cmath>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
+#include "ccm_bwd_out.cuh"
 #include "ccm_internal.cuh"
 #include "ccm_layout.cuh"
 #include "ccm_ptx.cuh"
@@ -262,46 +264,85 @@ __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ 
   }
 }
 
-// Tiled storage of the backward's operands on the sparse path (one-hot x1 /
-// x128 and the digits of R, Npad x S bytes each): the 32-row x 128-slot tile
-// (kb = n / 32, sb = s / 128) that one pipeline stage of one CTA reads is stored
-// contiguously (4 KB) as the shared-memory image the MMA reads -- rows of 128
-// slots, 16-byte chunk c of row r at chunk c ^ (r & 7) (128-byte swizzle) --
-// tiles in the order sb * KB + kb, KB = Npad / 32.  One TMA box of 16 rows of
-// 256 bytes moves a tile (twice the bytes per TMA row request of a 128-slot box
-// of the row-major matrix).
-__host__ __device__ constexpr long long i8_bwd_tile_offset(int n, int s, int KB) {
-  return ((long long)(s >> 7) * KB + (n >> 5)) * 4096 + (n & 31) * 128 +
-         (((((s & 127) >> 4) ^ (n & 7)) & 7) << 4) + (s & 15);
+// Backward operands of the sparse path.  Slots in natural order, s = q L + l (the
+// row and column index of the coupling matrix itself), the ones slot at 21 L, padded
+// to SB = a multiple of 256; rows n of the alignment are the contraction index and
+// lie contiguous (K-major).  The 128-slot x 32-row tile (sb = s / 128, kb = n / 32)
+// that one pipeline stage of one CTA reads is stored as the shared-memory image the
+// MMA reads, 32 bytes per slot with the 32-byte swizzle (16-byte half h of slot r
+// stored at half h ^ ((r >> 2) & 1)); the matrices that a stage needs side by side
+// follow one another, so that one TMA box of 256-byte rows moves them:
+//   one-hot  x1 | x128      8 KB at (sb * KB + kb) * 8192,  KB = Npad / 32
+//   digits   r0 | r1 | r2  12 KB at (sb * KB + kb) * 12288
+// Natural slots make a tile's rows and columns contiguous runs of the gradient (see
+// the output phase), K-major tiles let a warp of the forward's epilogue, whose lanes
+// are 32 consecutive rows n, write one full 32-byte sector per slot and digit for
+// any order of the slots.
+constexpr int kNatTile = 128 * 32;
+__host__ __device__ constexpr long long i8nat_offset(int n, int s, int KB, int mats) {
+  return ((long long)(s >> 7) * KB + (n >> 5)) * (mats * kNatTile) + (s & 127) * 32 +
+         ((n & 31) ^ ((s & 4) << 2));
 }
 
-// One-hot operands of the integer path (slot groups G): O1[n][s] = 1 and
-// O128[n][s] = 128 where the state of column l(s) in row n is q(s), and in the
-// ones slot of every real row; 0 elsewhere.  TILED: stored as i8_bwd_tile_offset.
-template <class G, bool TILED>
+// x1 | x128 one-hot of the backward: 1 / 128 where column l of row n holds state q,
+// and in the ones slot of every real row.  One thread per (slot, 32 rows):
+// consecutive threads read consecutive bytes of the alignment.
+__global__ void __launch_bounds__(128) i8nat_onehot_kernel(const uint8_t *__restrict__ msa,
+                                                           uint8_t *__restrict__ o, int L, int N,
+                                                           int KB) {
+  const int s = blockIdx.y * 128 + threadIdx.x, kb = blockIdx.x;
+  const int q = s / L, l = s % L;
+  uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const int n = kb * 32 + i;
+    bool one = false;
+    if (n < N) one = s == kQ * L || (s < kQ * L && msa[(long long)n * L + l] == q);
+    v[i >> 2] |= (one ? 1u : 0u) << (8 * (i & 3));
+  }
+  uint4 *p = reinterpret_cast<uint4 *>(o + i8nat_offset(kb * 32, s, KB, 2) - ((s & 4) << 2));
+  const int h = (s >> 2) & 1;
+  p[h] = make_uint4(v[0], v[1], v[2], v[3]);
+  p[h ^ 1] = make_uint4(v[4], v[5], v[6], v[7]);
+  p += kNatTile / 16;
+  p[h] = make_uint4(v[0] << 7, v[1] << 7, v[2] << 7, v[3] << 7);
+  p[h ^ 1] = make_uint4(v[4] << 7, v[5] << 7, v[6] << 7, v[7] << 7);
+}
+
+// One-hot operands of the dense integer path: O1[n][s] = 1 and O128[n][s] = 128 where
+// the state of column l(s) in row n is q(s), and in the ones slot of every real row;
+// 0 elsewhere.
 __global__ void i8_onehot_kernel(const uint8_t *__restrict__ msa, uint8_t *__restrict__ o1,
                                  uint8_t *__restrict__ o128, int L, int N, int S, int Npad) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)Npad * S) return;
   const int n = (int)(idx / S), s = (int)(idx % S);
-  const long long at = TILED ? i8_bwd_tile_offset(n, s, Npad >> 5) : idx;
-  const int t = s / G::kSlots, r = s % G::kSlots;
+  const int t = s / kGroupSlots, r = s % kGroupSlots;
   bool one = false;
   if (n < N) {
-    if (s == G::kOnes) {
+    if (s == kOnesSlot) {
       one = true;
-    } else if (r < G::kUsed) {
-      const int q = r / G::kCols, l = t * G::kCols + r % G::kCols;
+    } else if (r < kGroupUsed) {
+      const int q = r / kGroupCols, l = t * kGroupCols + r % kGroupCols;
       one = l < L && msa[(long long)n * L + l] == q;
     }
   }
-  o1[at] = one ? 1 : 0;
-  o128[at] = one ? 128 : 0;
+  o1[idx] = one ? 1 : 0;
+  o128[idx] = one ? 128 : 0;
 }
 
 }  // namespace ccm
 
 namespace ccm {
+
+// hi * 2^14 + lo rounded once to float, for |hi + (lo >> 14)| < 2^24 (the forward: at
+// most 129 L; the backward: |hi| <= 2^23, lo >> 14 < 2^17): the low 14 bits of lo and
+// the rest, carried into hi, are both exact floats, so the one rounding is the FMA's.
+// The same float as a conversion of the 64-bit sum, which runs at a quarter of the rate.
+__device__ __forceinline__ float i8_merge_exact(uint32_t hi, uint32_t lo) {
+  const int h = (int)hi + ((int)lo >> 14);
+  return fmaf(__int2float_rn(h), 16384.0f, __int2float_rn((int)(lo & 16383u)));
+}
 
 // ---------------------------------------------------------------- forward
 // Pair tiles of 256 rows x 256 slots as in tc_forward.  Per tile the MMAs run in
@@ -339,13 +380,6 @@ struct I8FwdSmem {
 //          M = max(m, m'), S = s exp(m - M) + s' exp(m' - M) (same order in both
 //          halves), lse = M + log S;
 //   C:     P = e * exp(m - M) / S, R = w (P - onehot) as its three digits.
-// G: the slot groups of the tile (one group = one tile, G::kSlots columns, half
-// of them per warp).  REGS: the merged logits leave both accumulators during the
-// merge -- the half's first 32-column chunk into a TMEM stash that no MMA writes
-// (t_stash), the other chunks into registers -- and the arrival on `lo_bar` after
-// the merge then releases both accumulators, so that the next tile's MMAs run
-// during passes B and C.  TILED: the digits of R go to the backward's tiled
-// storage (i8_bwd_tile_offset) instead of row-major Npad x S.
 // hi * 2^14 + lo, rounded once to float.  A row of the one-hot operand holds L
 // ones, so |hi| <= 128 L and 0 <= lo <= 16383 L: with L <= kI8NarrowMaxL the exact
 // sum lies in [-2^31, 2^31) and the 32-bit conversion (NARROW) gives the float the
@@ -360,15 +394,13 @@ __device__ __forceinline__ float i8_merge_digits(uint32_t hi, uint32_t lo) {
   }
 }
 
-template <class G, int H, bool REGS = false, bool TILED = false, bool NARROW = false>
+template <int H, bool NARROW>
 __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint32_t t_hi,
                                                      uint32_t t_lo, const float *tab_scale,
                                                      const float *tab_v, float *xbuf, int q,
                                                      int lane, int n, int t, long long part,
-                                                     uint32_t lo_bar, uint32_t t_stash = 0) {
-  constexpr int kGroupCols = G::kCols, kGroupUsed = G::kUsed;
-  constexpr int kChunks = G::kSlots / 64;  // 32-column chunks per half
-  uint32_t zr[REGS ? (kChunks - 1) * 32 : 1];  // REGS: chunks 1.. of the half
+                                                     uint32_t lo_bar) {
+  constexpr int kChunks = kGroupSlots / 64;  // 32-column chunks per half
   const int L = args.L;
   const int j0 = t * kGroupCols;
   const bool live = n < args.N;
@@ -385,34 +417,8 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
 #pragma unroll
   for (int jj = 0; jj < kGroupCols; ++jj) { mx[jj] = -INFINITY; tg[jj] = 0.0f; se[jj] = 0.0f; }
   // merge + maxima
-  if constexpr (REGS) {
-    // 16-column steps: steps 0 and 1 fill the stash, the others the registers
-    uint32_t st[32];
 #pragma unroll
-    for (int c = 0; c < 2 * kChunks; ++c) {
-      const int cc = 2 * kChunks * H + c;
-      uint32_t vh[16], vl[16];
-      __syncwarp();
-      tmem_ld16(t_hi + cc * 16, vh);
-      tmem_ld16(t_lo + cc * 16, vl);
-      tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int col = cc * 16 + i;
-        const float z = fmaf(i8_merge_digits<NARROW>(vh[i], vl[i]), tab_scale[col], tab_v[col]);
-        if (c < 2) st[c * 16 + i] = __float_as_uint(z);
-        else zr[(c - 2) * 16 + i] = __float_as_uint(z);
-        if (col < kGroupUsed) {
-          const int a = col / kGroupCols, jj = col % kGroupCols;
-          mx[jj] = fmaxf(mx[jj], z);
-          if (xr[jj] == a) tg[jj] = z;
-        }
-      }
-      if (c == 1) tmem_st32(t_stash, st);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < (REGS ? 0 : kChunks); ++c) {
+  for (int c = 0; c < kChunks; ++c) {
     const int cc = kChunks * H + c;
     uint32_t vh[32], vl[32];
     __syncwarp();
@@ -435,30 +441,15 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
   tmem_wait_st();
   tc_fence_before();
   __syncwarp();
-  // the next tile's low phase (REGS: its MMAs) may start
+  // the next tile's low phase may start
   if (lane == 0) mbar_arrive_cluster(lo_bar);
   // B: e = exp(z - m), sum
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int cc = kChunks * H + c;
-    if constexpr (REGS) {
-      if (c > 0) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int col = cc * 32 + i;
-          if (col < kGroupUsed) {
-            const int jj = col % kGroupCols;
-            const float e = expf(__uint_as_float(zr[(c - 1) * 32 + i]) - mx[jj]);
-            se[jj] += e;
-            zr[(c - 1) * 32 + i] = __float_as_uint(e);
-          }
-        }
-        continue;
-      }
-    }
     uint32_t v[32];
     __syncwarp();
-    tmem_ld32(REGS ? t_stash : t_hi + cc * 32, v);
+    tmem_ld32(t_hi + cc * 32, v);
     tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -470,7 +461,7 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
         v[i] = __float_as_uint(e);
       }
     }
-    tmem_st32(REGS ? t_stash : t_hi + cc * 32, v);
+    tmem_st32(t_hi + cc * 32, v);
   }
   float *mine = xbuf + (H * kI8BM + row) * (2 * kGroupCols);
   const float *other = xbuf + ((1 - H) * kI8BM + row) * (2 * kGroupCols);
@@ -492,25 +483,19 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
     const float S = H == 0 ? se[jj] * fa + so * fo : so * fo + se[jj] * fa;
     const float lse = M + logf(S);
     cw[jj] = xr[jj] >= 0 ? (fa / S) * won : 0.0f;
-    if (xr[jj] >= 0 && (xr[jj] * kGroupCols + jj) / (G::kSlots / 2) == H)
+    if (xr[jj] >= 0 && (xr[jj] * kGroupCols + jj) / (kGroupSlots / 2) == H)
       floss += (double)(wn * (lse - tg[jj]));
   }
   tmem_wait_st();
   // C: R = w (P - onehot), three digits per element
-  const long long rbase = (long long)n * args.S + (long long)t * G::kSlots;
+  const long long rbase = (long long)n * args.S + (long long)t * kGroupSlots;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int cc = kChunks * H + c;
-    uint32_t vbuf[32];
-    if (!REGS || c == 0) {
-      __syncwarp();
-      tmem_ld32(REGS ? t_stash : t_hi + cc * 32, vbuf);
-      tmem_wait_ld();
-    }
-    auto v = [&](int i) -> uint32_t {
-      if constexpr (REGS) return c == 0 ? vbuf[i] : zr[(c - 1) * 32 + i];
-      else return vbuf[i];
-    };
+    uint32_t v[32];
+    __syncwarp();
+    tmem_ld32(t_hi + cc * 32, v);
+    tmem_wait_ld();
     uint32_t w0[8], w1[8], w2[8];
 #pragma unroll
     for (int e4 = 0; e4 < 8; ++e4) {
@@ -522,7 +507,7 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
         float t = 0.0f;
         if (col < kGroupUsed) {
           const int a = col / kGroupCols, jj = col % kGroupCols;
-          t = fmaf(__uint_as_float(v(i)), cw[jj], xr[jj] == a ? -won : 0.0f);
+          t = fmaf(__uint_as_float(v[i]), cw[jj], xr[jj] == a ? -won : 0.0f);
         }
         // |R| 2^-eR <= 1: only the top of the range needs the clamp (P rounding to 1)
         qv[e] = min(__float2int_rn(t), (1 << kI8FracBits) - 1);
@@ -536,24 +521,7 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
       w1[e4] = pack(qv[0] >> 7, qv[1] >> 7, qv[2] >> 7, qv[3] >> 7) & 0x7F7F7F7Fu;
       w2[e4] = pack(qv[0], qv[1], qv[2], qv[3]) & 0x7F7F7F7Fu;
     }
-    long long off = rbase + cc * 32;
-    if constexpr (TILED) {
-      // the 32 slots [s0, s0 + 32) of row n are 16-byte chunks c, c + 1 (c even) of
-      // the tile row; swizzled to c ^ m and (c ^ m) ^ 1, m = n & 7: one aligned
-      // 32-byte pair, its halves exchanged when m is odd
-      const int s0 = t * G::kSlots + cc * 32;
-      const int m = n & 7, c = (s0 & 127) >> 4;
-      off = ((long long)(s0 >> 7) * (args.Npad >> 5) + (n >> 5)) * 4096 + (n & 31) * 128 +
-            (((c ^ m) & 6) << 4);
-      if (m & 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t v = w0[i]; w0[i] = w0[i + 4]; w0[i + 4] = v;
-          v = w1[i]; w1[i] = w1[i + 4]; w1[i + 4] = v;
-          v = w2[i]; w2[i] = w2[i + 4]; w2[i + 4] = v;
-        }
-      }
-    }
+    const long long off = rbase + cc * 32;
     st_global_v8(args.r[0] + off, w0);
     st_global_v8(args.r[1] + off, w1);
     st_global_v8(args.r[2] + off, w2);
@@ -759,18 +727,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
       const uint32_t lq = (uint32_t)(q * 32) << 16;
       const long long part = (long long)tile * 2 + rank;
       const bool narrow = L <= kI8NarrowMaxL;
-      if (half == 0 && narrow)
-        i8_fwd_epilogue_tile<Groups256, 0, false, false, true>(args, t_hi + lq, t_lo + lq, tab_scale,
-                                                           tab_v, xbuf, q, lane, n, t, part, lo_bar);
-      else if (half == 0)
-        i8_fwd_epilogue_tile<Groups256, 0>(args, t_hi + lq, t_lo + lq, tab_scale, tab_v, xbuf, q, lane, n, t,
-                                part, lo_bar);
-      else if (narrow)
-        i8_fwd_epilogue_tile<Groups256, 1, false, false, true>(args, t_hi + lq, t_lo + lq, tab_scale,
-                                                           tab_v, xbuf, q, lane, n, t, part, lo_bar);
-      else
-        i8_fwd_epilogue_tile<Groups256, 1>(args, t_hi + lq, t_lo + lq, tab_scale, tab_v, xbuf, q, lane, n, t,
-                                part, lo_bar);
+#define CCM_TILE_ARGS \
+  args, t_hi + lq, t_lo + lq, tab_scale, tab_v, xbuf, q, lane, n, t, part, lo_bar
+      if (half == 0 && narrow) i8_fwd_epilogue_tile<0, true>(CCM_TILE_ARGS);
+      else if (half == 0) i8_fwd_epilogue_tile<0, false>(CCM_TILE_ARGS);
+      else if (narrow) i8_fwd_epilogue_tile<1, true>(CCM_TILE_ARGS);
+      else i8_fwd_epilogue_tile<1, false>(CCM_TILE_ARGS);
+#undef CCM_TILE_ARGS
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(hi_bar);
@@ -848,12 +811,12 @@ __global__ void i8sp_onehot_kernel(const uint8_t *__restrict__ msa, uint32_t *__
 // for the three digit products (A x1, A x128, B d0..d2, E; 54 KB), so the one-hot
 // operand and its metadata cross L2 once per tile, not once per digit phase; the
 // kernel is bound by this L2 -> shared-memory operand stream.  The epilogue takes
-// the merged logits out of both accumulators during its merge pass (into TMEM
-// columns [192, 256) and registers) and releases them at once, so the next tile's
-// MMAs overlap the softmax and the R digits.
-// TMEM: hi = [0, 192), epilogue stash = [192, 256), lo = [256, 448), metadata
-// slots at 448 and 452.
+// the sums out of both accumulators into registers and releases them at once, so the
+// next tile's MMAs overlap the softmax and the R digits.
+// TMEM: hi = [0, 192), lo = [256, 448), metadata slots at 456 and 460.
 constexpr int kSpBN = Groups192::kSlots, kSpBK = 128;
+constexpr int kSpHalf = 99;  // tile columns of the epilogue's half 0 (half 1: 90)
+constexpr int kSpTab = 100;  // floats per half in its tables of scales and V
 
 struct I8SpSmem {
   static constexpr int kStages = 3;
@@ -866,13 +829,180 @@ struct I8SpSmem {
   static constexpr int kOffA1 = 0, kOffA128 = kA, kOffB = 2 * kA, kOffE = 2 * kA + 3 * kB;
   static constexpr int kStage = kOffE + kE;
   static constexpr int kBarOff = kStages * kStage;
-  static constexpr int kTabOff = kBarOff + 256;  // per tile: scale[192], V[192]
-  static constexpr int kXOff = kTabOff + 2 * kSpBN * 4;
-  static constexpr int kXBytes = 2 * kI8BM * 2 * Groups192::kCols * 4;
-  static constexpr int kTotal = kXOff + kXBytes + 1024;
+  static constexpr int kTabOff = kBarOff + 256;  // per tile: scale and V of both halves
+  static constexpr int kXOff = kTabOff + 4 * kSpTab * 4;  // per half, column and row: (max, sum)
+  static constexpr int kXBytes = 2 * Groups192::kCols * kI8BM * 8;
+  static constexpr int kROff = kXOff + kXBytes;  // per epilogue warp: 3 digits x 32 slots x 32 rows
+  static constexpr int kRWarp = 3 * 32 * 32;
+  static constexpr int kTotal = kROff + 8 * kRWarp + 1024;
 };
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
+// Epilogue of one tile for one warp (TMEM lane quarter q; half 0: states 0..10 of the
+// nine alignment columns, tile columns 0..98; half 1: states 11..20, columns 99..188):
+//   drain  hi * 2^14 + lo of the half into registers (NARROW: as the exact 32-bit
+//          integer, one instruction; else as the rounded float), the next 16 columns
+//          in flight; then both accumulators are released, so that the next tile's
+//          MMAs run during everything below;
+//   A      z = sum * scale + V; per alignment column the maximum m of the own states
+//          and the logit of the observed state;
+//   B      e = exp(z - m), s = sum e; (m, s) exchanged with the partner warp (same
+//          rows, other half): M = max(m, m'), S = s exp(m - M) + s' exp(m' - M) (same
+//          order in both halves), lse = M + log S;
+//   C      P = e * exp(m - M) / S, R = w (P - onehot) as its three digits, 32 slots x
+//          32 rows at a time through shared memory, so that a lane moves 16 rows of one
+//          slot with one store (byte stores straight to global memory, one sector each,
+//          took 60 k cycles per tile, this takes 20 k).
+// The whole half (99 values a thread) stays in registers: warpgroup 0 cedes its share
+// (kWgRegsLoad / kWgRegsEpi).  The accumulators are held for about 2 k of the tile's
+// 50 k cycles; a drain that also applied the scales and took the maxima held them 6 k.
+// Both halves run the same instructions (element i is state 11 half + i / 9, column
+// i % 9; half 1 ends at 90, its last nine elements have scale 0 and V = -inf): this
+// straight-line code is some 50 KB, and one copy per half did not fit the
+// instruction cache.
+template <bool NARROW>
+__device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32_t t_hi,
+                                                   uint32_t t_lo, const float *tab_scale,
+                                                   const float *tab_v, float2 *xbuf,
+                                                   uint8_t *rstage, int half, int q, int lane,
+                                                   int n, int t, long long part,
+                                                   uint64_t *full_bar, uint32_t full_par,
+                                                   long long budget, uint32_t empty_bar) {
+  constexpr int kCols = Groups192::kCols;
+  const int L = args.L;
+  const int j0 = t * kCols, a0 = 11 * half;
+  const bool live = n < args.N;
+  const float wn = live ? args.w[n] : 0.0f;
+  const int row = q * 32 + lane;
+  int xr[kCols];  // the observed state less a0; below -11: none
+#pragma unroll
+  for (int jj = 0; jj < kCols; ++jj)
+    xr[jj] = (live && j0 + jj < L) ? (int)args.msa[(long long)n * L + j0 + jj] - a0 : -100;
+  if (__any_sync(0xffffffffu, !mbar_wait(full_bar, full_par, budget))) {
+    named_bar_sync(2 + q, 64);  // the partner may have got past its wait
+    return false;
+  }
+  tc_fence_after();
+  float z[kSpHalf + 1];
+  {
+    const uint32_t c0 = half * kSpHalf;
+    auto merge = [](uint32_t hi, uint32_t lo) {
+      return NARROW ? __uint_as_float(hi * 16384u + lo) : i8_merge_exact(hi, lo);
+    };
+    uint32_t vh[2][16], vl[2][16];
+    tmem_ld16(t_hi + c0, vh[0]);
+    tmem_ld16(t_lo + c0, vl[0]);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      tmem_wait_ld();
+      if (c < 5) {
+        tmem_ld16(t_hi + c0 + (c + 1) * 16, vh[(c + 1) & 1]);
+        tmem_ld16(t_lo + c0 + (c + 1) * 16, vl[(c + 1) & 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) z[c * 16 + i] = merge(vh[c & 1][i], vl[c & 1][i]);
+    }
+    z[96] = z[97] = z[98] = 0.0f;
+    if (half == 0) {
+      uint32_t wh[4], wl[4];
+      tmem_ld4(t_hi + 96, wh);
+      tmem_ld4(t_lo + 96, wl);
+      tmem_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 3; ++i) z[96 + i] = merge(wh[i], wl[i]);
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive_cluster(empty_bar);
+  // A
+  float mx[kCols], tg[kCols], se[kCols];
+#pragma unroll
+  for (int jj = 0; jj < kCols; ++jj) { mx[jj] = -INFINITY; tg[jj] = 0.0f; se[jj] = 0.0f; }
+  tab_scale += half * kSpTab;
+  tab_v += half * kSpTab;
+#pragma unroll
+  for (int i4 = 0; i4 < kSpTab; i4 += 4) {
+    const float4 sc = *reinterpret_cast<const float4 *>(tab_scale + i4);
+    const float4 vv = *reinterpret_cast<const float4 *>(tab_v + i4);
+    const float scs[4] = {sc.x, sc.y, sc.z, sc.w}, vvs[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i4 + e;
+      if (i < kSpHalf) {
+        const int jj = i % kCols;
+        const float sum = NARROW ? __int2float_rn(__float_as_int(z[i])) : z[i];
+        z[i] = fmaf(sum, scs[e], vvs[e]);
+        mx[jj] = fmaxf(mx[jj], z[i]);
+        if (xr[jj] == i / kCols) tg[jj] = z[i];
+      }
+    }
+  }
+  // B
+#pragma unroll
+  for (int i = 0; i < kSpHalf; ++i) {
+    const int jj = i % kCols;
+    z[i] = expf(z[i] - mx[jj]);
+    se[jj] += z[i];
+  }
+#pragma unroll
+  for (int jj = 0; jj < kCols; ++jj)
+    xbuf[(half * kCols + jj) * kI8BM + row] = make_float2(mx[jj], se[jj]);
+  named_bar_sync(2 + q, 64);
+  double floss = 0.0;
+  // R * 2^21 = e * cw - [observed] * won, with cw = w exp(m - M) / S * 2^21
+  float cw[kCols];
+  const float won = live ? wn * args.r_enc : 0.0f;
+#pragma unroll
+  for (int jj = 0; jj < kCols; ++jj) {
+    const float2 other = xbuf[((1 - half) * kCols + jj) * kI8BM + row];
+    const float mo = other.x, so = other.y;
+    const float M = fmaxf(mx[jj], mo);
+    const float fa = expf(mx[jj] - M), fo = expf(mo - M);
+    const float S = half == 0 ? se[jj] * fa + so * fo : so * fo + se[jj] * fa;
+    const float lse = M + logf(S);
+    cw[jj] = xr[jj] > -100 ? (fa / S) * won : 0.0f;
+    // the half that holds the observed state adds the loss term
+    if (xr[jj] >= 0 && xr[jj] < 11) floss += (double)(wn * (lse - tg[jj]));
+  }
+  // C
+  uint8_t *const rrow = args.rnat + (long long)(n >> 5) * (3 * kNatTile);
+  const long long sbytes = (long long)(args.Npad >> 5) * (3 * kNatTile);
+  const int used = half == 0 ? kSpHalf : 90;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (c * 32 + i < kSpHalf) {
+        const int jj = (c * 32 + i) % kCols;
+        const float r = fmaf(z[c * 32 + i], cw[jj], xr[jj] == (c * 32 + i) / kCols ? -won : 0.0f);
+        // |R| 2^-eR <= 1: only the top of the range needs the clamp (P rounding to 1)
+        const int d = min(__float2int_rn(r), (1 << kI8FracBits) - 1);
+        rstage[i * 32 + lane] = (uint8_t)(d >> 14);
+        rstage[1024 + i * 32 + lane] = (uint8_t)((d >> 7) & 127);
+        rstage[2048 + i * 32 + lane] = (uint8_t)(d & 127);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < (c < 3 ? 2 : 1); ++u) {
+      const int i = 16 * u + (lane >> 1), el = c * 32 + i;
+      const int a = a0 + el / kCols, j = j0 + el % kCols;
+      if (el < used && j < L) {
+        const uint32_t s = (uint32_t)(a * L + j);
+        uint8_t *p = rrow + (long long)(s >> 7) * sbytes + (s & 127) * 32 + (((lane ^ (s >> 2)) & 1) << 4);
+        const uint4 *from = reinterpret_cast<const uint4 *>(rstage + i * 32 + (lane & 1) * 16);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4 *>(p + k * kNatTile) = from[k * 64];
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) floss += __shfl_xor_sync(0xffffffffu, floss, o);
+  if (lane == 0) args.part_f[part * 8 + half * 4 + q] = floss;
+  return true;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8sp_forward_kernel(const __grid_constant__ I8SpMaps maps, I8FwdArgs args) {
   using SM = I8SpSmem;
   constexpr int kStages = SM::kStages;
@@ -889,8 +1019,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(never + 1);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
   float *tab_scale = reinterpret_cast<float *>(smem + SM::kTabOff);
-  float *tab_v = tab_scale + kSpBN;
-  float *xbuf = reinterpret_cast<float *>(smem + SM::kXOff);
+  float *tab_v = tab_scale + 2 * kSpTab;
+  float2 *xbuf = reinterpret_cast<float2 *>(smem + SM::kXOff);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -921,10 +1051,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
   griddep_launch();
   griddep_wait();
   const uint32_t tmem_base = *tmem_slot;
-  // TMEM: hi [0, 192), the epilogue's stash [192, 256), lo [256, 448), metadata 448 / 452
-  const uint32_t t_hi = tmem_base, t_lo = tmem_base + 256, t_e = tmem_base + 448;
-  const uint32_t t_stash = tmem_base + kSpBN;
+  // TMEM: hi [0, 192), lo [256, 448), metadata 456 / 460 (the epilogue's 16-column
+  // loads reach up to three columns past an accumulator)
+  const uint32_t t_hi = tmem_base, t_lo = tmem_base + 256, t_e = tmem_base + 456;
 
+  if (warp < 4) reg_dec<kWgRegsLoad>();
   if (warp == 0) {
     if (lane == 0) {
       // ---------------- TMA producer (both CTAs), in the MMA's order
@@ -1009,61 +1140,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
       umma_commit_pair(drain, 0x1);
       if (!mbar_wait(drain, 0)) i8_record_error(args.status, kErrFwdTimeout, abort_flag);
     }
-  } else {
+  } else if (warp >= 4) {
+    reg_inc<kWgRegsEpi>();
     // ---------------- epilogue (both CTAs): 8 warps, lane quarter q, column half
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int ethr = threadIdx.x - 64;
+    const int half = (warp - 4) >> 2;
+    const int ethr = threadIdx.x - 128;
     const int L = args.L;
+    uint8_t *const rstage = smem + SM::kROff + (warp - 4) * SM::kRWarp;
     const uint32_t empty_bar = mapa_shared(smem_u32(acc_empty), 0);
 
     int local = 0;
     for (int tile = pair; tile < n_tiles; tile += npairs, ++local) {
       if (named_bar_or(1, 256, i8_aborted(abort_flag))) break;
       const int m = tile % args.m_tiles, t = tile / args.m_tiles;
-      if (ethr < kSpBN) {
-        const int r = ethr;
+      if (ethr < 2 * kSpTab) {
+        const int hf = ethr / kSpTab, i = ethr % kSpTab;
         float sc = 0.0f, vv = 0.0f;
-        if (r < Groups192::kUsed) {
-          const int a = r / Groups192::kCols, j = t * Groups192::kCols + r % Groups192::kCols;
+        if (i >= (hf == 0 ? kSpHalf : 90)) {
+          vv = -INFINITY;  // no state
+        } else {
+          const int a = 11 * hf + i / Groups192::kCols, j = t * Groups192::kCols + i % Groups192::kCols;
           if (j < L) {
             sc = pow2f(col_exponent(args.colmax[a * L + j]) - kI8FracBits);
             if (a < kQ - 1) vv = args.x1[a * L + j];
           }
         }
-        tab_scale[r] = sc;
-        tab_v[r] = vv;
+        tab_scale[ethr] = sc;
+        tab_v[ethr] = vv;
       }
       named_bar_sync(1, 256);
       const int n = m * kI8PairM + (int)rank * kI8BM + q * 32 + lane;
-      // (with acc_wait_cycles set, a wait that runs out by design: see `never`)
-      const bool ok = args.acc_wait_cycles > 0 ? mbar_wait(never, 0, args.acc_wait_cycles)
-                                               : mbar_wait(acc_full, local & 1);
-      if (__any_sync(0xffffffffu, !ok)) {
-        if (lane == 0) i8_record_error(args.status, kErrFwdTimeout, abort_flag);
-        continue;
-      }
-      tc_fence_after();
       const uint32_t lq = (uint32_t)(q * 32) << 16;
       const long long part = (long long)tile * 2 + rank;
-      // both accumulators are released inside, right after the merge
-      const bool narrow = L <= kI8NarrowMaxL;
-      if (half == 0 && narrow)
-        i8_fwd_epilogue_tile<Groups192, 0, true, true, true>(args, t_hi + lq, t_lo + lq, tab_scale,
-                                                       tab_v, xbuf, q, lane, n, t, part, empty_bar,
-                                                       t_stash + lq);
-      else if (half == 0)
-        i8_fwd_epilogue_tile<Groups192, 0, true, true>(args, t_hi + lq, t_lo + lq, tab_scale, tab_v,
-                                                 xbuf, q, lane, n, t, part, empty_bar,
-                                                 t_stash + lq);
-      else if (narrow)
-        i8_fwd_epilogue_tile<Groups192, 1, true, true, true>(args, t_hi + lq, t_lo + lq, tab_scale,
-                                                       tab_v, xbuf, q, lane, n, t, part, empty_bar,
-                                                       t_stash + 32 + lq);
-      else
-        i8_fwd_epilogue_tile<Groups192, 1, true, true>(args, t_hi + lq, t_lo + lq, tab_scale, tab_v,
-                                                 xbuf, q, lane, n, t, part, empty_bar,
-                                                 t_stash + 32 + lq);
+      // (with acc_wait_cycles set, a wait that runs out by design: see `never`)
+      const bool test = args.acc_wait_cycles > 0;
+#define CCM_TILE_ARGS                                                                             \
+  args, t_hi + lq, t_lo + lq, tab_scale, tab_v, xbuf, rstage, half, q, lane, n, t, part,          \
+      test ? never : acc_full, test ? 0u : (uint32_t)(local & 1),                                 \
+      test ? args.acc_wait_cycles : kWaitBudgetCycles, empty_bar
+      const bool ok = L <= kI8NarrowMaxL ? i8sp_epilogue_tile<true>(CCM_TILE_ARGS)
+                                         : i8sp_epilogue_tile<false>(CCM_TILE_ARGS);
+#undef CCM_TILE_ARGS
+      if (!ok && lane == 0) i8_record_error(args.status, kErrFwdTimeout, abort_flag);
     }
   }
 
@@ -1100,14 +1219,15 @@ struct I8BwdSmem {
   static constexpr int kStage = 10 * kTile;
   static constexpr int kBarOff = kStages * kStage;
   static constexpr int kTOff = kBarOff + 256;
-  static constexpr int kTBytes = 8 * 32 * 9 * 4;
+  static constexpr int kTBytes = 8 * kBwdOutWarpBytes;
   static constexpr int kTotal = kTOff + kTBytes + 1024;
 };
 
-// TILED: the operands are in the tiled storage of i8_bwd_tile_offset (the sparse
-// path); else row-major Npad x S.  The shared-memory images are the same.
-template <bool SYM, class G, bool TILED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
+// NAT: natural slots, K-major operands in the storage of i8nat_offset (the sparse
+// path); else Groups256 slots, row-major Npad x S operands (MN-major).  The MMAs run
+// at the same rate either way.
+template <bool SYM, bool NAT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8_backward_kernel(const __grid_constant__ I8BwdMaps maps, BwdArgs args) {
   using SM = I8BwdSmem;
   constexpr int kStages = SM::kStages;
@@ -1138,8 +1258,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
   }
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&maps.o1);
-    prefetch_tmap(&maps.o128);
-    for (int i = 0; i < 3; ++i) prefetch_tmap(&maps.r[i]);
+    prefetch_tmap(&maps.r[0]);
+    if (!NAT) {
+      prefetch_tmap(&maps.o128);
+      prefetch_tmap(&maps.r[1]);
+      prefetch_tmap(&maps.r[2]);
+    }
   }
   if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
   tc_fence_before();
@@ -1151,6 +1275,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t t_hi = tmem_base, t_lo = tmem_base + kBN;
 
+  if (warp < 4) reg_dec<kWgRegsLoad>();
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;
@@ -1168,25 +1293,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
             break;
           }
           uint8_t *st = smem + stage * SM::kStage;
-          // row-major: box (slot x, row y); tiled: the 4 KB tile of (slot block,
-          // K block) is 16 rows of 256 bytes at row 16 * (sb * KB + kb)
-          const int y = kb * kI8BwdBK;
-          const int xp = TILED ? 0 : xP, xq = TILED ? 0 : xQ;
-          const int yp = TILED ? ((xP >> 7) * k_blocks + kb) * 16 : y;
-          const int yq = TILED ? ((xQ >> 7) * k_blocks + kb) * 16 : y;
           const uint32_t fb = mapa_shared(smem_u32(&full[stage]), 0);
           if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * (SYM ? 10 : 5) * SM::kTile);
-          tma_load_2d_pair(st + 0 * SM::kTile, &maps.o1, fb, xp, yp);
-          tma_load_2d_pair(st + 1 * SM::kTile, &maps.o128, fb, xp, yp);
-          if (SYM)
+          uint8_t *const stq = st + 5 * SM::kTile;
+          if constexpr (NAT) {
+            // rows of 256 bytes: 32 per one-hot tile pair, 48 per digit tile triple
+            const int tp = (xP >> 7) * k_blocks + kb, tq = (xQ >> 7) * k_blocks + kb;
+            tma_load_2d_pair(st, &maps.o1, fb, 0, tp * 32);
+            if (SYM) tma_load_2d_pair(st + 2 * SM::kTile, &maps.r[0], fb, 0, tp * 48);
+            if (SYM) tma_load_2d_pair(stq, &maps.o1, fb, 0, tq * 32);
+            tma_load_2d_pair(stq + 2 * SM::kTile, &maps.r[0], fb, 0, tq * 48);
+          } else {
+            const int y = kb * kI8BwdBK;
+            tma_load_2d_pair(st + 0 * SM::kTile, &maps.o1, fb, xP, y);
+            tma_load_2d_pair(st + 1 * SM::kTile, &maps.o128, fb, xP, y);
+            if (SYM) {
+              for (int i = 0; i < 3; ++i)
+                tma_load_2d_pair(st + (2 + i) * SM::kTile, &maps.r[i], fb, xP, y);
+              tma_load_2d_pair(stq, &maps.o1, fb, xQ, y);
+              tma_load_2d_pair(stq + SM::kTile, &maps.o128, fb, xQ, y);
+            }
             for (int i = 0; i < 3; ++i)
-              tma_load_2d_pair(st + (2 + i) * SM::kTile, &maps.r[i], fb, xp, yp);
-          if (SYM) {
-            tma_load_2d_pair(st + 5 * SM::kTile, &maps.o1, fb, xq, yq);
-            tma_load_2d_pair(st + 6 * SM::kTile, &maps.o128, fb, xq, yq);
+              tma_load_2d_pair(stq + (2 + i) * SM::kTile, &maps.r[i], fb, xQ, y);
           }
-          for (int i = 0; i < 3; ++i)
-            tma_load_2d_pair(st + (7 + i) * SM::kTile, &maps.r[i], fb, xq, yq);
         }
       }
       const uint32_t issued = it;
@@ -1201,8 +1330,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
-      constexpr uint32_t id_us = idesc_i8_s32(kPairM, kBN, 0, 1, 1, 1);  // A = one-hot, B = R
-      constexpr uint32_t id_su = idesc_i8_s32(kPairM, kBN, 1, 0, 1, 1);  // A = R, B = one-hot
+      constexpr int mn = NAT ? 0 : 1;
+      constexpr uint32_t id_us = idesc_i8_s32(kPairM, kBN, 0, 1, mn, mn);  // A = one-hot, B = R
+      constexpr uint32_t id_su = idesc_i8_s32(kPairM, kBN, 1, 0, mn, mn);  // A = R, B = one-hot
       uint32_t it = 0, chunk = 0;
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok && !i8_aborted(abort_flag); tile += npairs) {
@@ -1224,7 +1354,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
             }
             tc_fence_after();
             const uint32_t s0 = smem_u32(smem + stage * SM::kStage);
-            auto d = [&](int i) { return sdesc_sw128(s0 + i * SM::kTile, SM::kTile, 1024); };
+            auto d = [&](int i) {
+              return NAT ? sdesc_sw32(s0 + i * SM::kTile, 16, 256)
+                         : sdesc_sw128(s0 + i * SM::kTile, SM::kTile, 1024);
+            };
             const uint32_t first = kb == kb0 ? 0u : 1u;
             umma_i8_pair(t_hi, d(0), d(7), id_us, first);  // O1_P^T r0_Q
             umma_i8_pair(t_lo, d(1), d(8), id_us, first);  // O128_P^T r1_Q
@@ -1243,104 +1376,63 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
       umma_commit_pair(drain, 0x1);
       if (!mbar_wait(drain, 0)) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
     }
-  } else {
-    // Epilogue: as tc_backward, with each K chunk merged from the two integer
-    // accumulators (16 columns per TMEM load) into FP32 registers.
+  } else if (warp >= 4) {
+    reg_inc<kWgRegsEpi>();
+    // Epilogue: each K chunk merged from the two integer accumulators (16 columns
+    // per TMEM load, the next 16 in flight) into FP32 registers, then added to g.
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int L = args.L;
-    float *__restrict__ g2 = args.g2;
-    float *Tb = reinterpret_cast<float *>(smem + SM::kTOff) + (warp - 2) * 32 * 9;
+    const int half = (warp - 4) >> 2;
+    float *Tb = reinterpret_cast<float *>(smem + SM::kTOff + (warp - 4) * kBwdOutWarpBytes);
     const float r_dec = args.r_dec;
     const uint32_t empty_bar = mapa_shared(smem_u32(acc_empty), 0);
+    const uint32_t col0 = half * kHalfN + ((uint32_t)(q * 32) << 16);
     uint32_t chunk = 0;
     bool ok = true;
     for (int tile = pair; tile < n_tiles && ok; tile += npairs) {
       float accv[kHalfN];
-#pragma unroll
-      for (int i = 0; i < kHalfN; ++i) accv[i] = 0.0f;
-      for (int kb0 = 0; kb0 < k_blocks; kb0 += kI8BwdChunkKB, ++chunk) {
+      // one K chunk: wait for it, merge it into accv (or add it there), release it
+      auto take = [&](auto first) {
         const bool w_ok = mbar_wait(acc_full, chunk & 1);
         if (__any_sync(0xffffffffu, !w_ok)) {
           if (lane == 0) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
-          ok = false;
-          break;
+          return false;
         }
         tc_fence_after();
-        const uint32_t col0 = half * kHalfN + ((uint32_t)(q * 32) << 16);
+        uint32_t vh[2][16], vl[2][16];
+        __syncwarp();
+        tmem_ld16(t_hi + col0, vh[0]);
+        tmem_ld16(t_lo + col0, vl[0]);
 #pragma unroll
         for (int c = 0; c < kHalfN / 16; ++c) {
-          uint32_t vh[16], vl[16];
-          __syncwarp();
-          tmem_ld16(t_hi + col0 + c * 16, vh);
-          tmem_ld16(t_lo + col0 + c * 16, vl);
           tmem_wait_ld();
+          if (c + 1 < kHalfN / 16) {
+            tmem_ld16(t_hi + col0 + (c + 1) * 16, vh[(c + 1) & 1]);
+            tmem_ld16(t_lo + col0 + (c + 1) * 16, vl[(c + 1) & 1]);
+          }
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const long long qs = (long long)(int)vh[i] * 16384 + (long long)(int)vl[i];
-            // exact 64-bit sum, one rounding to float, exact scaling by 2^(eR - 21)
-            accv[c * 16 + i] += __ll2float_rn(qs) * r_dec;
+            // exact scaling by 2^(eR - 21)
+            const float v = i8_merge_exact(vh[c & 1][i], vl[c & 1][i]);
+            if constexpr (decltype(first)::value) accv[c * 16 + i] = v * r_dec;
+            else accv[c * 16 + i] = fmaf(v, r_dec, accv[c * 16 + i]);
           }
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(empty_bar);
-      }
+        ++chunk;
+        return true;
+      };
+      ok = take(std::true_type{});
+      for (int kb0 = kI8BwdChunkKB; kb0 < k_blocks && ok; kb0 += kI8BwdChunkKB)
+        ok = take(std::false_type{});
       if (!ok) break;
-
       const int2 pq = args.tiles[tile];
-      const int rowbase = pq.x * kPairM + (int)rank * kBM + q * 32;
-      const int s1 = rowbase + lane;
-      const int t1 = s1 / G::kSlots, r1 = s1 % G::kSlots;
-      const int b = r1 / G::kCols, k = t1 * G::kCols + r1 % G::kCols;
-      const bool valid1 = r1 < G::kUsed && k < L;
-      const long long colt = (long long)b * L + k;
-      // the Q slots of this warp: sQ + i, i < 128 (with 192-slot groups a 256-slot
-      // tile half may cross a group boundary: decode each slot on its own)
-      const int sQ = pq.y * kBN + half * kHalfN;
-#pragma unroll
-      for (int cb = 0; cb < kHalfN / 8; ++cb) {
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) Tb[lane * 9 + e] = accv[cb * 8 + e];
-        __syncwarp();
-        if (SYM) {
-#pragma unroll 1
-          for (int col = 0; col < 8; ++col) {
-            const int s2 = sQ + cb * 8 + col;
-            const int t2 = s2 / G::kSlots, r2 = s2 % G::kSlots;
-            const int a = r2 / G::kCols, j = t2 * G::kCols + r2 % G::kCols;
-            const bool valid2 = r2 < G::kUsed && j < L;
-            if (s1 < s2) {
-              const float val = Tb[lane * 9 + col];
-              if (valid1 && valid2) {
-                if (k != j) atomicAdd(g2 + ((long long)a * L + j) * kQPad * L + colt, val);
-              } else if (s2 == G::kOnes && valid1 && b < kQ - 1) {
-                args.g1d[b * L + k] = val;
-              }
-            }
-          }
-        }
-        const int col = lane & 7;
-        const int s2 = sQ + cb * 8 + col;
-        const int t2 = s2 / G::kSlots, r2 = s2 % G::kSlots;
-        const int a = r2 / G::kCols, j = t2 * G::kCols + r2 % G::kCols;
-        const bool valid2 = r2 < G::kUsed && j < L;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int row = 4 * it + (lane >> 3);
-          const int s1r = rowbase + row;
-          if (SYM && s1r > s2) continue;
-          const float val = Tb[row * 9 + col];
-          const int tr = s1r / G::kSlots, rr = s1r % G::kSlots;
-          const int br = rr / G::kCols, kr = tr * G::kCols + rr % G::kCols;
-          if (rr < G::kUsed && kr < L) {
-            if (valid2 && (!SYM || kr != j)) atomicAdd(g2 + x2_index(br, kr, a, j, L), val);
-          } else if (s1r == G::kOnes && valid2 && a < kQ - 1) {
-            args.g1d[a * L + j] = val;
-          }
-        }
-      }
+      const int s1 = pq.x * kPairM + (int)rank * kBM + q * 32, s2 = pq.y * kBN + half * kHalfN;
+      if constexpr (NAT)
+        bwd_output_natural<SYM>(accv, Tb, args.g2, args.g1d, args.L, lane, s1, s2, pq.x == pq.y);
+      else
+        bwd_output<Groups256, SYM>(accv, Tb, args.g2, args.g1d, args.L, lane, s1, s2);
     }
   }
 
@@ -1417,6 +1509,7 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   I8FwdArgs fa{};
   fa.msa = c->d_msa; fa.w = c->d_w; fa.x1 = x1; fa.colmax = c->d_colmax;
   for (int i = 0; i < 3; ++i) fa.r[i] = c->d_rdig[i];
+  fa.rnat = c->d_rnat;
   fa.part_f = c->d_part_f; fa.status = c->d_status;
   fa.L = L; fa.N = c->N; fa.S = c->S; fa.T = c->T; fa.Npad = c->Npad;
   fa.m_tiles = c->Npad / kI8PairM;
@@ -1426,7 +1519,7 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   const int pair_tiles = fa.m_tiles * c->T;
   const int fpairs = pair_tiles < c->fwd_pairs ? pair_tiles : c->fwd_pairs;
   if (sp)
-    e = launch_pdl(i8sp_forward_kernel, dim3(2 * fpairs), dim3(kI8Threads), I8SpSmem::kTotal,
+    e = launch_pdl(i8sp_forward_kernel, dim3(2 * fpairs), dim3(kWgThreads), I8SpSmem::kTotal,
                    c->stream, c->i8sp_maps, fa);
   else
     e = launch_pdl(i8_forward_kernel, dim3(2 * fpairs), dim3(kI8Threads), I8FwdSmem::kTotal,
@@ -1442,11 +1535,11 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   const int bpairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
   const bool sym = c->gradient != CCM_GRADIENT_PARTIAL;
   const dim3 bgrid(2 * bpairs);
-  auto bwd = sp && sym ? i8_backward_kernel<true, Groups192, true>
-             : sp        ? i8_backward_kernel<false, Groups192, true>
-             : sym       ? i8_backward_kernel<true, Groups256, false>
-                         : i8_backward_kernel<false, Groups256, false>;
-  e = launch_pdl(bwd, bgrid, dim3(kI8Threads), I8BwdSmem::kTotal, c->stream, c->i8bwd_maps, ba);
+  auto bwd = sp && sym ? i8_backward_kernel<true, true>
+             : sp        ? i8_backward_kernel<false, true>
+             : sym       ? i8_backward_kernel<true, false>
+                         : i8_backward_kernel<false, false>;
+  e = launch_pdl(bwd, bgrid, dim3(kWgThreads), I8BwdSmem::kTotal, c->stream, c->i8bwd_maps, ba);
   if (e != cudaSuccess) return e;
   prof_mark(c);
 
@@ -1471,14 +1564,14 @@ cudaError_t i8_configure_kernels() {
       (e = cudaFuncSetAttribute(i8sp_forward_kernel, (cudaFuncAttribute)kMax, I8SpSmem::kTotal)) !=
           cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute(i8_backward_kernel<true, Groups256, false>, (cudaFuncAttribute)kMax,
+  if ((e = cudaFuncSetAttribute(i8_backward_kernel<true, false>, (cudaFuncAttribute)kMax,
                                 I8BwdSmem::kTotal)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8_backward_kernel<false, Groups256, false>, (cudaFuncAttribute)kMax,
+      (e = cudaFuncSetAttribute(i8_backward_kernel<false, false>, (cudaFuncAttribute)kMax,
                                 I8BwdSmem::kTotal)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8_backward_kernel<true, Groups192, true>, (cudaFuncAttribute)kMax,
+      (e = cudaFuncSetAttribute(i8_backward_kernel<true, true>, (cudaFuncAttribute)kMax,
                                 I8BwdSmem::kTotal)) != cudaSuccess)
     return e;
-  return cudaFuncSetAttribute(i8_backward_kernel<false, Groups192, true>, (cudaFuncAttribute)kMax,
+  return cudaFuncSetAttribute(i8_backward_kernel<false, true>, (cudaFuncAttribute)kMax,
                               I8BwdSmem::kTotal);
 }
 
@@ -1494,7 +1587,7 @@ cudaError_t i8_forward_max_pairs(int *pairs) {
 cudaError_t i8sp_forward_max_pairs(int *pairs) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2, 1, 1);
-  cfg.blockDim = dim3(kI8Threads, 1, 1);
+  cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = I8SpSmem::kTotal;
   *pairs = 0;
   return cudaOccupancyMaxActiveClusters(pairs, i8sp_forward_kernel, &cfg);
@@ -1503,30 +1596,48 @@ cudaError_t i8sp_forward_max_pairs(int *pairs) {
 cudaError_t i8_backward_max_pairs(int *pairs) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2, 1, 1);
-  cfg.blockDim = dim3(kI8Threads, 1, 1);
+  cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = I8BwdSmem::kTotal;
   *pairs = 0;
-  return cudaOccupancyMaxActiveClusters(pairs, i8_backward_kernel<true, Groups256, false>, &cfg);
+  return cudaOccupancyMaxActiveClusters(pairs, i8_backward_kernel<true, false>, &cfg);
 }
 
 // One-hot operands for a context of the integer paths (Npad x S bytes each), and
 // for the sparse path the compressed forward operand with its metadata.
 cudaError_t i8_build_onehot(ccm_context *c) {
-  const long long total = (long long)c->Npad * c->S;
-  const unsigned grid = (unsigned)((total + 255) / 256);
   if (c->path != CCM_PATH_TC_I8SP) {
-    i8_onehot_kernel<Groups256, false><<<grid, 256, 0, c->stream>>>(c->d_msa, c->d_o1, c->d_o128, c->L,
-                                                             c->N, c->S, c->Npad);
+    const long long total = (long long)c->Npad * c->S;
+    i8_onehot_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(
+        c->d_msa, c->d_o1, c->d_o128, c->L, c->N, c->S, c->Npad);
     return cudaGetLastError();
   }
-  // the sparse path's backward reads its operands from tiled storage
-  i8_onehot_kernel<Groups192, true><<<grid, 256, 0, c->stream>>>(c->d_msa, c->d_o1, c->d_o128, c->L,
-                                                           c->N, c->S, c->Npad);
+  i8nat_onehot_kernel<<<dim3(c->Npad / 32, c->SB / 128), 128, 0, c->stream>>>(
+      c->d_msa, c->d_onat, c->L, c->N, c->Npad / 32);
   const long long bytes = (long long)c->Npad * (c->KP / 8);
   i8sp_onehot_kernel<<<(unsigned)((bytes + 255) / 256), 256, 0, c->stream>>>(
       c->d_msa, reinterpret_cast<uint32_t *>(c->d_ac1), reinterpret_cast<uint32_t *>(c->d_ac128),
       c->d_meta, c->L, c->N, c->KP, c->Npad);
   return cudaGetLastError();
+}
+
+// Matrix `mat` of the `mats` side by side of the backward's natural storage
+// (i8nat_offset), as Npad x S bytes of the forward's 192-slot groups in 32-row x
+// 128-slot tiles, tile (n / 32, s / 128) at 4096 ((s / 128) KB + n / 32), the 16-byte
+// chunk c of a row n of 128 slots at chunk c ^ (n & 7): the order in which
+// ccm_debug_copy hands these operands out.
+void i8nat_to_groups(const ccm_context *c, const uint8_t *nat, int mats, int mat, uint8_t *dst) {
+  const int KB = c->Npad / 32;
+  for (int s = 0; s < c->S; ++s) {
+    const int t = s / Groups192::kSlots, r = s % Groups192::kSlots;
+    const int l = t * Groups192::kCols + r % Groups192::kCols;
+    int ns = -1;
+    if (s == Groups192::kOnes) ns = kQ * c->L;
+    else if (r < Groups192::kUsed && l < c->L) ns = (r / Groups192::kCols) * c->L + l;
+    for (int n = 0; n < c->Npad; ++n)
+      dst[((long long)(s >> 7) * KB + (n >> 5)) * 4096 + (n & 31) * 128 +
+          (((((s & 127) >> 4) ^ (n & 7)) & 7) << 4) + (s & 15)] =
+          ns < 0 ? 0 : nat[i8nat_offset(n, ns, KB, mats) + (long long)mat * kNatTile];
+  }
 }
 
 }  // namespace ccm
