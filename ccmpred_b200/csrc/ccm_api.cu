@@ -281,7 +281,12 @@ int alloc_tc(ccm_context *c) {
       CCM_CUDA_TRY(dev_alloc(c, &c->d_ac128, Np * c->KP / 2));
       CCM_CUDA_TRY(dev_alloc(c, &c->d_meta, Np * c->KP / 8));
     }
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_colmax, sizeof(uint32_t) * (((kQ * c->L + 3) & ~3) + S)));
+    CCM_CUDA_TRY(dev_alloc(c, &c->d_colmax,
+                           sizeof(uint32_t) * (((kQ * c->L + 3) & ~3) + (sp ? 0 : S))));
+    if (sp) {
+      CCM_CUDA_TRY(dev_alloc(c, &c->d_cmacc, sizeof(uint32_t) * kQ * c->L));
+      CCM_CUDA_TRY(cudaMemsetAsync(c->d_cmacc, 0, sizeof(uint32_t) * kQ * c->L, c->stream));
+    }
   } else {
     CCM_CUDA_TRY(dev_alloc(c, &c->d_onehot, sizeof(__nv_bfloat16) * Np * S));
     for (int i = 0; i < c->nsplit; ++i) {
@@ -382,7 +387,7 @@ void free_all(ccm_context *c) {
   f(c->d_msa); f(c->d_w); f(c->d_out); f(c->d_onehot);
   for (int i = 0; i < 3; ++i) { f(c->d_wperm[i]); f(c->d_r[i]); f(c->d_wdig[i]); f(c->d_rdig[i]); }
   f(c->d_o1); f(c->d_o128); f(c->d_colmax); f(c->d_ac1); f(c->d_ac128); f(c->d_meta);
-  f(c->d_onat); f(c->d_rnat);
+  f(c->d_onat); f(c->d_rnat); f(c->d_cmacc);
   f(c->d_part_f); f(c->d_part_reg); f(c->d_fin_part); f(c->d_fin_done); f(c->d_g1d); f(c->d_bwd_tiles);
   f(c->d_simt_pc); f(c->d_simt_g2); f(c->d_simt_part); f(c->d_simt_g1);
   f(c->d_xh); f(c->d_gh);
@@ -403,9 +408,17 @@ int check_status(ccm_context *c) {
   return CCM_OK;
 }
 
-int enqueue_eval(ccm_context *c, const float *d_x, float *d_g) {
+// The result record, cleared before an evaluation (the sparse path's first kernel does it).
+int clear_result(ccm_context *c) {
+  if (c->path == CCM_PATH_TC_I8SP) return CCM_OK;
   CCM_CUDA_TRY(zero_words(c->d_out, sizeof(ccm_result) / 4, c->stream));
   count_launch(c);
+  return CCM_OK;
+}
+
+int enqueue_eval(ccm_context *c, const float *d_x, float *d_g) {
+  int rc = clear_result(c);
+  if (rc != CCM_OK) return rc;
   c->prof_idx = 0;
   cudaError_t e;
   switch (c->path) {
@@ -444,8 +457,8 @@ int ccm::enqueue_evaluation_step(ccm_context *c, const float *d_x, const float *
   const bool i8 = c->path == CCM_PATH_TC_I8X3 || c->path == CCM_PATH_TC_I8SP;
   if (c->path != CCM_PATH_TC_BF16X2 && c->path != CCM_PATH_TC_BF16X3 && !i8)
     return set_error(CCM_ERR_INVALID, "fused step: tensor-core paths only");
-  CCM_CUDA_TRY(zero_words(c->d_out, sizeof(ccm_result) / 4, c->stream));
-  count_launch(c);
+  int rc = clear_result(c);
+  if (rc != CCM_OK) return rc;
   c->prof_idx = 0;
   const cudaError_t e = i8
                             ? i8_evaluate(c, d_x, d_g, d_s, d_alpha, d_xt)

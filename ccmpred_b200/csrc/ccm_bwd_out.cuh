@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include "ccm_internal.cuh"
 #include "ccm_layout.cuh"
 #include "ccm_ptx.cuh"
 
@@ -117,20 +118,24 @@ __device__ __forceinline__ void bwd_output(const float (&acc)[128], float *Tb, f
 // takes 10-18 k here; with 325 instead of 351 tiles the backward went from 470 to
 // 375 us at L = 300, N = 5000 and from 53 to 23 us at L = 50, N = 200.
 template <bool SYM>
-__device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb, float *g2,
-                                                   float *g1d, int L, int lane, int row0, int col0,
-                                                   bool diagonal) {
-  const int nat = kQ * L;
+__device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb,
+                                                   const BwdArgs &args, int lane, int row0,
+                                                   int col0, bool diagonal) {
+  const int L = args.L, nat = kQ * L;
+  float *g2 = args.g2;
   const int row = row0 + lane;
   const long long pitch = (long long)kQPad * L;
-  const bool vec = (reinterpret_cast<uintptr_t>(g2) & 15) == 0;
+  auto single = [&](int v, float data) {  // g1 entry v (below 20 L) from its data term
+    args.g1d[v] = data;
+    args.fin.g1[v] = data + 2.0f * args.fin.lambda_single * args.fin.x1[v];
+  };
   if (SYM) {
     // the ones slot's column: the single-field gradient
     if (col0 <= nat && nat < col0 + 128) {
       float v = 0.0f;
 #pragma unroll
       for (int i = 0; i < 128; ++i) v = i == nat - col0 ? acc[i] : v;
-      if (row < (kQ - 1) * L) g1d[row] = v;
+      if (row < (kQ - 1) * L) single(row, v);
     }
     // columns of the same alignment column as this row
     int self = (row - col0) % L;
@@ -145,7 +150,7 @@ __device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb,
     if (row == nat) {
 #pragma unroll
       for (int i = 0; i < 128; ++i)
-        if (col0 + i < (kQ - 1) * L) g1d[col0 + i] = acc[i];
+        if (col0 + i < (kQ - 1) * L) single(col0 + i, acc[i]);
     }
   }
   if (col0 + 128 > nat) {
@@ -176,7 +181,7 @@ __device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb,
       // (a 16-byte group that straddles 21 L adds zeros to a padding state)
       const bool in = row0 + r < nat && col0 + cb * 16 + 4 * (lane & 3) < nat;
       float *p = d + (row0 + r) * pitch + cb * 16;
-      if (vec) {
+      if (args.vec) {
         red_add4_if(p, v, in);
       } else {
         red_add_if(p, v.x, in);

@@ -69,13 +69,37 @@ struct I8SpMaps {
   CUtensorMap b[3];      // digits of W: 12 KB tiles (128 K rows x 96 slots), box 256 x 48
 };
 
+// Sparse path: one pass over x (column maxima, sum of squares, regulariser gradient, step).
+struct I8ScanArgs {
+  const float *x, *s;    // full vectors; s: the CG direction, with alpha and xt (STEP)
+  const double *alpha;
+  float *xt;
+  uint32_t *cmacc;       // column maxima as float bits, zero at the start
+  double *part_reg;      // one partial of sum x2^2 per block
+  float *g2;
+  ccm_result *out;       // cleared
+  long long nsp;
+  int L, rows_per_block;
+  int cols;              // elements of a row: 32 L, or 21 L (padding skipped)
+  int vec;               // every vector is 16-byte aligned
+  float g2_scale;        // g2 = g2_scale * x
+};
+
+// Sparse path: digits of W.
+struct I8DigitsArgs {
+  const float *x2;
+  const uint32_t *cmacc;
+  uint32_t *colmax;      // copy of cmacc for the forward
+  int8_t *wdig[3];
+  int L, T, KB, gpb, rows_per_block;
+};
+
 struct I8PrepArgs {
   int8_t *wdig[3];
   const uint32_t *colmax;  // per coupling column (a*L + j): max |W| as float bits
   const float *enc;        // per slot: the digit encoding factor 2^(21 - e), 0 for padding
   double *part_reg;
   int L, S;
-  int KB;  // sparse forward: K blocks of 128 rows (tiled digit layout)
   float inv_L;
   float lambda_pair;
   float g2_coef;
@@ -126,17 +150,6 @@ struct FwdArgs {
   int L, N, S, T, Npad, m_tiles;
 };
 
-struct BwdArgs {
-  const float *x2;
-  float *g2;
-  float *g1d;
-  const int2 *tiles;
-  int *status;
-  int n_tiles, L, S, Npad;
-  float lambda_pair;
-  float r_dec;  // integer path: 2^(eR - 21), the inverse of I8FwdArgs::r_enc
-};
-
 struct FinalizeArgs {
   const double *part_f;
   long long n_part_f;
@@ -152,6 +165,22 @@ struct FinalizeArgs {
   double *block_part;  // kFinBlocks x 3 sums
   unsigned *done;      // blocks finished (0 between evaluations)
 };
+
+struct BwdArgs {
+  const float *x2;
+  float *g2;
+  float *g1d;
+  const int2 *tiles;
+  int *status;
+  int n_tiles, L, S, Npad;
+  float lambda_pair;
+  float r_dec;  // integer path: 2^(eR - 21), the inverse of I8FwdArgs::r_enc
+  // sparse path: g2 is 16-byte aligned; cmacc is cleared; fin: the sums of f, and g1
+  int vec;
+  uint32_t *cmacc;
+  FinalizeArgs fin;
+};
+
 constexpr int kFinBlocks = 16, kFinThreads = 512;
 
 // Per-kernel CUDA-event timing of evaluations (ccm_profile_begin/end): one
@@ -190,6 +219,7 @@ cudaError_t i8_build_onehot(ccm_context *c);
 void i8nat_to_groups(const ccm_context *c, const uint8_t *nat, int mats, int mat, uint8_t *dst);
 cudaError_t i8sp_forward_max_pairs(int *pairs);
 // tc_finalize over the loss partials of n_fwd_tiles 128-row forward tiles.
+FinalizeArgs finalize_args(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles);
 cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles);
 // One CG trial on a tensor-core context: xt = x + alpha s (alpha on the device),
 // then the evaluation at xt, with the step fused into tc_prep.
@@ -291,7 +321,10 @@ struct ccm_context {
   uint8_t *d_o1 = nullptr, *d_o128 = nullptr;          // Npad x S one-hot, values 1 / 128
   int8_t *d_wdig[3] = {nullptr, nullptr, nullptr};     // S x S digits of W
   int8_t *d_rdig[3] = {nullptr, nullptr, nullptr};     // Npad x S digits of R
-  uint32_t *d_colmax = nullptr;  // 21 L column maxima of |W|, then S per-slot encoding factors
+  // 21 L column maxima of |W| (dense path: then S per-slot encoding factors); sparse
+  // path: cmacc accumulates them and is zero between evaluations
+  uint32_t *d_colmax = nullptr, *d_cmacc = nullptr;
+  int n_part_reg = 0;  // sparse path: regulariser partials of the last evaluation
   // the column-maximum and prep passes skip the padding states a >= 21 (set by a
   // device-side solve whose x0 has zero padding states, while it captures and
   // runs; ccm_debug_set_cg_skip_padding clears cg_skip_padding to forbid it)

@@ -791,11 +791,17 @@ __global__ void __launch_bounds__(kFinThreads) tc_finalize_kernel(FinalizeArgs a
     last = atomicAdd(args.done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
+  if (!last) return;
+  __shared__ double parts[3 * kFinBlocks];
+  if (threadIdx.x < 3 * gridDim.x) {
     __threadfence();
+    parts[threadIdx.x] = __ldcg(args.block_part + threadIdx.x);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     double s[3] = {0.0, 0.0, 0.0};
     for (int b = 0; b < (int)gridDim.x; ++b)
-      for (int k = 0; k < 3; ++k) s[k] += __ldcg(args.block_part + 3 * b + k);
+      for (int k = 0; k < 3; ++k) s[k] += parts[3 * b + k];
     const double F = s[0], R2 = s[1], R1 = s[2];
     const double fx = F + (double)args.lambda_single * R1 + 0.5 * (double)args.lambda_pair * R2;
     args.out->fx = fx;
@@ -864,14 +870,19 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   return cudaGetLastError();
 }
 
-cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles) {
+FinalizeArgs finalize_args(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles) {
   FinalizeArgs za{};
   za.part_f = c->d_part_f; za.n_part_f = n_fwd_tiles * 8;
   za.part_reg = c->d_part_reg; za.n_part_reg = (long long)kQ * c->L;
   za.x1 = x1; za.g1d = c->d_g1d; za.g1 = d_g; za.L = c->L; za.nsp = c->nsp;
   za.lambda_single = c->lambda_single; za.lambda_pair = c->lambda_pair; za.out = c->d_out;
   za.block_part = c->d_fin_part; za.done = c->d_fin_done;
-  return launch_pdl(tc_finalize_kernel, dim3(kFinBlocks), dim3(kFinThreads), 0, c->stream, za);
+  return za;
+}
+
+cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles) {
+  return launch_pdl(tc_finalize_kernel, dim3(kFinBlocks), dim3(kFinThreads), 0, c->stream,
+                    finalize_args(c, x1, d_g, n_fwd_tiles));
 }
 
 cudaError_t tc_backward_max_pairs(int nsplit, int *pairs) {

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) i8_colmax_kernel(const float *__restrict_
                                                         float *__restrict__ xt,
                                                         uint32_t *__restrict__ colmax, int L,
                                                         long long nsp, int rows_per_block,
-                                                        int krow_order, int cols) {
+                                                        int cols) {
   griddep_wait();
   griddep_launch();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,11 +93,9 @@ __global__ void __launch_bounds__(256) i8_colmax_kernel(const float *__restrict_
   const int r1 = min(r0 + rows_per_block, kQ * L);
   float m = 0.0f;
   for (int r = r0; r < r1; ++r) {
-    // rows in the reverse of the order in which prep reads them (plain row order, or
-    // the sparse path's K-row order k * 21 + b), so that prep's first rows are the
-    // ones read last here and are still in L2
-    const int rr = kQ * L - 1 - r;
-    const int row = krow_order ? (rr % kQ) * L + rr / kQ : rr;
+    // rows in the reverse of the order in which prep reads them, so that prep's first
+    // rows are the ones read last here and are still in L2
+    const int row = kQ * L - 1 - r;
     const long long i = nsp + (long long)row * w32 + c;
     float v = x[i];
     if (STEP) {
@@ -109,12 +107,12 @@ __global__ void __launch_bounds__(256) i8_colmax_kernel(const float *__restrict_
   if (c < kQ * L && m > 0.0f) atomicMax(colmax + c, __float_as_uint(m));
 }
 
-// Per slot s (of the slot groups G): the encoding factor 2^(21 - e) of the digits
+// Per slot s of the dense path: the encoding factor 2^(21 - e) of the digits
 // of its coupling column (e the column's exponent, from the maxima above), 0 for
 // padding slots; read by prep.
-template <class G>
 __global__ void i8_scales_kernel(const uint32_t *__restrict__ colmax, float *__restrict__ enc,
                                  int L, int S) {
+  using G = Groups256;
   griddep_wait();
   griddep_launch();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -158,25 +156,198 @@ __host__ __device__ constexpr long long i8sp_b_offset(int kr, int s, int KB) {
          ((((x >> 4) ^ (r >> 2)) & 1) << 4) + (x & 15);
 }
 
+// ---------------------------------------------------------------- scan and digits
+// The sparse path's first two kernels.
+//
+// i8sp_scan_kernel, one pass over x (row blocks of its 21 L coupling rows, four columns
+// per thread, eight rows of loads in flight): column maxima of |W| into cmacc (float
+// bits, atomicMax; zero between evaluations), sum x^2 partials (four squares in float,
+// added in FP64), the regulariser gradient g2 <- g2_scale * x2 (the backward adds C to
+// it), and, STEP, the CG trial step v = fmaf(alpha, s, x) into xt (the last row of
+// blocks steps the single fields).  It also clears the result record.
+// Rows go in K-row order k * 21 + b backwards, so that the digits kernel's first rows
+// are the ones read last here and are still in L2.  HBM-bound.  Together with the
+// digits kernel 108 us at L = 253, N = 7001 and 151 us at L = 300; the column-maximum,
+// factor and row-per-block digit kernels before them took 226 us (scalar loads where
+// 4 does not divide L) and 165 us.  (The backward writing g2_scale * x2 + C itself, or
+// filling g2 while its MMAs run, saves this kernel 20 us at L = 300 and costs the
+// backward 20-60: its loads and stores share the L2 port with the operand stream.)
+template <bool STEP>
+__global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
+  griddep_wait();
+  griddep_launch();
+  const int L = args.L, nreal = kQ * L;
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+  float alpha = 0.0f;
+  if (STEP) {
+    alpha = (float)args.alpha[0];
+    if (blockIdx.y == gridDim.y - 1) {
+      for (long long i = blockIdx.x * 256 + threadIdx.x; i < args.nsp; i += gridDim.x * 256LL)
+        args.xt[i] = fmaf(alpha, args.s[i], args.x[i]);
+      return;
+    }
+  }
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(ccm_result) / 4)
+    reinterpret_cast<uint32_t *>(args.out)[threadIdx.x] = 0u;
+  float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  double acc = 0.0;
+  if (c < args.cols) {
+    // (cols = 21 L: the group that straddles 21 L reaches up to three padding states,
+    // which are zero then)
+    const float *x2 = args.x + args.nsp + c;
+    auto load = [&](const float *p) {
+      return args.vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+    };
+    auto store = [&](float *p, float4 v) {
+      if (args.vec) *reinterpret_cast<float4 *>(p) = v;
+      else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+    };
+    const int r0 = blockIdx.y * args.rows_per_block;
+    const int r1 = min(r0 + args.rows_per_block, nreal);
+    constexpr int kU = STEP ? 4 : 8;
+    for (int r = r0; r < r1; r += kU) {
+      float4 v[kU], sv[STEP ? kU : 1];
+      long long at[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int rr = nreal - 1 - min(r + u, r1 - 1);
+        at[u] = ((long long)(rr % kQ) * L + rr / kQ) * kQPad * L;
+        v[u] = load(x2 + at[u]);
+        if (STEP) sv[u] = load(args.s + args.nsp + c + at[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (r + u >= r1) break;
+        if (STEP) {
+          v[u] = make_float4(fmaf(alpha, sv[u].x, v[u].x), fmaf(alpha, sv[u].y, v[u].y),
+                             fmaf(alpha, sv[u].z, v[u].z), fmaf(alpha, sv[u].w, v[u].w));
+          store(args.xt + args.nsp + c + at[u], v[u]);
+        }
+        acc += (double)fmaf(v[u].w, v[u].w, fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
+        m[0] = fmaxf(m[0], fabsf(v[u].x));
+        m[1] = fmaxf(m[1], fabsf(v[u].y));
+        m[2] = fmaxf(m[2], fabsf(v[u].z));
+        m[3] = fmaxf(m[3], fabsf(v[u].w));
+        const float k = args.g2_scale;
+        store(args.g2 + at[u] + c, make_float4(k * v[u].x, k * v[u].y, k * v[u].z, k * v[u].w));
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (c + e < nreal && m[e] > 0.0f) atomicMax(args.cmacc + c + e, __float_as_uint(m[e]));
+  }
+  __shared__ double red[8];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int w = 0; w < 8; ++w) sum += red[w];
+    args.part_reg[blockIdx.y * gridDim.x + blockIdx.x] = sum;
+  }
+}
+
+// i8sp_digits_kernel: the three digits of W in the forward's tiled storage
+// (i8sp_b_offset).  A block takes `gpb` slot groups (9 gpb alignment columns with their
+// 21 states) and a run of K rows, eight rows at a time: a thread's elements are the
+// same columns of every row, so that their index arithmetic and encoding factors are
+// computed once; consecutive threads read runs of 9 gpb floats.  The fixed-point
+// integers go through shared memory in slot order (groups 200 words apart, rows an odd
+// multiple of 4 words apart modulo 32: no bank conflict), and 16 consecutive threads
+// write 256 contiguous bytes of a tile.  The first row of blocks also copies the column
+// maxima to `colmax`, which the forward reads: cmacc is cleared by the backward.
+constexpr int kDigThreads = 384, kDigRows = 8, kDigGroups = 8, kDigGroupWords = 200;
+constexpr int dig_row_words(int gpb) { return (gpb * kDigGroupWords + 31) / 32 * 32 + 4; }
+__global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs args) {
+  extern __shared__ __align__(16) int qs[];  // kDigRows rows of dig_row_words(gpb)
+  griddep_wait();
+  griddep_launch();
+  constexpr int kE = (kDigGroups * Groups192::kUsed + kDigThreads - 1) / kDigThreads;
+  const int L = args.L, gpb = args.gpb, cols = gpb * Groups192::kCols;
+  const int t0 = blockIdx.x * gpb, j0 = t0 * Groups192::kCols;
+  const int row_words = dig_row_words(gpb);
+  int off[kE], slot[kE];
+  float enc[kE];
+#pragma unroll
+  for (int u = 0; u < kE; ++u) {
+    const int e = threadIdx.x + u * kDigThreads;
+    const int a = e / cols, jj = e % cols, j = j0 + jj;
+    off[u] = -1;
+    slot[u] = 0;
+    enc[u] = 0.0f;
+    if (a < kQ && j < L) {
+      off[u] = a * L + j;
+      slot[u] = jj / Groups192::kCols * kDigGroupWords + a * Groups192::kCols + jj % Groups192::kCols;
+      const uint32_t m = args.cmacc[off[u]];
+      enc[u] = pow2f(kI8FracBits - col_exponent(m));
+      if (blockIdx.y == 0) args.colmax[off[u]] = m;
+    }
+  }
+  // padding slots of the groups stay zero
+  for (int i = threadIdx.x; i < kDigRows * row_words; i += kDigThreads) qs[i] = 0;
+  const int k_rows = kQ * L;
+  const int r1 = min((int)(blockIdx.y + 1) * args.rows_per_block, k_rows);
+  for (int r0 = blockIdx.y * args.rows_per_block; r0 < r1; r0 += kDigRows) {
+    float v[kDigRows][kE];
+#pragma unroll
+    for (int i = 0; i < kDigRows; ++i) {
+      const int kr = min(r0 + i, r1 - 1);
+      const float *row = args.x2 + ((long long)(kr % kQ) * L + kr / kQ) * kQPad * L;
+#pragma unroll
+      for (int u = 0; u < kE; ++u) v[i][u] = off[u] >= 0 ? row[off[u]] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kDigRows; ++i)
+#pragma unroll
+      for (int u = 0; u < kE; ++u)
+        if (off[u] >= 0) {
+          const int q = __float2int_rn(v[i][u] * enc[u]);  // exact scaling
+          qs[i * row_words + slot[u]] = min(max(q, -(1 << kI8FracBits)), (1 << kI8FracBits) - 1);
+        }
+    __syncthreads();
+    // 16 slots of one row per thread: chunk (group, 32-slot atom), row, half
+    const int chunks = gpb * 6 * 2 * kDigRows;
+    for (int u = threadIdx.x; u < chunks; u += kDigThreads) {
+      const int hc = u & 1, i = (u >> 1) & (kDigRows - 1), ga = u / (2 * kDigRows);
+      const int g = ga / 6, c = ga % 6 * 32 + hc * 16;
+      if (r0 + i >= r1 || t0 + g >= args.T) continue;
+      const int *from = qs + i * row_words + g * kDigGroupWords + c;
+      uint32_t p0[4], p1[4], p2[4];
+#pragma unroll
+      for (int e4 = 0; e4 < 4; ++e4) {
+        const int4 qv = *reinterpret_cast<const int4 *>(from + e4 * 4);
+        // byte e of each word = digit of element e (as in the dense forward's R digits)
+        auto pack = [](int b0, int b1, int b2, int b3) {
+          return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+        };
+        p0[e4] = pack(qv.x >> 14, qv.y >> 14, qv.z >> 14, qv.w >> 14);
+        p1[e4] = pack(qv.x >> 7, qv.y >> 7, qv.z >> 7, qv.w >> 7) & 0x7F7F7F7Fu;
+        p2[e4] = pack(qv.x, qv.y, qv.z, qv.w) & 0x7F7F7F7Fu;
+      }
+      const long long at = i8sp_b_offset(r0 + i, (t0 + g) * Groups192::kSlots + c, args.KB);
+      *reinterpret_cast<uint4 *>(args.wdig[0] + at) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+      *reinterpret_cast<uint4 *>(args.wdig[1] + at) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+      *reinterpret_cast<uint4 *>(args.wdig[2] + at) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- prep
-// One block per row (b, k) of W, as tc_prep: g2 <- g2_coef * lambda2 * x, the FP64
-// partial of sum x^2, and one row of the three digit matrices of W (16 slots per
-// thread, one 16-byte store per digit matrix).  Columns are the slots of the
-// groups G; the row is s(b, k) (NAT = false: Wperm, both sides permuted) or
-// K row k * 21 + b of the sparse forward (NAT = true, alignment column major,
-// stored in its tiled layout).  args.S is the row length.  The row is staged in shared memory in slot order,
-// so that the digit pass reads 16 consecutive slots per thread (vector loads, no
-// index arithmetic) with their per-slot factors.
-template <class G, bool NAT>
+// The dense path's preparation.  One block per row (b, k) of W, as tc_prep: g2 <-
+// g2_coef * lambda2 * x, the FP64 partial of sum x^2, and row s(b, k) of the three digit
+// matrices of Wperm (16 slots per thread, one 16-byte store per digit matrix).  args.S
+// is the row length.  The row is staged in shared memory in slot order, so that the
+// digit pass reads 16 consecutive slots per thread (vector loads, no index arithmetic)
+// with their per-slot factors.
 __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ x2,
                                                       float *__restrict__ g2, I8PrepArgs args) {
   griddep_wait();
   griddep_launch();
   extern __shared__ __align__(16) float xrow[];  // S floats: the row in slot order
   const int L = args.L;
-  // NAT: blocks in K-row order k * 21 + b, so that blocks running together fill
-  // neighbouring rows of the same stored tiles
-  const int row = NAT ? (int)(blockIdx.x % kQ) * L + (int)(blockIdx.x / kQ) : (int)blockIdx.x;
+  using G = Groups256;
+  const int row = blockIdx.x;
   const int b = row / L, k = row % L;
   const long long base = (long long)row * kQPad * L;
   const float two_l2 = args.g2_coef * args.lambda_pair;
@@ -225,7 +396,7 @@ __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ 
     }
   }
   __syncthreads();
-  const long long srow = (long long)G::slot_of(b, k) * args.S;  // (NAT: tiled, i8sp_b_offset)
+  const long long srow = (long long)G::slot_of(b, k) * args.S;
   for (int u = threadIdx.x; u < args.S / 16; u += blockDim.x) {
     uint32_t p0[4], p1[4], p2[4];
 #pragma unroll
@@ -248,7 +419,7 @@ __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ 
       p1[e4] = pack(qv[0] >> 7, qv[1] >> 7, qv[2] >> 7, qv[3] >> 7) & 0x7F7F7F7Fu;
       p2[e4] = pack(qv[0], qv[1], qv[2], qv[3]) & 0x7F7F7F7Fu;
     }
-    const long long off = NAT ? i8sp_b_offset(k * kQ + b, u * 16, args.KB) : srow + (long long)u * 16;
+    const long long off = srow + (long long)u * 16;
     *reinterpret_cast<uint4 *>(args.wdig[0] + off) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
     *reinterpret_cast<uint4 *>(args.wdig[1] + off) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
     *reinterpret_cast<uint4 *>(args.wdig[2] + off) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
@@ -1226,6 +1397,42 @@ struct I8BwdSmem {
 // NAT: natural slots, K-major operands in the storage of i8nat_offset (the sparse
 // path); else Groups256 slots, row-major Npad x S operands (MN-major).  The MMAs run
 // at the same rate either way.
+// fx = sum(loss partials) + lambda1 sum V^2 + 0.5 lambda2 sum x2^2 in FP64, in a fixed
+// order, and the padding of g1 (the backward's output phase writes g1 itself); one warp.
+__device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, int lane) {
+  auto sum = [&](const double *p, long long n) {
+    double s = 0.0;
+    for (long long i0 = lane; i0 < n; i0 += 8 * 32) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + 32 * u < n ? p[i0 + 32 * u] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    return s;
+  };
+  const int ns = (int)nsingle_of(args.L);
+  double acc[3] = {sum(args.part_f, args.n_part_f), sum(args.part_reg, args.n_part_reg), 0.0};
+  for (int i0 = lane; i0 < ns; i0 += 16 * 32) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = i0 + 32 * u < ns ? args.x1[i0 + 32 * u] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) acc[2] += (double)v[u] * (double)v[u];
+  }
+  for (long long i = ns + lane; i < args.nsp; i += 32) args.g1[i] = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+  if (lane == 0) {
+    const double F = acc[0];
+    const double fx = F + (double)args.lambda_single * acc[2] + 0.5 * (double)args.lambda_pair * acc[1];
+    args.out->fx = fx;
+    args.out->f_data = F;
+    args.out->reg = fx - F;
+  }
+}
+
 template <bool SYM, bool NAT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8_backward_kernel(const __grid_constant__ I8BwdMaps maps, BwdArgs args) {
@@ -1376,6 +1583,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       umma_commit_pair(drain, 0x1);
       if (!mbar_wait(drain, 0)) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
     }
+  } else if (NAT && warp == 2) {
+    // the sums of the loss and regulariser partials, while the MMAs run
+    if (blockIdx.x == 0) i8nat_finalize(args.fin, lane);
+  } else if (NAT && warp == 3) {
+    // the column maxima's accumulator, for the next evaluation's scan
+    if (blockIdx.x == 0)
+      for (int i = lane; i < kQ * args.L; i += 32) args.cmacc[i] = 0u;
   } else if (warp >= 4) {
     reg_inc<kWgRegsEpi>();
     // Epilogue: each K chunk merged from the two integer accumulators (16 columns
@@ -1430,7 +1644,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       const int2 pq = args.tiles[tile];
       const int s1 = pq.x * kPairM + (int)rank * kBM + q * 32, s2 = pq.y * kBN + half * kHalfN;
       if constexpr (NAT)
-        bwd_output_natural<SYM>(accv, Tb, args.g2, args.g1d, args.L, lane, s1, s2, pq.x == pq.y);
+        bwd_output_natural<SYM>(accv, Tb, args, lane, s1, s2, pq.x == pq.y);
       else
         bwd_output<Groups256, SYM>(accv, Tb, args.g2, args.g1d, args.L, lane, s1, s2);
     }
@@ -1453,56 +1667,100 @@ namespace ccm {
 // Evaluation at d_x, or, with d_s, at d_xt = d_x + alpha d_s (the step is taken
 // by the column-max pass, which writes d_xt).  Profile marks: [colmax + prep |
 // forward | backward | finalize].
-cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
-                        const double *d_alpha, float *d_xt) {
+static cudaError_t i8_prepare_dense(ccm_context *c, const float *d_x, float *g2, const float *d_s,
+                                    const double *d_alpha, float *d_xt) {
   const int L = c->L;
   const bool step = d_s != nullptr;
-  const bool sp = c->path == CCM_PATH_TC_I8SP;
-  const float *xe = step ? d_xt : d_x;
-  const float *x1 = xe;
-  const float *x2 = xe + c->nsp;
-  float *g2 = d_g + c->nsp;
+  const float *x2 = (step ? d_xt : d_x) + c->nsp;
   cudaError_t e;
-
-  prof_mark(c);
   if ((e = zero_words(c->d_colmax, (long long)kQ * L, c->stream)) != cudaSuccess) return e;
   constexpr int kRows = 32;
   const int cols = (c->skip_padding ? kQ : kQPad) * L;
   const dim3 cgrid((cols + 255) / 256, (kQ * L + kRows - 1) / kRows + (step ? 1 : 0));
   if (step)
     e = launch_pdl(i8_colmax_kernel<true>, cgrid, dim3(256), 0, c->stream, d_x, d_s, d_alpha, d_xt,
-                   c->d_colmax, L, c->nsp, kRows, sp ? 1 : 0, cols);
+                   c->d_colmax, L, c->nsp, kRows, cols);
   else
     e = launch_pdl(i8_colmax_kernel<false>, cgrid, dim3(256), 0, c->stream, d_x,
                    (const float *)nullptr, (const double *)nullptr, (float *)nullptr, c->d_colmax,
-                   L, c->nsp, kRows, sp ? 1 : 0, cols);
+                   L, c->nsp, kRows, cols);
   if (e != cudaSuccess) return e;
   // per-slot factors after the column maxima, 16-byte aligned for the float4 loads
   float *enc = reinterpret_cast<float *>(c->d_colmax + ((kQ * L + 3) & ~3));
-  // W digit rows: S slots (dense forward) or SW slots of 192-slot groups (sparse)
-  const int wcols = sp ? c->SW : c->S;
-  if (sp)
-    e = launch_pdl(i8_scales_kernel<Groups192>, dim3((wcols + 255) / 256), dim3(256), 0, c->stream,
-                   (const uint32_t *)c->d_colmax, enc, L, wcols);
-  else
-    e = launch_pdl(i8_scales_kernel<Groups256>, dim3((wcols + 255) / 256), dim3(256), 0, c->stream,
-                   (const uint32_t *)c->d_colmax, enc, L, wcols);
+  e = launch_pdl(i8_scales_kernel, dim3((c->S + 255) / 256), dim3(256), 0, c->stream,
+                 (const uint32_t *)c->d_colmax, enc, L, c->S);
   if (e != cudaSuccess) return e;
   I8PrepArgs pa{};
   for (int i = 0; i < 3; ++i) pa.wdig[i] = c->d_wdig[i];
   pa.colmax = c->d_colmax;
   pa.enc = enc;
   pa.part_reg = c->d_part_reg;
-  pa.L = L; pa.S = wcols; pa.KB = c->KP / 128; pa.lambda_pair = c->lambda_pair;
+  pa.L = L; pa.S = c->S; pa.lambda_pair = c->lambda_pair;
   pa.g2_coef = c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f;
   pa.inv_L = 1.0f / (float)L;
   pa.ncols = cols;
-  if (sp)
-    e = launch_pdl(i8_prep_kernel<Groups192, true>, dim3(kQ * L), dim3(256), sizeof(float) * wcols,
-                   c->stream, x2, g2, pa);
-  else
-    e = launch_pdl(i8_prep_kernel<Groups256, false>, dim3(kQ * L), dim3(256), sizeof(float) * wcols,
-                   c->stream, x2, g2, pa);
+  count_launch(c, 4);
+  return launch_pdl(i8_prep_kernel, dim3(kQ * L), dim3(256), sizeof(float) * c->S, c->stream, x2, g2,
+                    pa);
+}
+
+// Rows of a scan block and of a digits block: enough blocks to fill the chip a few
+// times over, few enough that a block's set-up and its column maxima's atomics stay
+// small beside its rows.
+static int scan_rows(int L, int col_blocks) {
+  const int want = 8 * 148 / col_blocks;  // row blocks
+  const int rows = (kQ * L + want - 1) / want;
+  return rows < 16 ? 16 : rows > 64 ? 64 : (rows + 7) / 8 * 8;
+}
+
+static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2, const float *d_s,
+                                     const double *d_alpha, float *d_xt) {
+  const int L = c->L;
+  const bool step = d_s != nullptr;
+  const float *xe = step ? d_xt : d_x;
+  I8ScanArgs sa{};
+  sa.x = d_x; sa.s = d_s; sa.alpha = d_alpha; sa.xt = d_xt;
+  sa.cmacc = c->d_cmacc; sa.part_reg = c->d_part_reg; sa.g2 = g2; sa.out = c->d_out;
+  sa.nsp = c->nsp; sa.L = L;
+  sa.cols = (c->skip_padding ? kQ : kQPad) * L;
+  sa.g2_scale = (c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f) * c->lambda_pair;
+  auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
+  sa.vec = ((bits(d_x) | bits(d_s) | bits(d_xt) | bits(g2)) & 15) == 0;
+  const int cb = (sa.cols + 1023) / 1024;
+  sa.rows_per_block = scan_rows(L, cb);
+  const int rb = (kQ * L + sa.rows_per_block - 1) / sa.rows_per_block;
+  c->n_part_reg = cb * rb;
+  cudaError_t e = launch_pdl(step ? i8sp_scan_kernel<true> : i8sp_scan_kernel<false>,
+                             dim3(cb, rb + (step ? 1 : 0)), dim3(256), 0, c->stream, sa);
+  if (e != cudaSuccess) return e;
+
+  I8DigitsArgs da{};
+  for (int i = 0; i < 3; ++i) da.wdig[i] = c->d_wdig[i];
+  da.x2 = xe + c->nsp; da.cmacc = c->d_cmacc; da.colmax = c->d_colmax;
+  da.L = L; da.T = c->T; da.KB = c->KP / 128;
+  const int gb = (c->T + kDigGroups - 1) / kDigGroups;  // blocks along the groups, evenly filled
+  da.gpb = (c->T + gb - 1) / gb;
+  const int row_tiles = (kQ * L + kDigRows - 1) / kDigRows;
+  const int per = (row_tiles * gb + 8 * 148 - 1) / (8 * 148);
+  da.rows_per_block = kDigRows * (per < 4 ? per : 4);
+  count_launch(c, 2);
+  return launch_pdl(i8sp_digits_kernel,
+                    dim3(gb, (kQ * L + da.rows_per_block - 1) / da.rows_per_block),
+                    dim3(kDigThreads), sizeof(int) * kDigRows * dig_row_words(da.gpb), c->stream, da);
+}
+
+cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
+                        const double *d_alpha, float *d_xt) {
+  const int L = c->L;
+  const bool sp = c->path == CCM_PATH_TC_I8SP;
+  const float *x1 = d_s != nullptr ? d_xt : d_x;
+  const float *x2 = x1 + c->nsp;
+  float *g2 = d_g + c->nsp;
+  cudaError_t e;
+
+  prof_mark(c);
+  e = sp ? i8_prepare_sparse(c, d_x, g2, d_s, d_alpha, d_xt)
+         : i8_prepare_dense(c, d_x, g2, d_s, d_alpha, d_xt);
   if (e != cudaSuccess) return e;
   prof_mark(c);
 
@@ -1534,6 +1792,13 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   ba.r_dec = pow2_host(c->r_exp - kI8FracBits);
   const int bpairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
   const bool sym = c->gradient != CCM_GRADIENT_PARTIAL;
+  if (sp) {
+    // the sums and g1 are the backward's own (no finalize)
+    ba.cmacc = c->d_cmacc;
+    ba.vec = (reinterpret_cast<uintptr_t>(g2) & 15) == 0;
+    ba.fin = finalize_args(c, x1, d_g, 2LL * pair_tiles);
+    ba.fin.n_part_reg = c->n_part_reg;
+  }
   const dim3 bgrid(2 * bpairs);
   auto bwd = sp && sym ? i8_backward_kernel<true, true>
              : sp        ? i8_backward_kernel<false, true>
@@ -1543,9 +1808,9 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   if (e != cudaSuccess) return e;
   prof_mark(c);
 
-  if ((e = launch_tc_finalize(c, x1, d_g, 2LL * pair_tiles)) != cudaSuccess) return e;
+  if (!sp && (e = launch_tc_finalize(c, x1, d_g, 2LL * pair_tiles)) != cudaSuccess) return e;
   prof_mark(c);
-  count_launch(c, 7);
+  count_launch(c, sp ? 2 : 3);
   return cudaGetLastError();
 }
 
@@ -1554,10 +1819,9 @@ cudaError_t i8_configure_kernels() {
   const int kMax = cudaFuncAttributeMaxDynamicSharedMemorySize;
   // the staged row is S floats: up to L = 2688 (the 227 KB per block, less the
   // kernel's static reduction buffer)
-  if ((e = cudaFuncSetAttribute(i8_prep_kernel<Groups256, false>, (cudaFuncAttribute)kMax,
-                                230000)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8_prep_kernel<Groups192, true>, (cudaFuncAttribute)kMax,
-                                230000)) != cudaSuccess)
+  if ((e = cudaFuncSetAttribute(i8_prep_kernel, (cudaFuncAttribute)kMax, 230000)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(i8sp_digits_kernel, (cudaFuncAttribute)kMax,
+                                (int)sizeof(int) * kDigRows * dig_row_words(kDigGroups))) != cudaSuccess)
     return e;
   if ((e = cudaFuncSetAttribute(i8_forward_kernel, (cudaFuncAttribute)kMax, I8FwdSmem::kTotal)) !=
           cudaSuccess ||
