@@ -144,6 +144,7 @@ SIGNATURES = {
                                              _f32p, ctypes.c_int]),
     "ccm_calculate_weights_noalloc": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int,
                                                      ctypes.c_float, _vp, _vp]),
+    "ccm_release_memory": (ctypes.c_int, [ctypes.c_int]),
     "ccm_last_error": (ctypes.c_char_p, []),
     "ccm_debug_copy": (ctypes.c_longlong, [_vp, ctypes.c_int, _vp, ctypes.c_longlong]),
     "ccm_profile_begin": (ctypes.c_int, [_vp, ctypes.c_int]),

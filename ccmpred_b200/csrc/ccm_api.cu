@@ -51,13 +51,105 @@ bool is_context(const void *p) {
   return p && static_cast<const ccm_context *>(p)->magic == kContextMagic;
 }
 
+// Device memory of the library comes from one pool per device.  The default pool gives
+// every block back to the system at each synchronisation and maps it again for the next
+// call: 0.4 ms for a few MB, 3 ms for 256 MB, at every create, solve and weights call.
+// This pool keeps up to kPoolKeep of freed memory mapped (everything while a batch
+// runs), reuses it across threads and streams in stream order, and gives it back when
+// an allocation fails and in ccm_release_memory.
+constexpr uint64_t kPoolKeep = 4ull << 30;
+static std::mutex pool_mutex;
+static cudaMemPool_t pools[64] = {nullptr};
+static int pool_batches[64] = {0};
+
+static void set_pool_keep(cudaMemPool_t pool, uint64_t bytes) {
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes);
+}
+
+cudaMemPool_t library_pool(int device) {
+  if (device < 0 || device >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(pool_mutex);
+  if (!pools[device]) {
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&pools[device], &props) != cudaSuccess) {
+      (void)cudaGetLastError();
+      pools[device] = nullptr;  // the default pool serves then
+      return nullptr;
+    }
+    set_pool_keep(pools[device], kPoolKeep);
+  }
+  return pools[device];
+}
+
+void pool_batch_begin(int device) {
+  cudaMemPool_t pool = library_pool(device);
+  if (!pool) return;
+  std::lock_guard<std::mutex> lock(pool_mutex);
+  if (pool_batches[device]++ == 0) set_pool_keep(pool, UINT64_MAX);
+}
+
+void pool_batch_end(int device) {
+  cudaMemPool_t pool = library_pool(device);
+  if (!pool) return;
+  std::lock_guard<std::mutex> lock(pool_mutex);
+  if (--pool_batches[device] > 0) return;
+  set_pool_keep(pool, kPoolKeep);
+  cudaMemPoolTrimTo(pool, kPoolKeep);
+}
+
+cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream) {
+  cudaMemPool_t pool = library_pool(device);
+  if (!pool) return cudaMallocAsync(p, bytes, stream);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    // kept blocks of other sizes may stand in the way
+    (void)cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  }
+  return e;
+}
+
 cudaError_t dev_alloc_raw(ccm_context *c, void **p, size_t bytes) {
   // the cap of ccm_options.mem_limit: the bytes this context holds
   if (c->mem_limit > 0 && c->mem_used + bytes > c->mem_limit) return cudaErrorMemoryAllocation;
-  const cudaError_t e = c->pool ? cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream)
-                                : cudaMallocAsync(p, bytes, c->stream);
+  const cudaError_t e = pool_alloc(c->device, p, bytes, c->stream);
   if (e == cudaSuccess) c->mem_used += bytes;
   return e;
+}
+
+// Non-blocking streams of calls that need one for their own duration: creating and
+// destroying one takes 0.1 ms.  At most kSpareStreams per device are kept.
+constexpr size_t kSpareStreams = 16;
+static std::mutex stream_mutex;
+static std::vector<cudaStream_t> spare_streams[64];
+
+cudaError_t acquire_stream(int device, cudaStream_t *s) {
+  if (device >= 0 && device < 64) {
+    std::lock_guard<std::mutex> lock(stream_mutex);
+    if (!spare_streams[device].empty()) {
+      *s = spare_streams[device].back();
+      spare_streams[device].pop_back();
+      return cudaSuccess;
+    }
+  }
+  return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+
+// Waits for `s`; a stream that reports an error is not kept.
+void release_stream(int device, cudaStream_t s) {
+  if (device >= 0 && device < 64 && cudaStreamSynchronize(s) == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(stream_mutex);
+    if (spare_streams[device].size() < kSpareStreams) {
+      spare_streams[device].push_back(s);
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
 }
 
 // Small pinned host records (a context's result, the CG's step scalars) come
@@ -223,17 +315,43 @@ cudaError_t dev_alloc(ccm_context *c, T **p, size_t bytes) {
   return dev_alloc_raw(c, reinterpret_cast<void **>(p), bytes);
 }
 
-bool configured[64] = {false};
+// Per device, found once: kernel attributes set, compute capability and SM count, and the
+// CTA pairs of the tensor-core kernels that can be resident (forward, backward) by path.
+// (cudaGetDeviceProperties, asked at every create before, takes 2.6 ms.)
+struct DeviceFacts {
+  bool known = false;
+  int major = 0, minor = 0, sms = 0;
+  int pairs[6][2] = {};  // [CCM_PATH_*][forward, backward]
+};
+DeviceFacts device_facts[64];
 std::mutex configure_mutex;
 
-int ensure_configured(int device) {
+int ensure_configured(int device, DeviceFacts *facts) {
   if (device < 0 || device >= 64) return set_error(CCM_ERR_INVALID, "bad device %d", device);
   std::lock_guard<std::mutex> lock(configure_mutex);
-  if (configured[device]) return CCM_OK;
-  CCM_CUDA_TRY(tc_configure_kernels());
-  CCM_CUDA_TRY(i8_configure_kernels());
-  CCM_CUDA_TRY(simt_configure_kernels());
-  configured[device] = true;
+  DeviceFacts &f = device_facts[device];
+  if (!f.known) {
+    CCM_CUDA_TRY(cudaDeviceGetAttribute(&f.major, cudaDevAttrComputeCapabilityMajor, device));
+    CCM_CUDA_TRY(cudaDeviceGetAttribute(&f.minor, cudaDevAttrComputeCapabilityMinor, device));
+    CCM_CUDA_TRY(cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, device));
+    if (f.major == 10) {
+      CCM_CUDA_TRY(tc_configure_kernels());
+      CCM_CUDA_TRY(i8_configure_kernels());
+      for (int ns = 2; ns <= 3; ++ns) {
+        int *p = f.pairs[ns == 2 ? CCM_PATH_TC_BF16X2 : CCM_PATH_TC_BF16X3];
+        CCM_CUDA_TRY(tc_forward_max_pairs(ns, &p[0]));
+        CCM_CUDA_TRY(tc_backward_max_pairs(ns, &p[1]));
+      }
+      int b = 0;
+      CCM_CUDA_TRY(i8_backward_max_pairs(&b));
+      CCM_CUDA_TRY(i8_forward_max_pairs(&f.pairs[CCM_PATH_TC_I8X3][0]));
+      CCM_CUDA_TRY(i8sp_forward_max_pairs(&f.pairs[CCM_PATH_TC_I8SP][0]));
+      f.pairs[CCM_PATH_TC_I8X3][1] = f.pairs[CCM_PATH_TC_I8SP][1] = b;
+    }
+    CCM_CUDA_TRY(simt_configure_kernels());
+    f.known = true;
+  }
+  *facts = f;
   return CCM_OK;
 }
 
@@ -526,7 +644,7 @@ int init_backend(ccm_userdata *ud) {
 }  // namespace
 
 int ccm::create_context(ccm_context **out, const unsigned char *msa, int ncol, int nrow,
-                        const float *weights, const ccm_options *opt, cudaMemPool_t pool) {
+                        const float *weights, const ccm_options *opt) {
   if (!out || !msa || ncol <= 0 || nrow <= 0)
     return set_error(CCM_ERR_INVALID, "ccm_create: invalid arguments");
   *out = nullptr;
@@ -536,7 +654,10 @@ int ccm::create_context(ccm_context **out, const unsigned char *msa, int ncol, i
     return set_error(CCM_ERR_INVALID, "ccm_create: unknown path %d", o.path);
   if (o.gradient != CCM_GRADIENT_TIED && o.gradient != CCM_GRADIENT_PARTIAL)
     return set_error(CCM_ERR_INVALID, "ccm_create: unknown gradient mode %d", o.gradient);
-  for (long long i = 0; i < (long long)ncol * nrow; ++i)
+  const long long cells = (long long)ncol * nrow;
+  unsigned char top = 0;
+  for (long long i = 0; i < cells; ++i) top = std::max(top, msa[i]);
+  for (long long i = 0; top > 20 && i < cells; ++i)
     if (msa[i] > 20) return set_error(CCM_ERR_INVALID, "ccm_create: MSA state %d > 20 at %lld", msa[i], i);
   // the integer paths encode R = w (P - onehot), |R| <= max |w|, with 21
   // fractional bits below the smallest power of two 2^eR >= max |w| (below 1 too:
@@ -560,33 +681,26 @@ int ccm::create_context(ccm_context **out, const unsigned char *msa, int ncol, i
     return set_error(CCM_ERR_INVALID, "ccm_create: L=%d exceeds the int nvar of the reference ABI", ncol);
 
   CCM_CUDA_TRY(cudaSetDevice(o.device));
-  cudaDeviceProp prop;
-  CCM_CUDA_TRY(cudaGetDeviceProperties(&prop, o.device));
+  DeviceFacts facts;
+  int rc = ensure_configured(o.device, &facts);
+  if (rc != CCM_OK) return rc;
   const bool tc_path = o.path == CCM_PATH_TC_BF16X2 || o.path == CCM_PATH_TC_BF16X3 ||
                        o.path == CCM_PATH_TC_I8X3 || o.path == CCM_PATH_TC_I8SP;
-  if (tc_path && prop.major != 10)
+  if (tc_path && facts.major != 10)
     return set_error(CCM_ERR_UNSUPPORTED, "tensor-core path needs an sm_100 device (found sm_%d%d)",
-                     prop.major, prop.minor);
-  int rc = ensure_configured(o.device);
-  if (rc != CCM_OK) return rc;
+                     facts.major, facts.minor);
 
   ccm_context *c = new ccm_context();
-  c->pool = pool;
   c->mem_limit = o.mem_limit;
   c->r_exp = r_exp;
   c->device = o.device;
-  c->num_sms = prop.multiProcessorCount;
+  c->num_sms = facts.sms;
   if (tc_path) {
-    const int ns = o.path == CCM_PATH_TC_BF16X3 ? 3 : 2;
-    const bool i8 = o.path == CCM_PATH_TC_I8X3 || o.path == CCM_PATH_TC_I8SP;
-    cudaError_t e = o.path == CCM_PATH_TC_I8SP ? i8sp_forward_max_pairs(&c->fwd_pairs)
-                    : i8                       ? i8_forward_max_pairs(&c->fwd_pairs)
-                                               : tc_forward_max_pairs(ns, &c->fwd_pairs);
-    if (e == cudaSuccess)
-      e = i8 ? i8_backward_max_pairs(&c->bwd_pairs) : tc_backward_max_pairs(ns, &c->bwd_pairs);
-    if (e != cudaSuccess || c->fwd_pairs < 1 || c->bwd_pairs < 1) {
+    c->fwd_pairs = facts.pairs[o.path][0];
+    c->bwd_pairs = facts.pairs[o.path][1];
+    if (c->fwd_pairs < 1 || c->bwd_pairs < 1) {
       delete c;
-      return set_error(CCM_ERR_CUDA, "tc_forward cluster occupancy: %s", cudaGetErrorString(e));
+      return set_error(CCM_ERR_CUDA, "no CTA pair of the tensor-core kernels fits the device");
     }
     if (o.max_sms > 0) {
       const int pairs = std::max(1, o.max_sms / 2);
@@ -658,6 +772,13 @@ extern "C" {
 
 const char *ccm_last_error(void) { return g_last_error; }
 
+int ccm_release_memory(int device) {
+  if (device < 0 || device >= 64) return set_error(CCM_ERR_INVALID, "ccm_release_memory: bad device %d", device);
+  std::lock_guard<std::mutex> lock(pool_mutex);
+  if (pools[device]) CCM_CUDA_TRY(cudaMemPoolTrimTo(pools[device], 0));
+  return CCM_OK;
+}
+
 void ccm_set_default_path(int path) { g_default_path = path; }
 
 long long ccm_nsingle_padded(int ncol) { return nsingle_padded_of(ncol); }
@@ -677,7 +798,7 @@ void ccm_options_default(ccm_options *opt, int ncol) {
 
 int ccm_create(ccm_context **out, const unsigned char *msa, int ncol, int nrow,
                const float *weights, const ccm_options *opt) {
-  return ccm::create_context(out, msa, ncol, nrow, weights, opt, nullptr);
+  return ccm::create_context(out, msa, ncol, nrow, weights, opt);
 }
 
 int ccm_destroy(ccm_context *ctx) {
@@ -986,22 +1107,21 @@ int ccm_calculate_weights(const unsigned char *msa, int ncol, int nrow, float th
   const float prod = threshold * (float)(uint64_t)ncol;
   const int idthres = (int)ceil((double)prod);
   cudaStream_t s;
-  CCM_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  CCM_CUDA_TRY(acquire_stream(device, &s));
+  // the alignment, then the counts and the weights
+  const size_t cells = ((size_t)ncol * nrow + 255) & ~(size_t)255;
   uint8_t *d_msa = nullptr;
-  int *d_cnt = nullptr;
-  float *d_w = nullptr;
-  cudaError_t e = cudaMallocAsync(&d_msa, (size_t)ncol * nrow, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_cnt, sizeof(int) * nrow, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&d_w, sizeof(float) * nrow, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_msa, msa, (size_t)ncol * nrow, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = reweight_counts(d_msa, ncol, nrow, idthres, d_cnt, s);
+  cudaError_t e = pool_alloc(device, reinterpret_cast<void **>(&d_msa), cells + 8 * (size_t)nrow, s);
+  int *d_cnt = reinterpret_cast<int *>(d_msa + cells);
+  float *d_w = reinterpret_cast<float *>(d_cnt + nrow);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(d_msa, msa, (size_t)ncol * nrow, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = reweight_counts(device, d_msa, ncol, nrow, idthres, d_cnt, s);
   if (e == cudaSuccess) e = reweight_weights(d_cnt, d_w, nrow, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w, d_w, sizeof(float) * nrow, cudaMemcpyDeviceToHost, s);
   if (d_msa) cudaFreeAsync(d_msa, s);
-  if (d_cnt) cudaFreeAsync(d_cnt, s);
-  if (d_w) cudaFreeAsync(d_w, s);
   cudaError_t e2 = cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
+  release_stream(device, s);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess)
     return set_error(CCM_ERR_CUDA, "ccm_calculate_weights: %s", cudaGetErrorString(e));

@@ -77,21 +77,10 @@ int solve_waves(int n, const ccm_msa_desc *msas, const ccm_batch_params *params,
   cudaMemGetInfo(&mem_free, &mem_total);
   const size_t budget = params->wave_bytes > 0 ? params->wave_bytes : mem_free / 10 * 6;
   const int wave_max = params->wave_max > 0 ? params->wave_max : 64;
-  cudaMemPool_t pool = nullptr;
-  {
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
-      return set_last_error(CCM_ERR_CUDA, "ccm_solve_batch: cannot create a memory pool");
-    uint64_t keep = UINT64_MAX;
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  }
+  pool_batch_begin(dev);
   cudaStream_t stream = nullptr;
-  if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) {
-    cudaMemPoolDestroy(pool);
+  if (acquire_stream(dev, &stream) != cudaSuccess) {
+    pool_batch_end(dev);
     return set_last_error(CCM_ERR_CUDA, "ccm_solve_batch: cannot create a stream");
   }
   int rc = CCM_OK;
@@ -136,7 +125,7 @@ int solve_waves(int n, const ccm_msa_desc *msas, const ccm_batch_params *params,
         o.path = m.path >= 0 ? m.path : params->path;
         o.device = dev;
         o.stream = stream;
-        rc = create_context(&it.ctx, m.msa, L, N, w.data(), &o, pool);
+        rc = create_context(&it.ctx, m.msa, L, N, w.data(), &o);
       }
       if (rc == CCM_OK) {
         e = dev_alloc_raw(it.ctx, reinterpret_cast<void **>(&it.d_x), sizeof(float) * (size_t)nv);
@@ -209,8 +198,8 @@ int solve_waves(int n, const ccm_msa_desc *msas, const ccm_batch_params *params,
     if (graph) cudaGraphDestroy(graph);
   }
   cudaStreamSynchronize(stream);
-  cudaStreamDestroy(stream);
-  cudaMemPoolDestroy(pool);
+  release_stream(dev, stream);
+  pool_batch_end(dev);
   return rc;
 }
 
@@ -259,22 +248,11 @@ int ccm_solve_batch(int n, const ccm_msa_desc *msas, const ccm_batch_params *par
   // no share is faster: the prep and CG kernels spread over every SM anyway,
   // so a share only shrinks the GEMM grids.
   const int max_sms = params->sms_per_worker > 0 ? params->sms_per_worker : 0;
-  // One memory pool for the whole batch that keeps freed blocks mapped: each
-  // alignment's buffers reuse the previous alignment's memory instead of
-  // mapping fresh device memory (the default pool gives it back at every
-  // synchronisation).  Destroyed when the batch ends.
-  cudaMemPool_t pool = nullptr;
-  {
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = params->device;
-    if (cudaSetDevice(params->device) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess)
-      return ccm::set_last_error(CCM_ERR_CUDA, "ccm_solve_batch: cannot create a memory pool");
-    uint64_t keep = UINT64_MAX;
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  }
+  if (cudaSetDevice(params->device) != cudaSuccess)
+    return ccm::set_last_error(CCM_ERR_CUDA, "ccm_solve_batch: cannot select device %d", params->device);
+  // the library's pool keeps freed blocks mapped: each alignment's buffers reuse the
+  // previous alignment's memory instead of mapping fresh device memory
+  ccm::pool_batch_begin(params->device);
   std::atomic<int> next(0);
   std::atomic<int> first_error(CCM_OK);
   std::mutex err_mutex;
@@ -286,7 +264,7 @@ int ccm_solve_batch(int n, const ccm_msa_desc *msas, const ccm_batch_params *par
     // default stream, which would interfere with the CG's graph capture while
     // other workers are running
     cudaStream_t stream = nullptr;
-    if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (ccm::acquire_stream(params->device, &stream) != cudaSuccess) {
       int expected = CCM_OK;
       first_error.compare_exchange_strong(expected, CCM_ERR_CUDA);
       std::lock_guard<std::mutex> lock(err_mutex);
@@ -323,7 +301,7 @@ int ccm_solve_batch(int n, const ccm_msa_desc *msas, const ccm_batch_params *par
         o.device = params->device;
         o.stream = stream;
         o.max_sms = max_sms;
-        rc = ccm::create_context(&ctx, m.msa, L, N, w.data(), &o, pool);
+        rc = ccm::create_context(&ctx, m.msa, L, N, w.data(), &o);
       }
       auto cuda_ok = [&](cudaError_t e) {
         if (e != cudaSuccess && rc == CCM_OK)
@@ -364,14 +342,12 @@ int ccm_solve_batch(int n, const ccm_msa_desc *msas, const ccm_batch_params *par
         }
       }
     }
-    cudaStreamDestroy(stream);
+    ccm::release_stream(params->device, stream);
   };
   std::vector<std::thread> threads;
   for (int t = 0; t < nw; ++t) threads.emplace_back(work);
   for (auto &t : threads) t.join();
-  // every allocation has been freed on its worker's stream; the pool's memory
-  // is released once those frees have completed
-  cudaMemPoolDestroy(pool);
+  ccm::pool_batch_end(params->device);
   const int rc = first_error.load();
   if (rc != CCM_OK) ccm::set_last_error(rc, "ccm_solve_batch: %s", err_text.c_str());
   return rc;

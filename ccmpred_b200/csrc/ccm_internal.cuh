@@ -187,11 +187,18 @@ constexpr int kFinBlocks = 16, kFinThreads = 512;
 // event before the first kernel of an evaluation and one after each kernel.
 constexpr int kMaxProfMarks = 8;
 void prof_mark(ccm_context *c);
-// Stream-ordered device allocation on the context's stream, from its pool.
+// Stream-ordered device allocation from the library's pool of the device; for a context,
+// on its stream and counted against its limit.
+cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream);
 cudaError_t dev_alloc_raw(ccm_context *c, void **p, size_t bytes);
-// ccm_create with the pool that the context's device memory comes from.
+// While a batch runs, the pool keeps all freed memory mapped.
+void pool_batch_begin(int device);
+void pool_batch_end(int device);
+// A non-blocking stream for the duration of a call, from a few that are kept.
+cudaError_t acquire_stream(int device, cudaStream_t *s);
+void release_stream(int device, cudaStream_t s);
 int create_context(ccm_context **out, const unsigned char *msa, int ncol, int nrow,
-                   const float *weights, const ccm_options *opt, cudaMemPool_t pool);
+                   const float *weights, const ccm_options *opt);
 // init_bias restricted to the single fields x[0 .. 20L) (host).
 void init_single_fields(const unsigned char *msa, int ncol, int nrow, float *x);
 // sum_submatrices of a device x into a device L x L map.
@@ -241,8 +248,8 @@ int enqueue_evaluation(ccm_context *c, const float *d_x, float *d_g);
 int enqueue_evaluation_step(ccm_context *c, const float *d_x, const float *d_s,
                             const double *d_alpha, float *d_xt, float *d_g);
 
-cudaError_t reweight_counts(const uint8_t *d_msa, int L, int N, int idthres, int *d_counts,
-                            cudaStream_t stream);
+cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int idthres,
+                            int *d_counts, cudaStream_t stream);
 
 // An evaluate callback of the reference's shape (include/evaluate_cuda.h:8-13).
 typedef float (*ccm_eval_callback)(void *instance, const float *x, float *g, const int n);
@@ -281,7 +288,6 @@ struct ccm_context {
   int fwd_pairs = 74;             // resident CTA pairs of tc_forward
   int bwd_pairs = 74;             // resident CTA pairs of tc_backward
   cudaStream_t stream = nullptr;
-  cudaMemPool_t pool = nullptr;   // device memory pool, or null for the device's default pool
   size_t mem_limit = 0;           // ccm_options.mem_limit (0: none)
   size_t mem_used = 0;            // device bytes held through dev_alloc_raw
   bool own_stream = false;

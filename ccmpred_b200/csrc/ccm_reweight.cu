@@ -175,12 +175,12 @@ __global__ void rw_weights_kernel(const int *__restrict__ counts, float *__restr
   w[i] = (float)(1.0 / (double)(cf - 1.0f));
 }
 
-cudaError_t reweight_counts(const uint8_t *d_msa, int L, int N, int idthres, int *d_counts,
-                            cudaStream_t stream) {
+cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int idthres,
+                            int *d_counts, cudaStream_t stream) {
   const int words = ((L + 31) / 32 + kRwWords - 1) / kRwWords * kRwWords;
   const size_t plane_bytes = sizeof(uint32_t) * 8 * (size_t)N * words;
   uint32_t *planes = nullptr;  // the planes, then the flag of states above 31
-  cudaError_t e = cudaMallocAsync(&planes, plane_bytes + 16, stream);
+  cudaError_t e = pool_alloc(device, reinterpret_cast<void **>(&planes), plane_bytes + 16, stream);
   if (e != cudaSuccess) return e;
   int *high = reinterpret_cast<int *>(reinterpret_cast<char *>(planes) + plane_bytes);
   cudaMemsetAsync(high, 0, sizeof(int), stream);

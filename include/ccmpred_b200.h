@@ -242,6 +242,12 @@ CCM_API int ccm_debug_set_cg_skip_padding(ccm_context *ctx, int allow);
 CCM_API int ccm_calculate_weights_noalloc(const unsigned char *d_msa, int ncol, int nrow,
                                           float threshold, float *d_w, void *stream);
 
+/* The library keeps up to 4 GB of device memory that its calls freed mapped for its next
+ * calls (contexts, solves, sequence weights; all of it while a batch runs).  This gives
+ * what is unused on `device` back to the system; an allocation of the library's own that
+ * fails does the same before it is reported. */
+CCM_API int ccm_release_memory(int device);
+
 /* Description of the last error on this host thread. */
 CCM_API const char *ccm_last_error(void);
 
