@@ -275,10 +275,12 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t saddr, uint32_t rank) {
   return r;
 }
 
-// Arrive (release, cluster scope) on an mbarrier given by its shared::cluster address.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
+// Arrive on an mbarrier given by its shared::cluster address.  The CTA-scope release
+// (the default) is enough for what these barriers hand over, tensor memory read or
+// written under tcgen05.wait and tcgen05.fence; a cluster-scope release takes about a
+// thousand cycles.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // Whole-cluster barrier (all threads of both CTAs).  The non-.aligned form:
@@ -399,18 +401,53 @@ __device__ __forceinline__ void tmem_cp_pair_128x128b(uint32_t taddr, uint64_t s
   asm volatile("tcgen05.cp.cta_group::2.128x128b [%0], %1;" ::"r"(taddr), "l"(src) : "memory");
 }
 
-// Pair MMA (leader only) with 2:4-sparse A: D (+)= A * B, 8-bit integers,
-// K = 64 logical (32 stored bytes of A per row), metadata at TMEM column `meta`
-// (two columns per instruction: 4 bits per group of four logical K).
-__device__ __forceinline__ void umma_i8sp_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                               uint32_t idesc, uint32_t meta,
-                                               uint32_t accumulate) {
+// Pair MMAs (leader only) with 2:4-sparse A: D (+)= A * B, 8-bit integers, K = 64 logical
+// each (32 stored bytes of A per row), metadata at TMEM column `meta` (two columns per
+// instruction: 4 bits per group of four logical K).  One block of 128 logical K of the
+// three digit products: hi += A1 B0, lo += A128 B1 + A1 B2 (the first ones overwrite
+// unless `accumulate`).  a, b: low words of the descriptors of A x1 and of digit 0
+// (k = 0); kA, kB: from there to A x128 and to the next digit; kAK, kBK: to k = 1.
+// One asm statement: the sparse MMAs do not queue behind one another, so every
+// instruction of the issuing thread between them is tensor time lost.
+template <int kA, int kAK, int kB, int kBK>
+__device__ __forceinline__ void umma_i8sp_block(uint32_t hi, uint32_t lo, uint32_t a, uint32_t a_top,
+                                                uint32_t b, uint32_t b_top, uint32_t idesc,
+                                                uint32_t meta, uint32_t accumulate) {
+#define CCM_AT(D, FROM, OFF, TOP) "add.u32 w, " FROM ", " OFF ";\n\tmov.b64 " D ", {w, " TOP "};\n\t"
+#define CCM_MMA(D, A, B, M, P) \
+  "tcgen05.mma.sp.cta_group::2.kind::i8 [" D "], " A ", " B ", [" M "], %6, " P ";\n\t"
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.sp.cta_group::2.kind::i8 [%0], %1, %2, [%4], %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(meta), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\t.reg .b32 w, m1;\n\t"
+      ".reg .b64 a0, a1, c0, c1, b00, b01, b10, b11, b20, b21;\n\t"
+      "setp.ne.b32 p, %8, 0;\n\tsetp.eq.b32 q, %8, %8;\n\t"
+      "add.u32 m1, %7, 2;\n\t"
+      CCM_AT("a0", "%2", "0", "%3") CCM_AT("b00", "%4", "0", "%5")
+      CCM_MMA("%0", "a0", "b00", "%7", "p")
+      CCM_AT("c0", "%2", "%9", "%3") CCM_AT("b10", "%4", "%11", "%5")
+      CCM_MMA("%1", "c0", "b10", "%7", "p")
+      CCM_AT("b20", "%4", "%12", "%5")
+      CCM_MMA("%1", "a0", "b20", "%7", "q")
+      CCM_AT("a1", "%2", "%10", "%3") CCM_AT("b01", "%4", "%13", "%5")
+      CCM_MMA("%0", "a1", "b01", "m1", "q")
+      CCM_AT("c1", "%2", "%14", "%3") CCM_AT("b11", "%4", "%15", "%5")
+      CCM_MMA("%1", "c1", "b11", "m1", "q")
+      CCM_AT("b21", "%4", "%16", "%5")
+      CCM_MMA("%1", "a1", "b21", "m1", "q")
+      "}\n" ::"r"(hi), "r"(lo), "r"(a), "r"(a_top), "r"(b), "r"(b_top), "r"(idesc), "r"(meta),
+      "r"(accumulate), "n"(kA), "n"(kAK), "n"(kB), "n"(2 * kB), "n"(kBK), "n"(kA + kAK),
+      "n"(kB + kBK), "n"(2 * kB + kBK)
       : "memory");
+#undef CCM_AT
+#undef CCM_MMA
+}
+
+// The two words of a shared-memory descriptor (sdesc_* above): the low one moves with the
+// address (in units of 16 bytes), the high one is a constant of the layout.
+__host__ __device__ constexpr uint32_t sdesc_low(uint32_t saddr, uint32_t lbo_bytes) {
+  return (saddr >> 4) | (lbo_bytes >> 4) << 16;
+}
+__host__ __device__ constexpr uint32_t sdesc_high(uint32_t sbo_bytes, uint32_t layout) {
+  return (sbo_bytes >> 4) | 1u << 14 | layout << 29;
 }
 
 // 32 lanes x 32 columns of 32-bit, registers -> TMEM (the inverse of tmem_ld32).

@@ -613,7 +613,7 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
   tc_fence_before();
   __syncwarp();
   // the next tile's low phase may start
-  if (lane == 0) mbar_arrive_cluster(lo_bar);
+  if (lane == 0) mbar_arrive_remote(lo_bar);
   // B: e = exp(z - m), sum
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
@@ -907,7 +907,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kI8Threads, 1)
 #undef CCM_TILE_ARGS
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(hi_bar);
+      if (lane == 0) mbar_arrive_remote(hi_bar);
     }
   }
 
@@ -1084,7 +1084,7 @@ __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32
   }
   tc_fence_before();
   __syncwarp();
-  if (lane == 0) mbar_arrive_cluster(empty_bar);
+  if (lane == 0) mbar_arrive_remote(empty_bar);
   // A
   float mx[kCols], tg[kCols], se[kCols];
 #pragma unroll
@@ -1267,44 +1267,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
-      // ---------------- MMA issuer (leader): 256 x 192 x 64 (logical) sparse pair MMAs
+      // ---------------- MMA issuer (leader): 256 x 192 x 64 (logical) sparse pair MMAs.
+      // The loop carries its stage, phase and descriptor words along: see umma_i8sp_block
       constexpr uint32_t idesc = idesc_i8_s32(kI8PairM, kSpBN, 0, 1, 0, 1) | kIdescSparse;
-      uint32_t it = 0, ecopies = 0;
+      constexpr uint32_t kStep = SM::kStage >> 4;
+      const uint32_t s0 = smem_u32(smem);
+      const uint32_t a0 = sdesc_low(s0 + SM::kOffA1, 16), b0 = sdesc_low(s0 + SM::kOffB, SM::kAtom);
+      const uint32_t a_top = sdesc_high(512, 4), b_top = sdesc_high(256, 6);
+      uint32_t stage = 0, phase = 0, te = t_e;
       int local = 0;
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok && !i8_aborted(abort_flag);
            tile += npairs, ++local) {
-        // both accumulators free: the previous tile's epilogue finished its merge
+        // both accumulators free: the previous tile's epilogue has drained them
         if (!mbar_wait(acc_empty, (local & 1) ^ 1)) {
           i8_record_error(args.status, kErrFwdTimeout, abort_flag);
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int stage = it % kStages;
-          const uint32_t round = it / kStages;
-          if (!mbar_wait(&full[stage], round & 1)) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait(&full[stage], phase)) {
             i8_record_error(args.status, kErrFwdTimeout, abort_flag);
             ok = false;
             break;
           }
-          tc_fence_after();
-          const uint32_t s0 = smem_u32(smem + stage * SM::kStage);
-          const uint32_t te = t_e + 4 * (ecopies++ & 1);
-          tmem_cp_pair_128x128b(te, sdesc_noswz(s0 + SM::kOffE, 2048, 128));
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const uint64_t a1 = sdesc_sw64(s0 + SM::kOffA1 + k * 32, 16, 512);
-            const uint64_t a128 = sdesc_sw64(s0 + SM::kOffA128 + k * 32, 16, 512);
-            const uint64_t b0 = sdesc_sw32(s0 + SM::kOffB + k * 2048, SM::kAtom, 256);
-            const uint64_t b1 = sdesc_sw32(s0 + SM::kOffB + SM::kB + k * 2048, SM::kAtom, 256);
-            const uint64_t b2 = sdesc_sw32(s0 + SM::kOffB + 2 * SM::kB + k * 2048, SM::kAtom, 256);
-            const uint32_t first = (kb | k) != 0;
-            umma_i8sp_pair(t_hi, a1, b0, idesc, te + 2 * k, first);    // O1 x d0
-            umma_i8sp_pair(t_lo, a128, b1, idesc, te + 2 * k, first);  // O128 x d1
-            umma_i8sp_pair(t_lo, a1, b2, idesc, te + 2 * k, 1);        // O1 x d2
-          }
+          tmem_cp_pair_128x128b(te, sdesc_noswz(s0 + stage * SM::kStage + SM::kOffE, 2048, 128));
+          umma_i8sp_block<SM::kA / 16, 2, SM::kB / 16, 128>(t_hi, t_lo, a0 + stage * kStep, a_top,
+                                                            b0 + stage * kStep, b_top, idesc, te, kb);
           umma_commit_pair(&empty[stage], 0x3);
+          te ^= 4;
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
         if (ok) umma_commit_pair(acc_full, 0x3);
       }
@@ -1633,7 +1625,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(empty_bar);
+        if (lane == 0) mbar_arrive_remote(empty_bar);
         ++chunk;
         return true;
       };
