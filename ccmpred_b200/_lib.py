@@ -174,6 +174,12 @@ SIGNATURES = {
     "ccm_sum_submatrices": (ctypes.c_double, [_f32p, _f32p, ctypes.c_int]),
     "ccm_sum_submatrices_gpu": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                                ctypes.c_void_p]),
+    "ccm_pack_parameters": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_longlong), _vp,
+                                           ctypes.POINTER(ctypes.c_longlong), ctypes.c_int,
+                                           ctypes.c_int, _vp, _vp]),
+    "ccm_unpack_gradient": (ctypes.c_int, [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp,
+                                           ctypes.POINTER(ctypes.c_longlong), _vp,
+                                           ctypes.POINTER(ctypes.c_longlong), _vp]),
     "ccm_apc": (None, [_f32p, ctypes.c_int]),
     "ccm_normalize": (ctypes.c_int, [_f32p, ctypes.c_int]),
     "ccm_write_matrix": (ctypes.c_int, [ctypes.c_char_p, _f32p, ctypes.c_int, ctypes.c_int]),

@@ -15,9 +15,12 @@ Tensor layouts:
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import Evaluator, nsingle_padded, nvar_padded
+from ._lib import check, lib
 
 Q = 21
 QPAD = 32
@@ -61,8 +64,70 @@ class PseudoLikelihoodFunction(torch.autograd.Function):
         return grad_out * g, None
 
 
+def _strides(t: torch.Tensor):
+    return (ctypes.c_longlong * t.dim())(*t.stride())
+
+
+def _plain(t: torch.Tensor) -> bool:
+    """A dense CUDA tensor with memory of its own (not one of a function transform)."""
+    if not t.is_cuda or t.layout != torch.strided or t.is_conj() or t.is_neg():
+        return False
+    try:
+        return t.data_ptr() != 0
+    except RuntimeError:  # batched, functional or fake: no storage
+        return False
+
+
+def _native(V: torch.Tensor, W: torch.Tensor, evaluator: Evaluator) -> bool:
+    """Whether the packing kernels take V and W: the shapes and the type of the
+    evaluator's path, on the current device.  Everything else goes through pack(), with
+    its own errors and promotions."""
+    L = evaluator.L
+    dtype = torch.float64 if evaluator.path == "simt_f64" else torch.float32
+    return (V.shape == (L, Q - 1) and W.shape == (L, L, Q, Q) and V.dtype == W.dtype == dtype
+            and _plain(V) and _plain(W) and V.device == W.device
+            and V.device.index == torch.cuda.current_device())
+
+
+class PseudoLikelihoodVWFunction(torch.autograd.Function):
+    """f(V, W): the parameters packed and the gradient unpacked by one kernel each."""
+
+    @staticmethod
+    def forward(ctx, V: torch.Tensor, W: torch.Tensor, evaluator: Evaluator):
+        if evaluator.gradient != "partial":
+            raise ValueError("autograd needs an Evaluator with gradient='partial'")
+        x = torch.empty(evaluator.nvar, dtype=V.dtype, device=V.device)
+        g = torch.empty_like(x)
+        check(lib().ccm_pack_parameters(V.data_ptr(), _strides(V), W.data_ptr(), _strides(W),
+                                        evaluator.L, x.element_size(), x.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream))
+        f = evaluator.evaluate(x, g)
+        ctx.save_for_backward(g)
+        ctx.L = evaluator.L
+        return torch.full((), f, dtype=V.dtype, device=V.device)
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        (g,) = ctx.saved_tensors
+        L = ctx.L
+        need_v, need_w, _ = ctx.needs_input_grad
+        if (torch.is_grad_enabled() or not _plain(grad_out) or not _plain(g)
+                or grad_out.dtype != g.dtype or g.device.index != torch.cuda.current_device()):
+            dV, dW = unpack(grad_out * g, L)  # differentiable, and open to transforms
+            return dV if need_v else None, dW if need_w else None, None
+        dV = torch.empty((L, Q - 1), dtype=g.dtype, device=g.device)
+        dW = torch.empty((L, L, Q, Q), dtype=g.dtype, device=g.device)
+        check(lib().ccm_unpack_gradient(g.data_ptr(), grad_out.data_ptr(), L, g.element_size(),
+                                        dV.data_ptr() if need_v else None, _strides(dV),
+                                        dW.data_ptr() if need_w else None, _strides(dW),
+                                        torch.cuda.current_stream().cuda_stream))
+        return dV if need_v else None, dW if need_w else None, None
+
+
 def pseudo_likelihood(V: torch.Tensor, W: torch.Tensor, evaluator: Evaluator) -> torch.Tensor:
     """Differentiable f(V, W) (float32 on the tensor-core paths, float64 on simt_f64)."""
+    if _native(V, W, evaluator):
+        return PseudoLikelihoodVWFunction.apply(V, W, evaluator)
     x = pack(V, W)
     assert x.numel() == nvar_padded(V.shape[0])
     return PseudoLikelihoodFunction.apply(x, evaluator)

@@ -386,6 +386,18 @@ CCM_API double ccm_sum_submatrices(const float *x, float *out, int ncol);
  * equal to ccm_sum_submatrices bit for bit.  For callers that keep x on the
  * GPU after ccm_conjugrad_gpu: only L*L floats need to come back to the host. */
 CCM_API int ccm_sum_submatrices_gpu(const float *d_x, float *d_out, int ncol, void *stream);
+/* The autograd wrapper's parameters to the padded layout and its gradient back, on the
+ * device, enqueued on `stream` (a cudaStream_t, NULL for the legacy default stream):
+ * V (ncol x 20) and W (ncol x ncol x 21 x 21, W[k, j, b, a] = W(b,k,a,j)) with any element
+ * strides; elem_bytes 4 (float) or 8 (double).  ccm_pack_parameters writes all of x
+ * (nvar_padded elements, padding zero); ccm_unpack_gradient writes scale[0] * g (one
+ * device element) into dV and dW, each of which may be NULL. */
+CCM_API int ccm_pack_parameters(const void *V, const long long *v_strides, const void *W,
+                                const long long *w_strides, int ncol, int elem_bytes, void *x,
+                                void *stream);
+CCM_API int ccm_unpack_gradient(const void *g, const void *scale, int ncol, int elem_bytes, void *dV,
+                                const long long *v_strides, void *dW, const long long *w_strides,
+                                void *stream);
 /* src/util.c:66-108 apc, in place. */
 CCM_API void ccm_apc(float *mat, int ncol);
 /* src/util.c:110-140 normalize, in place; CCM_ERR_INVALID on a constant map. */
