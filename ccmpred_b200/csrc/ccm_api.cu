@@ -526,9 +526,10 @@ int check_status(ccm_context *c) {
   return CCM_OK;
 }
 
-// The result record, cleared before an evaluation (the sparse path's first kernel does it).
+// The result record, cleared before an evaluation (the first kernel of the sparse integer
+// and the split-bf16 paths does it).
 int clear_result(ccm_context *c) {
-  if (c->path == CCM_PATH_TC_I8SP) return CCM_OK;
+  if (c->path != CCM_PATH_TC_I8X3 && c->path != CCM_PATH_SIMT_F32) return CCM_OK;
   CCM_CUDA_TRY(zero_words(c->d_out, sizeof(ccm_result) / 4, c->stream));
   count_launch(c);
   return CCM_OK;

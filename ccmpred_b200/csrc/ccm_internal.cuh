@@ -135,7 +135,9 @@ struct PrepArgs {
   float *xt;                     // full vector out
   long long nsp;                 // nsingle_padded
   double *part_reg;
+  ccm_result *out;  // cleared
   int L, S;
+  int vec;  // every vector is 16-byte aligned
   float lambda_pair;
   float g2_coef;  // g2 starts at g2_coef * lambda_pair * x
 };

@@ -24,6 +24,7 @@
 namespace ccm {
 
 // ------------------------------------------------------------------ tc_prep
+// The first block also clears the result record.
 // One block per row (b,k) of the reference W matrix.  The row's 21 L real
 // entries are staged in shared memory (coalesced float4 loads); every thread
 // then emits 8 consecutive slots of row s(b,k) of each Wperm_i as one 16-byte
@@ -39,7 +40,11 @@ namespace ccm {
 template <int NSPLIT, bool STEP>
 __global__ void __launch_bounds__(256) tc_prep_kernel(const float *__restrict__ x2,
                                                       float *__restrict__ g2, PrepArgs args) {
-  extern __shared__ __align__(16) float xrow[];  // 21 L floats
+  extern __shared__ __align__(16) float xrow[];  // 21 L floats (and three of padding)
+  griddep_wait();
+  griddep_launch();
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(ccm_result) / 4)
+    reinterpret_cast<uint32_t *>(args.out)[threadIdx.x] = 0u;
   const int L = args.L;
   const int row = blockIdx.x;  // b*L + k
   float a = 0.0f;
@@ -60,13 +65,13 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const float *__restrict__ 
   const float two_l2 = args.g2_coef * args.lambda_pair;  // 2 (tied) or 1 (partial)
   const int nreal = kQ * L;
   double acc = 0.0;
-  // rows start at a multiple of 32 L floats (16-byte aligned); L % 4 == 0 allows float4
-  if ((L & 3) == 0) {
+  // rows start at a multiple of 32 L floats: 16-byte aligned where the vectors are
+  if (args.vec) {
     // the whole 32 L row as float4: four independent 16-byte loads in flight per
     // thread; the real states (first 21 L floats) are also staged in shared memory
     const float4 *src = reinterpret_cast<const float4 *>(x2 + base);
     float4 *dst = reinterpret_cast<float4 *>(g2 + base);
-    const int n4 = kQPad * L / 4, nreal4 = nreal / 4;
+    const int n4 = kQPad * L / 4, nreal4 = (nreal + 3) / 4;
     constexpr int kU = 4;
     for (int i0 = threadIdx.x; i0 < n4; i0 += kU * blockDim.x) {
       float4 v[kU];
@@ -161,9 +166,8 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const float *__restrict__ 
 constexpr int kFwdBM = 128, kFwdBN = 256, kFwdBK = 32;
 constexpr int kFwdPairM = 2 * kFwdBM;   // rows per pair tile
 constexpr int kFwdHalfN = kFwdBN / 2;   // B columns held by each CTA
-// forward: warp 0 TMA, warp 1 MMA (leader CTA), warps 2-9 epilogue (two warps per
+// forward: warp 0 TMA, warp 1 MMA (leader CTA), warps 4-11 epilogue (two warps per
 // TMEM lane quarter, each owning half of the 256 accumulator columns)
-constexpr int kFwdThreads = 320;
 
 template <int NSPLIT>
 struct FwdSmem {
@@ -172,9 +176,9 @@ struct FwdSmem {
   static constexpr int kBBytes = kFwdHalfN * kFwdBK * 2;         // 8 KB per term, MN-major
   static constexpr int kStage = kABytes + NSPLIT * kBBytes;
   static constexpr int kBarOff = kStages * kStage;
-  static constexpr int kVOff = kBarOff + 256;                     // V of the tile's 12 columns
+  static constexpr int kVOff = kBarOff + 256;                     // V per slot of the tile
   static constexpr int kXOff = kVOff + 1024;                       // half-to-half exchange
-  static constexpr int kXBytes = 2 * kFwdBM * 12 * 4;              // [half][row][12]
+  static constexpr int kXBytes = 2 * kGroupCols * kFwdBM * 8;      // [half][column][row] (max, sum)
   static constexpr int kTotal = kXOff + kXBytes + 1024;            // + alignment slack
 };
 
@@ -192,139 +196,135 @@ __device__ __forceinline__ bool aborted(const int *abort_flag) {
   return *reinterpret_cast<const volatile int *>(abort_flag) != 0;
 }
 
-// Forward epilogue for one warp: TMEM lane quarter q, column half H (chunks
-// 4H..4H+3 of the 8 x 32 accumulator columns).  The softmax over the 21
-// states of each of the 12 alignment columns of the tile needs both halves:
-// the per-column max and sum of exp are exchanged with the partner warp
-// (same rows, other half) through shared memory.
-template <int NSPLIT, int H>
-__device__ __forceinline__ void fwd_epilogue_tile(const FwdArgs &args, uint32_t taddr, const float *Vs,
-                                                  float *xbuf, int q, int lane, int n, int t,
-                                                  long long part) {
+// Forward epilogue for one warp: TMEM lane quarter q, column half `half` (tile columns
+// 128 half .. 128 half + 127).  The logits of the half are drained into registers and
+// the accumulator released; then per alignment column the maximum m of the own states,
+// e = exp(logit - m) and its sum, (m, s) exchanged with the partner warp (same rows,
+// other half), and R = w (P - onehot), P = e exp(m - M) / S, as its bf16 terms.
+// Both halves run the same instructions: element i of half 1 is tile column 128 + i,
+// alignment column (i + 8) mod 12, so that with its columns taken in the order lj = i
+// mod 12 its state is i / 12 + 10 (+ 1 from lj = 4 on); `xr` holds the observed states
+// less these.  (One copy of the code per half, with two exponentials an element, was
+// 250 KB of straight-line code, four times the instruction cache.)
+template <int NSPLIT>
+__device__ __forceinline__ bool fwd_epilogue_tile(const FwdArgs &args, uint32_t taddr, const float *Vs,
+                                                  float2 *xbuf, int half, int q, int lane, int n,
+                                                  int t, long long part, uint64_t *full_bar,
+                                                  uint32_t full_par, uint32_t empty_bar) {
   const int L = args.L;
   const int j0 = t * kGroupCols;
   const bool live = n < args.N;
   const float wn = live ? args.w[n] : 0.0f;
   const int row = q * 32 + lane;
-  const int pair_bar = 2 + q;
   int xr[kGroupCols];
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) {
-    const int j = j0 + jj;
-    xr[jj] = (live && j < L) ? (int)args.msa[(long long)n * L + j] : -1;
+  for (int lj = 0; lj < kGroupCols; ++lj) {
+    const int j = j0 + (half ? (lj + 8) % kGroupCols : lj);
+    const int first = half ? 10 + (lj >= 4) : 0;
+    xr[lj] = (live && j < L) ? (int)args.msa[(long long)n * L + j] - first : -100;
   }
-  const volatile float *Vv = Vs;
-  float *mine = xbuf + (H * kFwdBM + row) * kGroupCols;
-  const float *other = xbuf + ((1 - H) * kFwdBM + row) * kGroupCols;
+  if (__any_sync(0xffffffffu, !mbar_wait(full_bar, full_par))) {
+    named_bar_sync(2 + q, 64);  // the partner may have got past its wait
+    return false;
+  }
+  tc_fence_after();
+  float z[kFwdHalfN];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t v[32];
+    tmem_ld32(taddr + half * kFwdHalfN + c * 32, v);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) z[c * 32 + i] = __uint_as_float(v[i]);
+  }
+  tmem_wait_ld();
+  // the loads are complete from here on: keep the compiler from using z before
+#pragma unroll
+  for (int i = 0; i < kFwdHalfN; ++i) asm volatile("" : "+f"(z[i]));
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive_remote(empty_bar);
 
   float mx[kGroupCols], tg[kGroupCols], se[kGroupCols];
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) { mx[jj] = -INFINITY; tg[jj] = 0.0f; se[jj] = 0.0f; }
-  // pass A: max over own states, logit of the observed state if it is ours
+  for (int lj = 0; lj < kGroupCols; ++lj) { mx[lj] = -INFINITY; tg[lj] = 0.0f; se[lj] = 0.0f; }
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    __syncwarp();
-    tmem_ld32(taddr + (4 * H + c) * 32, v);
-    tmem_wait_ld();
+  for (int i4 = 0; i4 < kFwdHalfN; i4 += 4) {
+    const float4 v4 = *reinterpret_cast<const float4 *>(Vs + half * kFwdHalfN + i4);
+    const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const int col = (4 * H + c) * 32 + i;
-      if (col < kGroupUsed) {
-        const int a = col / kGroupCols, jj = col % kGroupCols;
-        const float z = __uint_as_float(v[i]) + (a < kQ - 1 ? Vv[a * kGroupCols + jj] : 0.0f);
-        mx[jj] = fmaxf(mx[jj], z);
-        if (xr[jj] == a) tg[jj] = z;
-      }
+    for (int e = 0; e < 4; ++e) {
+      const int i = i4 + e, lj = i % kGroupCols;
+      z[i] += vs[e];
+      mx[lj] = fmaxf(mx[lj], z[i]);
+      if (xr[lj] == i / kGroupCols) tg[lj] = z[i];
     }
   }
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) mine[jj] = mx[jj];
-  named_bar_sync(pair_bar, 64);
-#pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) mx[jj] = fmaxf(mx[jj], other[jj]);
-  named_bar_sync(pair_bar, 64);  // partner has read `mine`
-  // pass B: own part of the sum of exp
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    __syncwarp();
-    tmem_ld32(taddr + (4 * H + c) * 32, v);
-    tmem_wait_ld();
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const int col = (4 * H + c) * 32 + i;
-      if (col < kGroupUsed) {
-        const int a = col / kGroupCols, jj = col % kGroupCols;
-        const float z = __uint_as_float(v[i]) + (a < kQ - 1 ? Vv[a * kGroupCols + jj] : 0.0f);
-        se[jj] += expf(z - mx[jj]);
-      }
-    }
+  for (int i = 0; i < kFwdHalfN; ++i) {
+    const int lj = i % kGroupCols;
+    z[i] = expf(z[i] - mx[lj]);
+    se[lj] += z[i];
   }
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) mine[jj] = se[jj];
-  named_bar_sync(pair_bar, 64);
-  float lse[kGroupCols];
+  for (int lj = 0; lj < kGroupCols; ++lj) {
+    const int jj = half ? (lj + 8) % kGroupCols : lj;
+    xbuf[(half * kGroupCols + jj) * kFwdBM + row] = make_float2(mx[lj], se[lj]);
+  }
+  named_bar_sync(2 + q, 64);
   double floss = 0.0;
+  float cw[kGroupCols];  // P w = e cw
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) {
-    // both halves form the same sum: H=0 adds (own + partner), H=1 (partner + own)
-    const float tot = H == 0 ? se[jj] + other[jj] : other[jj] + se[jj];
-    lse[jj] = mx[jj] + logf(tot);
+  for (int lj = 0; lj < kGroupCols; ++lj) {
+    const int jj = half ? (lj + 8) % kGroupCols : lj;
+    const float2 other = xbuf[((1 - half) * kGroupCols + jj) * kFwdBM + row];
+    const float mo = other.x, so = other.y;
+    const float M = fmaxf(mx[lj], mo);
+    const float fa = expf(mx[lj] - M), fo = expf(mo - M);
+    // both halves form the same sum
+    const float S = half == 0 ? se[lj] * fa + so * fo : so * fo + se[lj] * fa;
+    const float lse = M + logf(S);
+    cw[lj] = xr[lj] > -100 ? (fa / S) * wn : 0.0f;
     // the loss term belongs to the half holding the observed state's column
-    if (xr[jj] >= 0 && ((xr[jj] * kGroupCols + jj) >> 7) == H)
-      floss += (double)(wn * (lse[jj] - tg[jj]));
+    const int col = (xr[lj] + (half ? 10 + (lj >= 4) : 0)) * kGroupCols + jj;
+    if (xr[lj] > -100 && (col >> 7) == half) floss += (double)(wn * (lse - tg[lj]));
   }
-  // pass C: R = w (P - onehot) over own 128 slots, split into bf16 terms
-  const long long rbase = (long long)n * args.S + (long long)t * kGroupSlots;
+  // R = w (P - onehot), split into bf16 terms, 16 columns = 32 bytes of each term at a
+  // time: one full-sector store per term
+  const long long rbase = (long long)n * args.S + (long long)t * kGroupSlots + half * kFwdHalfN;
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int cc = 4 * H + c;
-    uint32_t v[32];
-    __syncwarp();
-    tmem_ld32(taddr + cc * 32, v);
-    tmem_wait_ld();
+  for (int c = 0; c < kFwdHalfN / 16; ++c) {
+    uint32_t ph[8], pl[8], pl2[8];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      // 16 columns = 32 bytes of each bf16 term: one full-sector store per term
-      uint32_t ph[8], pl[8], pl2[8];
+    for (int e2 = 0; e2 < 8; ++e2) {
+      float r[2];
 #pragma unroll
-      for (int e2 = 0; e2 < 8; ++e2) {
-        uint32_t hh = 0, ll = 0, l2 = 0;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = u * 16 + e2 * 2 + e;
-          const int col = cc * 32 + i;
-          float r = 0.0f;
-          if (col < kGroupUsed) {
-            const int a = col / kGroupCols, jj = col % kGroupCols;
-            const float z = __uint_as_float(v[i]) + (a < kQ - 1 ? Vv[a * kGroupCols + jj] : 0.0f);
-            if (xr[jj] >= 0) r = wn * (expf(z - lse[jj]) - (xr[jj] == a ? 1.0f : 0.0f));
-          }
-          const __nv_bfloat16 hb = __float2bfloat16_rn(r);
-          const float rr = r - __bfloat162float(hb);
-          const __nv_bfloat16 lb = __float2bfloat16_rn(rr);
-          hh |= (uint32_t)__bfloat16_as_ushort(hb) << (16 * e);
-          ll |= (uint32_t)__bfloat16_as_ushort(lb) << (16 * e);
-          if (NSPLIT > 2)
-            l2 |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(rr - __bfloat162float(lb)))
-                  << (16 * e);
-        }
-        ph[e2] = hh; pl[e2] = ll; pl2[e2] = l2;
+      for (int e = 0; e < 2; ++e) {
+        const int i = c * 16 + e2 * 2 + e, lj = i % kGroupCols;
+        r[e] = fmaf(z[i], cw[lj], xr[lj] == i / kGroupCols ? -wn : 0.0f);
       }
-      const long long off = rbase + cc * 32 + u * 16;
-      st_global_v8(args.r[0] + off, ph);
-      st_global_v8(args.r[1] + off, pl);
-      if (NSPLIT > 2) st_global_v8(args.r[2] + off, pl2);
+      auto split = [&]() {  // the two values' bf16 term, low one first; r keeps the rest
+        const __nv_bfloat162 h = __floats2bfloat162_rn(r[0], r[1]);
+        const uint32_t w = *reinterpret_cast<const uint32_t *>(&h);
+        r[0] -= __uint_as_float(w << 16);
+        r[1] -= __uint_as_float(w & 0xffff0000u);
+        return w;
+      };
+      ph[e2] = split();
+      pl[e2] = split();
+      if (NSPLIT > 2) pl2[e2] = split();
     }
+    st_global_v8(args.r[0] + rbase + c * 16, ph);
+    st_global_v8(args.r[1] + rbase + c * 16, pl);
+    if (NSPLIT > 2) st_global_v8(args.r[2] + rbase + c * 16, pl2);
   }
   // loss partial, one per (tile, epilogue warp), summed in fixed order by tc_finalize
   for (int o = 16; o > 0; o >>= 1) floss += __shfl_xor_sync(0xffffffffu, floss, o);
-  if (lane == 0) args.part_f[part * 8 + H * 4 + q] = floss;
+  if (lane == 0) args.part_f[part * 8 + half * 4 + q] = floss;
+  return true;
 }
 
 template <int NSPLIT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFwdThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     tc_forward_kernel(const __grid_constant__ FwdMaps maps, FwdArgs args) {
   using SM = FwdSmem<NSPLIT>;
   constexpr int kFwdStages = SM::kStages;
@@ -341,7 +341,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFwdThreads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
   float *Vs = reinterpret_cast<float *>(smem + SM::kVOff);
-  float *xbuf = reinterpret_cast<float *>(smem + SM::kXOff);
+  float2 *xbuf = reinterpret_cast<float2 *>(smem + SM::kXOff);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -365,8 +365,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFwdThreads, 1)
   tc_fence_before();
   cluster_sync();
   tc_fence_after();
+  // the prologue above overlaps the previous kernel's tail; its outputs from here
+  griddep_launch();
+  griddep_wait();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (warp < 4) reg_dec<kWgRegsLoad>();
   if (warp == 0) {
     if (lane == 0) {
       // ---------------- TMA producer (both CTAs): own A rows, own half of B
@@ -452,12 +456,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFwdThreads, 1)
       umma_commit_pair(drain, 0x1);
       if (!mbar_wait(drain, 0)) record_error(args.status, kErrFwdTimeout, abort_flag);
     }
-  } else {
+  } else if (warp >= 4) {
+    reg_inc<kWgRegsEpi>();
     // ---------------- epilogue (both CTAs): 8 warps; warp w owns TMEM lanes
-    // 32*(w%4) ... and column half (w-2)/4 of this CTA's 128 rows
+    // 32*(w%4) ... and column half (w-4)/4 of this CTA's 128 rows
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int ethr = threadIdx.x - 64;
+    const int half = (warp - 4) >> 2;
+    const int ethr = threadIdx.x - 128;
     const int L = args.L;
     int local = 0;
     for (int tile = pair; tile < n_tiles; tile += npairs, ++local) {
@@ -468,30 +473,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFwdThreads, 1)
       const uint32_t use = local >> 1;
       const int m = tile % args.m_tiles, t = tile / args.m_tiles;
       const int j0 = t * kGroupCols;
-      if (ethr < (kQ - 1) * kGroupCols) {
+      {
         const int a = ethr / kGroupCols, j = j0 + ethr % kGroupCols;
-        Vs[ethr] = (j < L) ? args.x1[a * L + j] : 0.0f;
+        float v = 0.0f;
+        if (a >= kQ) v = -INFINITY;  // padding slots
+        else if (a < kQ - 1 && j < L) v = args.x1[a * L + j];
+        Vs[ethr] = v;
       }
       named_bar_sync(1, 256);
       const int n = m * kFwdPairM + (int)rank * kFwdBM + q * 32 + lane;
-      bool ok = mbar_wait(&tfull[acc], use & 1);
-      if (__any_sync(0xffffffffu, !ok)) {
-        // leave through the agreement barrier at the top of the loop; the
-        // partner warp times out on the same barrier
-        if (lane == 0) record_error(args.status, kErrFwdTimeout, abort_flag);
-        continue;
-      }
-      tc_fence_after();
       const uint32_t taddr = tmem_base + acc * kFwdBN + ((uint32_t)(q * 32) << 16);
-      const long long part = (long long)tile * 2 + rank;
-      if (half == 0)
-        fwd_epilogue_tile<NSPLIT, 0>(args, taddr, Vs, xbuf, q, lane, n, t, part);
-      else
-        fwd_epilogue_tile<NSPLIT, 1>(args, taddr, Vs, xbuf, q, lane, n, t, part);
-      // accumulator may be reused by the leader's MMA warp
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&tempty[acc]), 0));
+      const bool ok = fwd_epilogue_tile<NSPLIT>(args, taddr, Vs, xbuf, half, q, lane, n, t,
+                                                (long long)tile * 2 + rank, &tfull[acc], use & 1,
+                                                mapa_shared(smem_u32(&tempty[acc]), 0));
+      // left through the agreement barrier at the top of the loop
+      if (!ok && lane == 0) record_error(args.status, kErrFwdTimeout, abort_flag);
     }
   }
 
@@ -583,6 +579,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
   tc_fence_before();
   cluster_sync();
   tc_fence_after();
+  griddep_launch();
+  griddep_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp < 4) reg_dec<kWgRegsLoad>();
@@ -751,7 +749,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
 // -------------------------------------------------------------- tc_finalize
 // fx = sum(loss partials) + lambda1 sum V^2 + 0.5 lambda2 sum x2^2 (all in FP64,
 // fixed summation order); g1 = g1d + 2 lambda1 V, g1 padding = 0
-// (src/evaluate_cpu.c:151-163).  kFinBlocks blocks each sum a fixed share of
+// (src/evaluate_cpu.c:151-163).  Up to kFinBlocks blocks each sum a fixed share of
 // the partials; the block that finishes last (a ticket counter, reset by it)
 // adds the blocks' sums in block order and writes the result.
 __global__ void __launch_bounds__(kFinThreads) tc_finalize_kernel(FinalizeArgs args) {
@@ -829,14 +827,21 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   pa.g2_coef = c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f;
   for (int i = 0; i < 3; ++i) pa.wperm[i] = c->d_wperm[i];
   prof_mark(c);
+  auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
+  pa.vec = ((bits(d_x) | bits(d_g) | bits(step_x) | bits(step_s)) & 15) == 0;
+  pa.out = c->d_out;
+  const size_t row_smem = sizeof(float) * (kQ * L + 3);
+  cudaError_t e;
   if (step) {
     pa.step_x = step_x; pa.step_s = step_s; pa.alpha = alpha;
     pa.xt = const_cast<float *>(d_x); pa.nsp = c->nsp;
-    tc_prep_kernel<NSPLIT, true><<<kQ * L + 1, 256, sizeof(float) * kQ * L, c->stream>>>(
-        step_x + c->nsp, g2, pa);
+    e = launch_pdl(tc_prep_kernel<NSPLIT, true>, dim3(kQ * L + 1), dim3(256), row_smem, c->stream,
+                   step_x + c->nsp, g2, pa);
   } else {
-    tc_prep_kernel<NSPLIT, false><<<kQ * L, 256, sizeof(float) * kQ * L, c->stream>>>(x2, g2, pa);
+    e = launch_pdl(tc_prep_kernel<NSPLIT, false>, dim3(kQ * L), dim3(256), row_smem, c->stream, x2, g2,
+                   pa);
   }
+  if (e != cudaSuccess) return e;
   prof_mark(c);
 
   FwdArgs fa{};
@@ -847,8 +852,9 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   const int pair_tiles = fa.m_tiles * c->T;
   const int fwd_tiles = 2 * pair_tiles;  // 128-row halves, one loss partial set each
   const int pairs = pair_tiles < c->fwd_pairs ? pair_tiles : c->fwd_pairs;
-  tc_forward_kernel<NSPLIT><<<2 * pairs, kFwdThreads, FwdSmem<NSPLIT>::kTotal, c->stream>>>(
-      c->fwd_maps, fa);
+  e = launch_pdl(tc_forward_kernel<NSPLIT>, dim3(2 * pairs), dim3(kWgThreads),
+                 FwdSmem<NSPLIT>::kTotal, c->stream, c->fwd_maps, fa);
+  if (e != cudaSuccess) return e;
   prof_mark(c);
 
   BwdArgs ba{};
@@ -856,15 +862,14 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   ba.n_tiles = c->n_bwd_tiles; ba.status = c->d_status; ba.L = L; ba.S = c->S; ba.Npad = c->Npad;
   ba.lambda_pair = c->lambda_pair;
   const int bwd_pairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
-  if (c->gradient == CCM_GRADIENT_PARTIAL)
-    tc_backward_kernel<NSPLIT, false>
-        <<<2 * bwd_pairs, kWgThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
-  else
-    tc_backward_kernel<NSPLIT, true>
-        <<<2 * bwd_pairs, kWgThreads, BwdSmem<NSPLIT>::kTotal, c->stream>>>(c->bwd_maps, ba);
+  e = launch_pdl(c->gradient == CCM_GRADIENT_PARTIAL ? tc_backward_kernel<NSPLIT, false>
+                                                     : tc_backward_kernel<NSPLIT, true>,
+                 dim3(2 * bwd_pairs), dim3(kWgThreads), BwdSmem<NSPLIT>::kTotal, c->stream,
+                 c->bwd_maps, ba);
+  if (e != cudaSuccess) return e;
   prof_mark(c);
 
-  launch_tc_finalize(c, x1, d_g, fwd_tiles);
+  if ((e = launch_tc_finalize(c, x1, d_g, fwd_tiles)) != cudaSuccess) return e;
   prof_mark(c);
   count_launch(c, 4);
   return cudaGetLastError();
@@ -881,8 +886,11 @@ FinalizeArgs finalize_args(ccm_context *c, const float *x1, float *d_g, long lon
 }
 
 cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles) {
-  return launch_pdl(tc_finalize_kernel, dim3(kFinBlocks), dim3(kFinThreads), 0, c->stream,
-                    finalize_args(c, x1, d_g, n_fwd_tiles));
+  // one block up to eight partials a thread
+  const FinalizeArgs za = finalize_args(c, x1, d_g, n_fwd_tiles);
+  const long long blocks = (za.n_part_f + za.n_part_reg + za.nsp) / (8 * kFinThreads) + 1;
+  return launch_pdl(tc_finalize_kernel, dim3((unsigned)(blocks < kFinBlocks ? blocks : kFinBlocks)),
+                    dim3(kFinThreads), 0, c->stream, za);
 }
 
 cudaError_t tc_backward_max_pairs(int nsplit, int *pairs) {
@@ -901,7 +909,7 @@ cudaError_t tc_backward_max_pairs(int nsplit, int *pairs) {
 cudaError_t tc_forward_max_pairs(int nsplit, int *pairs) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2, 1, 1);
-  cfg.blockDim = dim3(kFwdThreads, 1, 1);
+  cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = nsplit == 3 ? FwdSmem<3>::kTotal : FwdSmem<2>::kTotal;
   int n = 0;
   cudaError_t e = nsplit == 3
