@@ -591,6 +591,14 @@ int ccm::enqueue_evaluation_step(ccm_context *c, const float *d_x, const float *
   return CCM_OK;
 }
 
+int ccm::enqueue_evaluation_trial(ccm_context *c, const CgTrialArgs &trial) {
+  c->prof_idx = 0;
+  const cudaError_t e = i8_evaluate(c, nullptr, nullptr, nullptr, nullptr, nullptr, &trial);
+  if (e != cudaSuccess)
+    return set_error(CCM_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+  return CCM_OK;
+}
+
 int ccm::enqueue_evaluation(ccm_context *c, const float *d_x, float *d_g) {
   return enqueue_eval(c, d_x, d_g);
 }

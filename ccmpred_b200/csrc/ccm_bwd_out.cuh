@@ -119,15 +119,15 @@ __device__ __forceinline__ void bwd_output(const float (&acc)[128], float *Tb, f
 // 375 us at L = 300, N = 5000 and from 53 to 23 us at L = 50, N = 200.
 template <bool SYM>
 __device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb,
-                                                   const BwdArgs &args, int lane, int row0,
-                                                   int col0, bool diagonal) {
+                                                   const BwdArgs &args, float *g1, float *g2,
+                                                   const float *x1, int lane, int row0, int col0,
+                                                   bool diagonal) {
   const int L = args.L, nat = kQ * L;
-  float *g2 = args.g2;
   const int row = row0 + lane;
   const long long pitch = (long long)kQPad * L;
   auto single = [&](int v, float data) {  // g1 entry v (below 20 L) from its data term
     args.g1d[v] = data;
-    args.fin.g1[v] = data + 2.0f * args.fin.lambda_single * args.fin.x1[v];
+    g1[v] = data + 2.0f * args.fin.lambda_single * x1[v];
   };
   if (SYM) {
     // the ones slot's column: the single-field gradient

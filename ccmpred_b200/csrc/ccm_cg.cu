@@ -91,19 +91,56 @@ __device__ __forceinline__ void for_span(const VecSpan &v, F f) {
   }
 }
 
-// Per-block FP64 partials of  a.b, a.a, a.c  (b and c may be null).  Fixed grid
-// and fixed summation order: the result does not depend on scheduling.
+// Per-block FP64 partials of  a.b, a.a, a.c  (b and c may be null); with sw.parity set,
+// a and c are the gradients of the trial and of the current point.  Fixed grid and
+// fixed summation order: the result does not depend on scheduling.  Bound by memory:
+// two 16-byte loads per vector and thread in flight where the vectors allow it (`vec`;
+// with single floats, a pass took 190 us at L = 300 where its bytes take 75).
 __global__ void __launch_bounds__(256) cg_dots_kernel(const float *__restrict__ a,
                                                       const float *__restrict__ b,
-                                                      const float *__restrict__ c, VecSpan v,
-                                                      double *__restrict__ part) {
+                                                      const float *__restrict__ c, CgSwap sw,
+                                                      VecSpan v, int vec, double *__restrict__ part) {
+  if (sw.parity) {
+    const int q = *sw.parity;
+    a = sw.at_g(1 - q);
+    c = sw.at_g(q);
+  }
   double ab = 0.0, aa = 0.0, ac = 0.0;
-  for_span(v, [&](long long i) {
-    const double av = a[i];
-    if (b) ab += av * (double)b[i];
-    aa += av * av;
-    if (c) ac += av * (double)c[i];
-  });
+  auto add = [&](float av, float bv, float cv) {
+    ab += (double)av * (double)bv;
+    aa += (double)av * (double)av;
+    ac += (double)av * (double)cv;
+  };
+  auto one = [&](long long i) { add(a[i], b ? b[i] : 0.0f, c ? c[i] : 0.0f); };
+  // elements [i0, i0 + n) by the block's threads, from an aligned i0
+  auto run = [&](long long i0, int n) {
+    if (!vec) {
+      for (int i = threadIdx.x; i < n; i += 256) one(i0 + i);
+      return;
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 *a4 = reinterpret_cast<const float4 *>(a + i0);
+    const float4 *b4 = reinterpret_cast<const float4 *>(b + i0);
+    const float4 *c4 = reinterpret_cast<const float4 *>(c + i0);
+    const int n4 = n / 4;
+    for (int i = threadIdx.x; i < n4; i += 512) {
+      const bool two = i + 256 < n4;
+      const float4 a0 = a4[i], a1 = two ? a4[i + 256] : zero;
+      const float4 b0 = b ? b4[i] : zero, b1 = b && two ? b4[i + 256] : zero;
+      const float4 c0 = c ? c4[i] : zero, c1 = c && two ? c4[i + 256] : zero;
+      add(a0.x, b0.x, c0.x); add(a0.y, b0.y, c0.y); add(a0.z, b0.z, c0.z); add(a0.w, b0.w, c0.w);
+      add(a1.x, b1.x, c1.x); add(a1.y, b1.y, c1.y); add(a1.z, b1.z, c1.z); add(a1.w, b1.w, c1.w);
+    }
+    for (int i = n4 * 4 + threadIdx.x; i < n; i += 256) one(i0 + i);
+  };
+  if (v.cols == 0) {
+    // all n: runs of 4096
+    for (long long i0 = blockIdx.x * 4096LL; i0 < v.n; i0 += gridDim.x * 4096LL)
+      run(i0, (int)(v.n - i0 < 4096 ? v.n - i0 : 4096));
+  } else {
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < v.nsp; i += gridDim.x * 256LL) one(i);
+    for (int r = blockIdx.x; r < v.rows; r += gridDim.x) run(v.nsp + (long long)r * v.row, v.cols);
+  }
   __shared__ double red[3][8];
   for (int o = 16; o > 0; o >>= 1) {
     ab += __shfl_xor_sync(0xffffffffu, ab, o);
@@ -148,7 +185,7 @@ __device__ double reduce_part(const double *part, int nblocks, int k, double *re
 }
 
 // Conditional-node values a control kernel sets: the value of the WHILE node
-// whose body holds it (its line search) when mode >= 1.  Mode 0: none
+// whose body holds it, its line search (mode 1) or its solve (mode 2).  Mode 0: none
 // (host-driven).  Every conditional value in these graphs is set in one of two
 // ways only: by a kernel in the body of a WHILE node, for that node (the
 // control and the guard), or by a kernel upstream of an IF or WHILE node in the
@@ -240,7 +277,8 @@ __global__ void __launch_bounds__(256) cg_control_kernel(CgCtl *ctl, CgRuleParam
     ctl->ls_active = 0;
   }
   (void)accepted;
-  if (h.mode >= 1) cudaGraphSetConditional(h.ls_self, ctl->ls_active ? 1u : 0u);
+  if (h.mode == 1) cudaGraphSetConditional(h.ls_self, ctl->ls_active ? 1u : 0u);
+  if (h.mode == 2) cudaGraphSetConditional(h.ls_self, ctl->status == kCgRunning ? 1u : 0u);
 }
 
 }  // namespace ccm
@@ -289,6 +327,7 @@ struct CgRun {
   cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};  // whole solve | parity 0 | parity 1
   bool want_xx = false;
   bool fused = false;
+  bool swap = false;     // whole solves choose their buffers on the device (sparse path)
   bool padfree = false;  // x0's padding states are zero: every pass skips them
   VecSpan span{};        // the elements the vector passes visit
   size_t mem_mark = 0;  // the context's mem_used before this solve's buffers
@@ -360,11 +399,33 @@ void free_run(CgRun &r) {
   r.c->mem_used = r.mem_mark;
 }
 
+void launch_dots(CgRun &r, const float *a, const float *b, const float *c, const CgSwap &sw,
+                 double *part) {
+  auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
+  const int vec = ((bits(a) | bits(b) | bits(c) | bits(sw.g[0]) | bits(sw.g[1])) & 15) == 0;
+  cg_dots_kernel<<<kDotBlocks, 256, 0, r.c->stream>>>(a, b, c, sw, r.span, vec, part);
+}
+
 // One trial on the stream (in capture): direction, step + evaluation, dots,
-// control.  Parity p: x = xb[p], trial into xb[1 - p].
+// control.  Parity p: x = xb[p], trial into xb[1 - p].  h.mode 2: the buffers are chosen
+// on the device, the direction is updated by the evaluation's first kernel.
 int enqueue_trial(CgRun &r, int p, const CgRuleParams &rp, CgHandles h) {
   ccm_context *c = r.c;
   cudaStream_t s = c->stream;
+  if (h.mode == 2) {
+    const long long before = c->launches;
+    const CgSwap sw{{r.xb[0], r.xb[1]}, {r.gb[0], r.gb[1]}, &r.d_ctl->parity};
+    const int rc = enqueue_evaluation_trial(
+        c, CgTrialArgs{sw, r.s, &r.d_ctl->alpha, &r.d_ctl->beta, &r.d_ctl->dir_mode});
+    if (rc != CCM_OK) return rc;
+    launch_dots(r, nullptr, r.s, nullptr, sw, r.d_part);
+    cg_control_kernel<<<1, 256, 0, s>>>(r.d_ctl, rp, r.d_part, kDotBlocks, 0, c->d_out, nullptr, h);
+    r.trial_kernels = (int)(c->launches - before) + 2;
+    c->launches = before;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return set_last_error(CCM_ERR_CUDA, "cg trial: %s", cudaGetErrorString(e));
+    return CCM_OK;
+  }
   float *x = r.xb[p], *xt = r.xb[1 - p], *g = r.gb[p], *gt = r.gb[1 - p];
   const long long before = c->launches;
   cg_dir_kernel<<<grid_for(r.n), 256, 0, s>>>(g, r.s, r.d_ctl, r.span);
@@ -376,9 +437,8 @@ int enqueue_trial(CgRun &r, int p, const CgRuleParams &rp, CgHandles h) {
     rc = enqueue_evaluation(c, xt, gt);
   }
   if (rc != CCM_OK) return rc;
-  cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gt, r.s, g, r.span, r.d_part);
-  if (r.want_xx) cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(xt, nullptr, nullptr, r.span,
-                                                           r.d_part + 3 * kDotBlocks);
+  launch_dots(r, gt, r.s, g, CgSwap{}, r.d_part);
+  if (r.want_xx) launch_dots(r, xt, nullptr, nullptr, CgSwap{}, r.d_part + 3 * kDotBlocks);
   cg_control_kernel<<<1, 256, 0, s>>>(r.d_ctl, rp, r.d_part, kDotBlocks, r.want_xx ? 1 : 0,
                                       c->d_out, nullptr, h);
   r.trial_kernels = (int)(c->launches - before) + (r.fused ? 0 : 1) + (r.want_xx ? 4 : 3);
@@ -494,6 +554,13 @@ int add_parity_trial(CgRun &r, const CgRuleParams &rp, cudaGraph_t b_out, cudaGr
 // the solve runs and bounds the rounds by itself.  (Line searches as WHILE
 // nodes nested inside this loop stopped iterating after a few rounds on B200
 // with driver 580; one level of IF nodes inside one WHILE does not need it.)
+// On the sparse path the kernels choose their buffers by the parity in the state record
+// themselves:
+//   WHILE(outer) { trial }
+// and the control kernel keeps the loop open while the solve runs (every trial counts
+// an evaluation, which bounds it).  Six kernels a trial where the selectors, skipped IF
+// nodes, the guard and the direction kernel made it a dozen nodes: 190 -> 165 us per
+// trial at L = 120, N = 1500.
 int add_solve_loop(CgRun &r, const CgRuleParams &rp, cudaGraph_t g,
                    cudaGraphConditionalHandle h_out, const cudaGraphNode_t *deps, size_t ndeps,
                    cudaGraphNode_t *n_out) {
@@ -505,6 +572,7 @@ int add_solve_loop(CgRun &r, const CgRuleParams &rp, cudaGraph_t g,
   cudaError_t e = cudaGraphAddNode(n_out, g, deps, ndeps, &np);
   if (e != cudaSuccess) return set_last_error(CCM_ERR_UNSUPPORTED, "cg graph: %s", cudaGetErrorString(e));
   cudaGraph_t b_out = np.conditional.phGraph_out[0];
+  if (r.swap) return capture_trial_into(r, b_out, 0, rp, CgHandles{h_out, 2, 0});
   cudaGraphNode_t n_start = nullptr, n_t0 = nullptr, n_t1 = nullptr, n_guard = nullptr;
   e = cudaGraphAddEmptyNode(&n_start, b_out, nullptr, 0);
   if (e != cudaSuccess) return set_last_error(CCM_ERR_UNSUPPORTED, "cg graph: %s", cudaGetErrorString(e));
@@ -619,6 +687,7 @@ int ccm::cg_graph_solve_add(ccm_context *c, float *d_x, const ccm_cg_params *par
   r.xb[0] = d_x;
   r.fused = c->path == CCM_PATH_TC_BF16X2 || c->path == CCM_PATH_TC_BF16X3 ||
             c->path == CCM_PATH_TC_I8X3 || c->path == CCM_PATH_TC_I8SP;
+  r.swap = c->path == CCM_PATH_TC_I8SP;
   const size_t bytes = sizeof(float) * (size_t)r.n;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
@@ -654,7 +723,7 @@ int ccm::cg_graph_solve_add(ccm_context *c, float *d_x, const ccm_cg_params *par
     e = cudaStreamBeginCaptureToGraph(s, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     rc = enqueue_evaluation(c, r.xb[0], r.gb[0]);
-    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(r.gb[0], nullptr, nullptr, r.span, r.d_part);
+    launch_dots(r, r.gb[0], nullptr, nullptr, CgSwap{}, r.d_part);
     cg_start_kernel<<<1, 256, 0, s>>>(r.d_ctl, r.d_part, kDotBlocks, c->d_out, nullptr, h_out, 1);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t *deps = nullptr;
@@ -752,6 +821,7 @@ int ccm_conjugrad_gpu(ccm_context *c, float *d_x, long long n, const ccm_cg_para
   // tensor-core paths take the step inside the first pass over x
   r.fused = c->path == CCM_PATH_TC_BF16X2 || c->path == CCM_PATH_TC_BF16X3 ||
             c->path == CCM_PATH_TC_I8X3 || c->path == CCM_PATH_TC_I8SP;
+  r.swap = c->path == CCM_PATH_TC_I8SP;
   const size_t bytes = sizeof(float) * (size_t)n;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
@@ -781,7 +851,7 @@ int ccm_conjugrad_gpu(ccm_context *c, float *d_x, long long n, const ccm_cg_para
   // initial evaluation at x0: f0, g0, g0.g0
   rc = enqueue_evaluation(c, r.xb[0], r.gb[0]);
   if (rc == CCM_OK) {
-    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(r.gb[0], nullptr, nullptr, r.span, r.d_part);
+    launch_dots(r, r.gb[0], nullptr, nullptr, CgSwap{}, r.d_part);
     cg_start_kernel<<<1, 256, 0, s>>>(r.d_ctl, r.d_part, kDotBlocks, c->d_out, nullptr, 0, 0);
     count_launch(c, 2);
     e = cudaMemcpyAsync(r.h_ctl, r.d_ctl, kCgCtlHead, cudaMemcpyDeviceToHost, s);
@@ -852,6 +922,7 @@ int ccm::conjugrad_callback_gpu(float *d_x, long long n, ccm_eval_callback eval,
   cudaStream_t s = 0;  // legacy default stream
   const size_t bytes = sizeof(float) * (size_t)n;
   const VecSpan flat{n, 0, 0, 0, 0};  // a foreign evaluation: every element
+  const int vec = (reinterpret_cast<uintptr_t>(d_x) & 15) == 0;
   float *xb[2] = {d_x, nullptr}, *gb[2] = {nullptr, nullptr}, *dir = nullptr;
   CgCtl *d_ctl = nullptr;
   double *d_part = nullptr, *d_f = nullptr;
@@ -876,7 +947,7 @@ int ccm::conjugrad_callback_gpu(float *d_x, long long n, ccm_eval_callback eval,
   };
   if (e == cudaSuccess) e = evaluate(0);
   if (e == cudaSuccess) {
-    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gb[0], nullptr, nullptr, flat, d_part);
+    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gb[0], nullptr, nullptr, CgSwap{}, flat, vec, d_part);
     cg_start_kernel<<<1, 256, 0, s>>>(d_ctl, d_part, kDotBlocks, nullptr, d_f, 0, 0);
     e = cudaMemcpyAsync(h, d_ctl, kCgCtlHead, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -887,9 +958,9 @@ int ccm::conjugrad_callback_gpu(float *d_x, long long n, ccm_eval_callback eval,
     cg_step_kernel<<<grid_for(n), 256, 0, s>>>(xb[p], dir, &d_ctl->alpha, xb[1 - p], n);
     e = evaluate(1 - p);
     if (e != cudaSuccess) break;
-    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gb[1 - p], dir, gb[p], flat, d_part);
-    if (progress) cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(xb[1 - p], nullptr, nullptr, flat,
-                                                           d_part + 3 * kDotBlocks);
+    cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gb[1 - p], dir, gb[p], CgSwap{}, flat, vec, d_part);
+    if (progress) cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(xb[1 - p], nullptr, nullptr, CgSwap{}, flat,
+                                                           vec, d_part + 3 * kDotBlocks);
     cg_control_kernel<<<1, 256, 0, s>>>(d_ctl, rp, d_part, kDotBlocks, progress ? 1 : 0, nullptr,
                                         d_f, none);
     e = cudaMemcpyAsync(h, d_ctl, kCgCtlHead, cudaMemcpyDeviceToHost, s);

@@ -69,10 +69,34 @@ struct I8SpMaps {
   CUtensorMap b[3];      // digits of W: 12 KB tiles (128 K rows x 96 slots), box 256 x 48
 };
 
+// The buffers of a device-side solve, chosen on the device: with q = *parity the current
+// point is x[q] and its gradient g[q], the trial goes to x[1 - q], g[1 - q].
+struct CgSwap {
+  float *x[2], *g[2];
+  const int *parity;  // null: not used, the plain pointers beside it hold
+#ifdef __CUDACC__
+  // (without indexing, which would copy the argument to local memory)
+  __device__ __forceinline__ float *at_x(int q) const { return q ? x[1] : x[0]; }
+  __device__ __forceinline__ float *at_g(int q) const { return q ? g[1] : g[0]; }
+#endif
+};
+// A trial of such a solve: before the step the direction is updated, s <- -g (dir_mode
+// 1) or beta s - g (2).
+struct CgTrialArgs {
+  CgSwap sw;
+  float *s;
+  const double *alpha, *beta;
+  const int *dir_mode;
+};
+
 // Sparse path: one pass over x (column maxima, sum of squares, regulariser gradient, step).
 struct I8ScanArgs {
-  const float *x, *s;    // full vectors; s: the CG direction, with alpha and xt (STEP)
+  const float *x;        // full vectors
+  float *s;              // STEP: the CG direction, with alpha and xt
   const double *alpha;
+  CgSwap sw;             // STEP: x, xt, g2 and the gradient of x, chosen on the device
+  const double *beta;    // with sw: the direction update
+  const int *dir_mode;
   float *xt;
   uint32_t *cmacc;       // column maxima as float bits, zero at the start
   double *part_reg;      // one partial of sum x2^2 per block
@@ -88,6 +112,8 @@ struct I8ScanArgs {
 // Sparse path: digits of W.
 struct I8DigitsArgs {
   const float *x2;
+  CgSwap sw;
+  long long nsp;
   const uint32_t *cmacc;
   uint32_t *colmax;      // copy of cmacc for the forward
   int8_t *wdig[3];
@@ -110,6 +136,7 @@ struct I8FwdArgs {
   const uint8_t *msa;
   const float *w;
   const float *x1;
+  CgSwap sw;
   const uint32_t *colmax;
   int8_t *r[3];
   uint8_t *rnat;  // sparse path: digits of R in the backward's natural storage
@@ -180,6 +207,7 @@ struct BwdArgs {
   // sparse path: g2 is 16-byte aligned; cmacc is cleared; fin: the sums of f, and g1
   int vec;
   uint32_t *cmacc;
+  CgSwap sw;
   FinalizeArgs fin;
 };
 
@@ -220,7 +248,7 @@ cudaError_t tc_backward_max_pairs(int nsplit, int *pairs);
 cudaError_t tc_evaluate(ccm_context *c, const float *d_x, float *d_g);
 // The integer path: evaluation at d_x, or (d_s != null) at d_xt = d_x + alpha d_s.
 cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
-                        const double *d_alpha, float *d_xt);
+                        const double *d_alpha, float *d_xt, const CgTrialArgs *trial = nullptr);
 cudaError_t i8_configure_kernels();
 cudaError_t i8_forward_max_pairs(int *pairs);
 cudaError_t i8_backward_max_pairs(int *pairs);
@@ -249,6 +277,9 @@ int enqueue_evaluation(ccm_context *c, const float *d_x, float *d_g);
 // evaluation at d_xt.
 int enqueue_evaluation_step(ccm_context *c, const float *d_x, const float *d_s,
                             const double *d_alpha, float *d_xt, float *d_g);
+
+// Sparse integer path: one trial of a device-side solve.
+int enqueue_evaluation_trial(ccm_context *c, const CgTrialArgs &trial);
 
 cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int idthres,
                             int *d_counts, cudaStream_t stream);

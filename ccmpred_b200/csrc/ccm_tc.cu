@@ -281,7 +281,8 @@ __device__ __forceinline__ bool fwd_epilogue_tile(const FwdArgs &args, uint32_t 
     const float M = fmaxf(mx[lj], mo);
     const float fa = expf(mx[lj] - M), fo = expf(mo - M);
     // both halves form the same sum
-    const float S = half == 0 ? se[lj] * fa + so * fo : so * fo + se[lj] * fa;
+    // (half 0's term is the fused one in both halves: the same float)
+    const float S = half == 0 ? fmaf(se[lj], fa, __fmul_rn(so, fo)) : fmaf(so, fo, __fmul_rn(se[lj], fa));
     const float lse = M + logf(S);
     cw[lj] = xr[lj] > -100 ? (fa / S) * wn : 0.0f;
     // the loss term belongs to the half holding the observed state's column
@@ -886,9 +887,9 @@ FinalizeArgs finalize_args(ccm_context *c, const float *x1, float *d_g, long lon
 }
 
 cudaError_t launch_tc_finalize(ccm_context *c, const float *x1, float *d_g, long long n_fwd_tiles) {
-  // one block up to eight partials a thread
+  // one block up to two partials a thread
   const FinalizeArgs za = finalize_args(c, x1, d_g, n_fwd_tiles);
-  const long long blocks = (za.n_part_f + za.n_part_reg + za.nsp) / (8 * kFinThreads) + 1;
+  const long long blocks = (za.n_part_f + za.n_part_reg + za.nsp) / (2 * kFinThreads) + 1;
   return launch_pdl(tc_finalize_kernel, dim3((unsigned)(blocks < kFinBlocks ? blocks : kFinBlocks)),
                     dim3(kFinThreads), 0, c->stream, za);
 }

@@ -161,10 +161,10 @@ __host__ __device__ constexpr long long i8sp_b_offset(int kr, int s, int KB) {
 //
 // i8sp_scan_kernel, one pass over x (row blocks of its 21 L coupling rows, four columns
 // per thread, eight rows of loads in flight): column maxima of |W| into cmacc (float
-// bits, atomicMax; zero between evaluations), sum x^2 partials (four squares in float,
-// added in FP64), the regulariser gradient g2 <- g2_scale * x2 (the backward adds C to
+// bits, atomicMax; zero between evaluations), sum x^2 partials (in FP64; where 4 divides
+// L, four squares in float and their sum in FP64), the regulariser gradient g2 <- g2_scale * x2 (the backward adds C to
 // it), and, STEP, the CG trial step v = fmaf(alpha, s, x) into xt (the last row of
-// blocks steps the single fields).  It also clears the result record.
+// blocks steps the single fields), in a solve's trial after the update of s.  It also clears the result record.
 // Rows go in K-row order k * 21 + b backwards, so that the digits kernel's first rows
 // are the ones read last here and are still in L2.  HBM-bound.  Together with the
 // digits kernel 108 us at L = 253, N = 7001 and 151 us at L = 300; the column-maximum,
@@ -178,14 +178,30 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
   griddep_launch();
   const int L = args.L, nreal = kQ * L;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
-  float alpha = 0.0f;
+  float alpha = 0.0f, beta = 0.0f;
+  int mode = 0;  // of the direction update
+  const float *x = args.x, *gp = nullptr;
+  float *xt = args.xt, *g2 = args.g2, *const s = args.s;
   if (STEP) {
     alpha = (float)args.alpha[0];
-    if (blockIdx.y == gridDim.y - 1) {
-      for (long long i = blockIdx.x * 256 + threadIdx.x; i < args.nsp; i += gridDim.x * 256LL)
-        args.xt[i] = fmaf(alpha, args.s[i], args.x[i]);
-      return;
+    if (args.sw.parity) {
+      const int q = *args.sw.parity;
+      mode = *args.dir_mode;
+      beta = (float)*args.beta;
+      x = args.sw.at_x(q);
+      xt = args.sw.at_x(1 - q);
+      gp = args.sw.at_g(q);
+      g2 = args.sw.at_g(1 - q) + args.nsp;
     }
+  }
+  auto direct = [&](float sv, float gv) { return mode == 1 ? -gv : fmaf(beta, sv, -gv); };
+  if (STEP && blockIdx.y == gridDim.y - 1) {
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i < args.nsp; i += gridDim.x * 256LL) {
+      float sv = s[i];
+      if (mode) s[i] = sv = direct(sv, gp[i]);
+      xt[i] = fmaf(alpha, sv, x[i]);
+    }
+    return;
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(ccm_result) / 4)
     reinterpret_cast<uint32_t *>(args.out)[threadIdx.x] = 0u;
@@ -194,7 +210,7 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
   if (c < args.cols) {
     // (cols = 21 L: the group that straddles 21 L reaches up to three padding states,
     // which are zero then)
-    const float *x2 = args.x + args.nsp + c;
+    const float *x2 = x + args.nsp + c;
     auto load = [&](const float *p) {
       return args.vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
     };
@@ -213,7 +229,18 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
         const int rr = nreal - 1 - min(r + u, r1 - 1);
         at[u] = ((long long)(rr % kQ) * L + rr / kQ) * kQPad * L;
         v[u] = load(x2 + at[u]);
-        if (STEP) sv[u] = load(args.s + args.nsp + c + at[u]);
+        if (STEP) sv[u] = load(s + args.nsp + c + at[u]);
+      }
+      if (STEP && mode) {
+        float4 gv[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) gv[u] = load(gp + args.nsp + c + at[u]);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          sv[u] = make_float4(direct(sv[u].x, gv[u].x), direct(sv[u].y, gv[u].y),
+                              direct(sv[u].z, gv[u].z), direct(sv[u].w, gv[u].w));
+          if (r + u < r1) store(s + args.nsp + c + at[u], sv[u]);
+        }
       }
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
@@ -221,15 +248,19 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
         if (STEP) {
           v[u] = make_float4(fmaf(alpha, sv[u].x, v[u].x), fmaf(alpha, sv[u].y, v[u].y),
                              fmaf(alpha, sv[u].z, v[u].z), fmaf(alpha, sv[u].w, v[u].w));
-          store(args.xt + args.nsp + c + at[u], v[u]);
+          store(xt + args.nsp + c + at[u], v[u]);
         }
-        acc += (double)fmaf(v[u].w, v[u].w, fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
+        if ((L & 3) == 0)
+          acc += (double)fmaf(v[u].w, v[u].w, fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
+        else
+          acc += ((double)v[u].x * v[u].x + (double)v[u].y * v[u].y) +
+                 ((double)v[u].z * v[u].z + (double)v[u].w * v[u].w);
         m[0] = fmaxf(m[0], fabsf(v[u].x));
         m[1] = fmaxf(m[1], fabsf(v[u].y));
         m[2] = fmaxf(m[2], fabsf(v[u].z));
         m[3] = fmaxf(m[3], fabsf(v[u].w));
         const float k = args.g2_scale;
-        store(args.g2 + at[u] + c, make_float4(k * v[u].x, k * v[u].y, k * v[u].z, k * v[u].w));
+        store(g2 + at[u] + c, make_float4(k * v[u].x, k * v[u].y, k * v[u].z, k * v[u].w));
       }
     }
 #pragma unroll
@@ -286,13 +317,14 @@ __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs a
   // padding slots of the groups stay zero
   for (int i = threadIdx.x; i < kDigRows * row_words; i += kDigThreads) qs[i] = 0;
   const int k_rows = kQ * L;
+  const float *x2 = args.sw.parity ? args.sw.at_x(1 - *args.sw.parity) + args.nsp : args.x2;
   const int r1 = min((int)(blockIdx.y + 1) * args.rows_per_block, k_rows);
   for (int r0 = blockIdx.y * args.rows_per_block; r0 < r1; r0 += kDigRows) {
     float v[kDigRows][kE];
 #pragma unroll
     for (int i = 0; i < kDigRows; ++i) {
       const int kr = min(r0 + i, r1 - 1);
-      const float *row = args.x2 + ((long long)(kr % kQ) * L + kr / kQ) * kQPad * L;
+      const float *row = x2 + ((long long)(kr % kQ) * L + kr / kQ) * kQPad * L;
 #pragma unroll
       for (int u = 0; u < kE; ++u) v[i][u] = off[u] >= 0 ? row[off[u]] : 0.0f;
     }
@@ -986,8 +1018,7 @@ __global__ void i8sp_onehot_kernel(const uint8_t *__restrict__ msa, uint32_t *__
 // next tile's MMAs overlap the softmax and the R digits.
 // TMEM: hi = [0, 192), lo = [256, 448), metadata slots at 456 and 460.
 constexpr int kSpBN = Groups192::kSlots, kSpBK = 128;
-constexpr int kSpHalf = 99;  // tile columns of the epilogue's half 0 (half 1: 90)
-constexpr int kSpTab = 100;  // floats per half in its tables of scales and V
+constexpr int kSpHalf = kSpBN / 2;  // tile columns of an epilogue warp
 
 struct I8SpSmem {
   static constexpr int kStages = 3;
@@ -1000,16 +1031,16 @@ struct I8SpSmem {
   static constexpr int kOffA1 = 0, kOffA128 = kA, kOffB = 2 * kA, kOffE = 2 * kA + 3 * kB;
   static constexpr int kStage = kOffE + kE;
   static constexpr int kBarOff = kStages * kStage;
-  static constexpr int kTabOff = kBarOff + 256;  // per tile: scale and V of both halves
-  static constexpr int kXOff = kTabOff + 4 * kSpTab * 4;  // per half, column and row: (max, sum)
+  static constexpr int kTabOff = kBarOff + 256;  // per tile: scale and V per column
+  static constexpr int kXOff = kTabOff + 2 * kSpBN * 4;  // per half, column and row: (max, sum)
   static constexpr int kXBytes = 2 * Groups192::kCols * kI8BM * 8;
   static constexpr int kROff = kXOff + kXBytes;  // per epilogue warp: 3 digits x 32 slots x 32 rows
   static constexpr int kRWarp = 3 * 32 * 32;
   static constexpr int kTotal = kROff + 8 * kRWarp + 1024;
 };
 
-// Epilogue of one tile for one warp (TMEM lane quarter q; half 0: states 0..10 of the
-// nine alignment columns, tile columns 0..98; half 1: states 11..20, columns 99..188):
+// Epilogue of one tile for one warp (TMEM lane quarter q, column half `half`: tile columns
+// 96 half .. 96 half + 95):
 //   drain  hi * 2^14 + lo of the half into registers (NARROW: as the exact 32-bit
 //          integer, one instruction; else as the rounded float), the next 16 columns
 //          in flight; then both accumulators are released, so that the next tile's
@@ -1023,13 +1054,15 @@ struct I8SpSmem {
 //          32 rows at a time through shared memory, so that a lane moves 16 rows of one
 //          slot with one store (byte stores straight to global memory, one sector each,
 //          took 60 k cycles per tile, this takes 20 k).
-// The whole half (99 values a thread) stays in registers: warpgroup 0 cedes its share
+// The whole half (96 values a thread) stays in registers: warpgroup 0 cedes its share
 // (kWgRegsLoad / kWgRegsEpi).  The accumulators are held for about 2 k of the tile's
 // 50 k cycles; a drain that also applied the scales and took the maxima held them 6 k.
-// Both halves run the same instructions (element i is state 11 half + i / 9, column
-// i % 9; half 1 ends at 90, its last nine elements have scale 0 and V = -inf): this
-// straight-line code is some 50 KB, and one copy per half did not fit the
-// instruction cache.
+// Both halves run the same instructions: element i of half 1 is tile column 96 + i,
+// alignment column (i + 6) mod 9, so that with its columns taken in the order lj = i mod
+// 9 its state is i / 9 + 10 (+ 1 from lj = 3 on); `xr` holds the observed states less
+// these, and its last three elements (no state) have scale 0 and V = -inf.  This
+// straight-line code is some 50 KB, and one copy per half did not fit the instruction
+// cache.
 template <bool NARROW>
 __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32_t t_hi,
                                                    uint32_t t_lo, const float *tab_scale,
@@ -1040,20 +1073,23 @@ __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32
                                                    long long budget, uint32_t empty_bar) {
   constexpr int kCols = Groups192::kCols;
   const int L = args.L;
-  const int j0 = t * kCols, a0 = 11 * half;
+  const int j0 = t * kCols;
   const bool live = n < args.N;
   const float wn = live ? args.w[n] : 0.0f;
   const int row = q * 32 + lane;
-  int xr[kCols];  // the observed state less a0; below -11: none
+  int xr[kCols];  // by lj; -100: none
 #pragma unroll
-  for (int jj = 0; jj < kCols; ++jj)
-    xr[jj] = (live && j0 + jj < L) ? (int)args.msa[(long long)n * L + j0 + jj] - a0 : -100;
+  for (int lj = 0; lj < kCols; ++lj) {
+    const int j = j0 + (half ? (lj + 6) % kCols : lj);
+    const int first = half ? 10 + (lj >= 3) : 0;
+    xr[lj] = (live && j < L) ? (int)args.msa[(long long)n * L + j] - first : -100;
+  }
   if (__any_sync(0xffffffffu, !mbar_wait(full_bar, full_par, budget))) {
     named_bar_sync(2 + q, 64);  // the partner may have got past its wait
     return false;
   }
   tc_fence_after();
-  float z[kSpHalf + 1];
+  float z[kSpHalf];
   {
     const uint32_t c0 = half * kSpHalf;
     auto merge = [](uint32_t hi, uint32_t lo) {
@@ -1072,15 +1108,6 @@ __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32
 #pragma unroll
       for (int i = 0; i < 16; ++i) z[c * 16 + i] = merge(vh[c & 1][i], vl[c & 1][i]);
     }
-    z[96] = z[97] = z[98] = 0.0f;
-    if (half == 0) {
-      uint32_t wh[4], wl[4];
-      tmem_ld4(t_hi + 96, wh);
-      tmem_ld4(t_lo + 96, wl);
-      tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 3; ++i) z[96 + i] = merge(wh[i], wl[i]);
-    }
   }
   tc_fence_before();
   __syncwarp();
@@ -1088,78 +1115,75 @@ __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32
   // A
   float mx[kCols], tg[kCols], se[kCols];
 #pragma unroll
-  for (int jj = 0; jj < kCols; ++jj) { mx[jj] = -INFINITY; tg[jj] = 0.0f; se[jj] = 0.0f; }
-  tab_scale += half * kSpTab;
-  tab_v += half * kSpTab;
+  for (int lj = 0; lj < kCols; ++lj) { mx[lj] = -INFINITY; tg[lj] = 0.0f; se[lj] = 0.0f; }
 #pragma unroll
-  for (int i4 = 0; i4 < kSpTab; i4 += 4) {
-    const float4 sc = *reinterpret_cast<const float4 *>(tab_scale + i4);
-    const float4 vv = *reinterpret_cast<const float4 *>(tab_v + i4);
+  for (int i4 = 0; i4 < kSpHalf; i4 += 4) {
+    const float4 sc = *reinterpret_cast<const float4 *>(tab_scale + half * kSpHalf + i4);
+    const float4 vv = *reinterpret_cast<const float4 *>(tab_v + half * kSpHalf + i4);
     const float scs[4] = {sc.x, sc.y, sc.z, sc.w}, vvs[4] = {vv.x, vv.y, vv.z, vv.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int i = i4 + e;
-      if (i < kSpHalf) {
-        const int jj = i % kCols;
-        const float sum = NARROW ? __int2float_rn(__float_as_int(z[i])) : z[i];
-        z[i] = fmaf(sum, scs[e], vvs[e]);
-        mx[jj] = fmaxf(mx[jj], z[i]);
-        if (xr[jj] == i / kCols) tg[jj] = z[i];
-      }
+      const int i = i4 + e, lj = i % kCols;
+      const float sum = NARROW ? __int2float_rn(__float_as_int(z[i])) : z[i];
+      z[i] = fmaf(sum, scs[e], vvs[e]);
+      mx[lj] = fmaxf(mx[lj], z[i]);
+      if (xr[lj] == i / kCols) tg[lj] = z[i];
     }
   }
   // B
 #pragma unroll
   for (int i = 0; i < kSpHalf; ++i) {
-    const int jj = i % kCols;
-    z[i] = expf(z[i] - mx[jj]);
-    se[jj] += z[i];
+    const int lj = i % kCols;
+    z[i] = expf(z[i] - mx[lj]);
+    se[lj] += z[i];
   }
 #pragma unroll
-  for (int jj = 0; jj < kCols; ++jj)
-    xbuf[(half * kCols + jj) * kI8BM + row] = make_float2(mx[jj], se[jj]);
+  for (int lj = 0; lj < kCols; ++lj) {
+    const int jj = half ? (lj + 6) % kCols : lj;
+    xbuf[(half * kCols + jj) * kI8BM + row] = make_float2(mx[lj], se[lj]);
+  }
   named_bar_sync(2 + q, 64);
   double floss = 0.0;
   // R * 2^21 = e * cw - [observed] * won, with cw = w exp(m - M) / S * 2^21
   float cw[kCols];
   const float won = live ? wn * args.r_enc : 0.0f;
 #pragma unroll
-  for (int jj = 0; jj < kCols; ++jj) {
+  for (int lj = 0; lj < kCols; ++lj) {
+    const int jj = half ? (lj + 6) % kCols : lj;
     const float2 other = xbuf[((1 - half) * kCols + jj) * kI8BM + row];
     const float mo = other.x, so = other.y;
-    const float M = fmaxf(mx[jj], mo);
-    const float fa = expf(mx[jj] - M), fo = expf(mo - M);
-    const float S = half == 0 ? se[jj] * fa + so * fo : so * fo + se[jj] * fa;
+    const float M = fmaxf(mx[lj], mo);
+    const float fa = expf(mx[lj] - M), fo = expf(mo - M);
+    // (half 0's term is the fused one in both halves: the same float)
+    const float S = half == 0 ? fmaf(se[lj], fa, __fmul_rn(so, fo)) : fmaf(so, fo, __fmul_rn(se[lj], fa));
     const float lse = M + logf(S);
-    cw[jj] = xr[jj] > -100 ? (fa / S) * won : 0.0f;
-    // the half that holds the observed state adds the loss term
-    if (xr[jj] >= 0 && xr[jj] < 11) floss += (double)(wn * (lse - tg[jj]));
+    cw[lj] = xr[lj] > -100 ? (fa / S) * won : 0.0f;
+    // the half that holds the observed state's column adds the loss term
+    const int col = (xr[lj] + (half ? 10 + (lj >= 3) : 0)) * kCols + jj;
+    if (xr[lj] > -100 && (col >= kSpHalf) == (half == 1)) floss += (double)(wn * (lse - tg[lj]));
   }
   // C
   uint8_t *const rrow = args.rnat + (long long)(n >> 5) * (3 * kNatTile);
   const long long sbytes = (long long)(args.Npad >> 5) * (3 * kNatTile);
-  const int used = half == 0 ? kSpHalf : 90;
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < kSpHalf / 32; ++c) {
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      if (c * 32 + i < kSpHalf) {
-        const int jj = (c * 32 + i) % kCols;
-        const float r = fmaf(z[c * 32 + i], cw[jj], xr[jj] == (c * 32 + i) / kCols ? -won : 0.0f);
-        // |R| 2^-eR <= 1: only the top of the range needs the clamp (P rounding to 1)
-        const int d = min(__float2int_rn(r), (1 << kI8FracBits) - 1);
-        rstage[i * 32 + lane] = (uint8_t)(d >> 14);
-        rstage[1024 + i * 32 + lane] = (uint8_t)((d >> 7) & 127);
-        rstage[2048 + i * 32 + lane] = (uint8_t)(d & 127);
-      }
+      const int lj = (c * 32 + i) % kCols;
+      const float r = fmaf(z[c * 32 + i], cw[lj], xr[lj] == (c * 32 + i) / kCols ? -won : 0.0f);
+      // |R| 2^-eR <= 1: only the top of the range needs the clamp (P rounding to 1)
+      const int d = min(__float2int_rn(r), (1 << kI8FracBits) - 1);
+      rstage[i * 32 + lane] = (uint8_t)(d >> 14);
+      rstage[1024 + i * 32 + lane] = (uint8_t)((d >> 7) & 127);
+      rstage[2048 + i * 32 + lane] = (uint8_t)(d & 127);
     }
     __syncwarp();
 #pragma unroll
-    for (int u = 0; u < (c < 3 ? 2 : 1); ++u) {
-      const int i = 16 * u + (lane >> 1), el = c * 32 + i;
-      const int a = a0 + el / kCols, j = j0 + el % kCols;
-      if (el < used && j < L) {
+    for (int u = 0; u < 2; ++u) {
+      const int i = 16 * u + (lane >> 1), col = half * kSpHalf + c * 32 + i;
+      const int a = col / kCols, j = j0 + col % kCols;
+      if (col < Groups192::kUsed && j < L) {
         const uint32_t s = (uint32_t)(a * L + j);
         uint8_t *p = rrow + (long long)(s >> 7) * sbytes + (s & 127) * 32 + (((lane ^ (s >> 2)) & 1) << 4);
         const uint4 *from = reinterpret_cast<const uint4 *>(rstage + i * 32 + (lane & 1) * 16);
@@ -1190,7 +1214,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(never + 1);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
   float *tab_scale = reinterpret_cast<float *>(smem + SM::kTabOff);
-  float *tab_v = tab_scale + 2 * kSpTab;
+  float *tab_v = tab_scale + kSpBN;
   float2 *xbuf = reinterpret_cast<float2 *>(smem + SM::kXOff);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1222,8 +1246,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
   griddep_launch();
   griddep_wait();
   const uint32_t tmem_base = *tmem_slot;
-  // TMEM: hi [0, 192), lo [256, 448), metadata 456 / 460 (the epilogue's 16-column
-  // loads reach up to three columns past an accumulator)
+  // TMEM: hi [0, 192), lo [256, 448), metadata 456 / 460
   const uint32_t t_hi = tmem_base, t_lo = tmem_base + 256, t_e = tmem_base + 456;
 
   if (warp < 4) reg_dec<kWgRegsLoad>();
@@ -1310,6 +1333,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     const int half = (warp - 4) >> 2;
     const int ethr = threadIdx.x - 128;
     const int L = args.L;
+    const float *x1 = args.sw.parity ? args.sw.at_x(1 - *args.sw.parity) : args.x1;
     uint8_t *const rstage = smem + SM::kROff + (warp - 4) * SM::kRWarp;
     const uint32_t empty_bar = mapa_shared(smem_u32(acc_empty), 0);
 
@@ -1317,17 +1341,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     for (int tile = pair; tile < n_tiles; tile += npairs, ++local) {
       if (named_bar_or(1, 256, i8_aborted(abort_flag))) break;
       const int m = tile % args.m_tiles, t = tile / args.m_tiles;
-      if (ethr < 2 * kSpTab) {
-        const int hf = ethr / kSpTab, i = ethr % kSpTab;
+      if (ethr < kSpBN) {
+        const int a = ethr / Groups192::kCols, j = t * Groups192::kCols + ethr % Groups192::kCols;
         float sc = 0.0f, vv = 0.0f;
-        if (i >= (hf == 0 ? kSpHalf : 90)) {
+        if (a >= kQ) {
           vv = -INFINITY;  // no state
-        } else {
-          const int a = 11 * hf + i / Groups192::kCols, j = t * Groups192::kCols + i % Groups192::kCols;
-          if (j < L) {
-            sc = pow2f(col_exponent(args.colmax[a * L + j]) - kI8FracBits);
-            if (a < kQ - 1) vv = args.x1[a * L + j];
-          }
+        } else if (j < L) {
+          sc = pow2f(col_exponent(args.colmax[a * L + j]) - kI8FracBits);
+          if (a < kQ - 1) vv = x1[a * L + j];
         }
         tab_scale[ethr] = sc;
         tab_v[ethr] = vv;
@@ -1391,7 +1412,8 @@ struct I8BwdSmem {
 // at the same rate either way.
 // fx = sum(loss partials) + lambda1 sum V^2 + 0.5 lambda2 sum x2^2 in FP64, in a fixed
 // order, and the padding of g1 (the backward's output phase writes g1 itself); one warp.
-__device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, int lane) {
+__device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const float *x1, float *g1,
+                                               int lane) {
   auto sum = [&](const double *p, long long n) {
     double s = 0.0;
     for (long long i0 = lane; i0 < n; i0 += 8 * 32) {
@@ -1408,11 +1430,11 @@ __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, int lan
   for (int i0 = lane; i0 < ns; i0 += 16 * 32) {
     float v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = i0 + 32 * u < ns ? args.x1[i0 + 32 * u] : 0.0f;
+    for (int u = 0; u < 16; ++u) v[u] = i0 + 32 * u < ns ? x1[i0 + 32 * u] : 0.0f;
 #pragma unroll
     for (int u = 0; u < 16; ++u) acc[2] += (double)v[u] * (double)v[u];
   }
-  for (long long i = ns + lane; i < args.nsp; i += 32) args.g1[i] = 0.0f;
+  for (long long i = ns + lane; i < args.nsp; i += 32) g1[i] = 0.0f;
 #pragma unroll
   for (int k = 0; k < 3; ++k)
     for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
@@ -1577,7 +1599,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     }
   } else if (NAT && warp == 2) {
     // the sums of the loss and regulariser partials, while the MMAs run
-    if (blockIdx.x == 0) i8nat_finalize(args.fin, lane);
+    if (blockIdx.x == 0) {
+      const int q = args.sw.parity ? 1 - *args.sw.parity : 0;
+      i8nat_finalize(args.fin, args.sw.parity ? args.sw.at_x(q) : args.fin.x1,
+                     args.sw.parity ? args.sw.at_g(q) : args.fin.g1, lane);
+    }
   } else if (NAT && warp == 3) {
     // the column maxima's accumulator, for the next evaluation's scan
     if (blockIdx.x == 0)
@@ -1592,6 +1618,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     const float r_dec = args.r_dec;
     const uint32_t empty_bar = mapa_shared(smem_u32(acc_empty), 0);
     const uint32_t col0 = half * kHalfN + ((uint32_t)(q * 32) << 16);
+    // the point evaluated and its gradient
+    const int buf = args.sw.parity ? 1 - *args.sw.parity : 0;
+    const float *x1 = args.sw.parity ? args.sw.at_x(buf) : args.fin.x1;
+    float *g1 = args.sw.parity ? args.sw.at_g(buf) : args.fin.g1;
     uint32_t chunk = 0;
     bool ok = true;
     for (int tile = pair; tile < n_tiles && ok; tile += npairs) {
@@ -1636,7 +1666,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       const int2 pq = args.tiles[tile];
       const int s1 = pq.x * kPairM + (int)rank * kBM + q * 32, s2 = pq.y * kBN + half * kHalfN;
       if constexpr (NAT)
-        bwd_output_natural<SYM>(accv, Tb, args, lane, s1, s2, pq.x == pq.y);
+        bwd_output_natural<SYM>(accv, Tb, args, g1, g1 + args.fin.nsp, x1, lane, s1, s2, pq.x == pq.y);
       else
         bwd_output<Groups256, SYM>(accv, Tb, args.g2, args.g1d, args.L, lane, s1, s2);
     }
@@ -1657,7 +1687,8 @@ namespace ccm {
 
 // ---------------------------------------------------------------- launchers
 // Evaluation at d_x, or, with d_s, at d_xt = d_x + alpha d_s (the step is taken
-// by the column-max pass, which writes d_xt).  Profile marks: [colmax + prep |
+// by the column-max pass, which writes d_xt), or, with trial (sparse path), a solve's
+// trial on its own buffers.  Profile marks: [colmax + prep |
 // forward | backward | finalize].
 static cudaError_t i8_prepare_dense(ccm_context *c, const float *d_x, float *g2, const float *d_s,
                                     const double *d_alpha, float *d_xt) {
@@ -1706,18 +1737,24 @@ static int scan_rows(int L, int col_blocks) {
 }
 
 static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2, const float *d_s,
-                                     const double *d_alpha, float *d_xt) {
+                                     const double *d_alpha, float *d_xt, const CgTrialArgs *trial) {
   const int L = c->L;
-  const bool step = d_s != nullptr;
+  const bool step = d_s != nullptr || trial;
   const float *xe = step ? d_xt : d_x;
   I8ScanArgs sa{};
-  sa.x = d_x; sa.s = d_s; sa.alpha = d_alpha; sa.xt = d_xt;
+  sa.x = d_x; sa.s = const_cast<float *>(d_s); sa.alpha = d_alpha; sa.xt = d_xt;
+  if (trial) {
+    sa.s = trial->s; sa.alpha = trial->alpha;
+    sa.sw = trial->sw; sa.beta = trial->beta; sa.dir_mode = trial->dir_mode;
+  }
   sa.cmacc = c->d_cmacc; sa.part_reg = c->d_part_reg; sa.g2 = g2; sa.out = c->d_out;
   sa.nsp = c->nsp; sa.L = L;
   sa.cols = (c->skip_padding ? kQ : kQPad) * L;
   sa.g2_scale = (c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f) * c->lambda_pair;
   auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
-  sa.vec = ((bits(d_x) | bits(d_s) | bits(d_xt) | bits(g2)) & 15) == 0;
+  const CgSwap &w = sa.sw;
+  sa.vec = ((bits(d_x) | bits(sa.s) | bits(d_xt) | bits(g2) | bits(w.x[0]) | bits(w.x[1]) |
+             bits(w.g[0]) | bits(w.g[1])) & 15) == 0;
   const int cb = (sa.cols + 1023) / 1024;
   sa.rows_per_block = scan_rows(L, cb);
   const int rb = (kQ * L + sa.rows_per_block - 1) / sa.rows_per_block;
@@ -1728,7 +1765,7 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
 
   I8DigitsArgs da{};
   for (int i = 0; i < 3; ++i) da.wdig[i] = c->d_wdig[i];
-  da.x2 = xe + c->nsp; da.cmacc = c->d_cmacc; da.colmax = c->d_colmax;
+  da.x2 = trial ? nullptr : xe + c->nsp; da.sw = sa.sw; da.nsp = c->nsp; da.cmacc = c->d_cmacc; da.colmax = c->d_colmax;
   da.L = L; da.T = c->T; da.KB = c->KP / 128;
   const int gb = (c->T + kDigGroups - 1) / kDigGroups;  // blocks along the groups, evenly filled
   da.gpb = (c->T + gb - 1) / gb;
@@ -1742,16 +1779,16 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
 }
 
 cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
-                        const double *d_alpha, float *d_xt) {
+                        const double *d_alpha, float *d_xt, const CgTrialArgs *trial) {
   const int L = c->L;
   const bool sp = c->path == CCM_PATH_TC_I8SP;
   const float *x1 = d_s != nullptr ? d_xt : d_x;
-  const float *x2 = x1 + c->nsp;
-  float *g2 = d_g + c->nsp;
+  const float *x2 = trial ? nullptr : x1 + c->nsp;
+  float *g2 = trial ? nullptr : d_g + c->nsp;
   cudaError_t e;
 
   prof_mark(c);
-  e = sp ? i8_prepare_sparse(c, d_x, g2, d_s, d_alpha, d_xt)
+  e = sp ? i8_prepare_sparse(c, d_x, g2, d_s, d_alpha, d_xt, trial)
          : i8_prepare_dense(c, d_x, g2, d_s, d_alpha, d_xt);
   if (e != cudaSuccess) return e;
   prof_mark(c);
@@ -1760,6 +1797,7 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   fa.msa = c->d_msa; fa.w = c->d_w; fa.x1 = x1; fa.colmax = c->d_colmax;
   for (int i = 0; i < 3; ++i) fa.r[i] = c->d_rdig[i];
   fa.rnat = c->d_rnat;
+  if (trial) fa.sw = trial->sw;
   fa.part_f = c->d_part_f; fa.status = c->d_status;
   fa.L = L; fa.N = c->N; fa.S = c->S; fa.T = c->T; fa.Npad = c->Npad;
   fa.m_tiles = c->Npad / kI8PairM;
@@ -1788,6 +1826,10 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
     // the sums and g1 are the backward's own (no finalize)
     ba.cmacc = c->d_cmacc;
     ba.vec = (reinterpret_cast<uintptr_t>(g2) & 15) == 0;
+    if (trial) {
+      ba.sw = trial->sw;
+      ba.vec = ((reinterpret_cast<uintptr_t>(ba.sw.g[0]) | reinterpret_cast<uintptr_t>(ba.sw.g[1])) & 15) == 0;
+    }
     ba.fin = finalize_args(c, x1, d_g, 2LL * pair_tiles);
     ba.fin.n_part_reg = c->n_part_reg;
   }
