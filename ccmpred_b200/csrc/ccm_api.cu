@@ -429,6 +429,26 @@ int alloc_tc(ccm_context *c) {
   for (int Q = 0; Q < blocks; ++Q)
     for (int P = 0; P < blocks; ++P)
       if (c->gradient == CCM_GRADIENT_PARTIAL || P <= Q) tiles.push_back(make_int2(P, Q));
+  std::vector<int> cuts;  // outlives the copy below
+  const int parts = sp ? i8_cut_parts((int)tiles.size(), c->bwd_pairs, c->Npad,
+                                      c->gradient != CCM_GRADIENT_PARTIAL) : 1;
+  if (parts > 1) {
+    // the tiles left over by whole waves, each as `parts` entries
+    const int rest = (int)tiles.size() % c->bwd_pairs, whole = (int)tiles.size() - rest;
+    const std::vector<int2> over(tiles.begin() + whole, tiles.end());
+    tiles.resize(whole);
+    cuts.assign(whole, 1 << 8);
+    for (int i = 0; i < rest; ++i)
+      for (int p = 0; p < parts; ++p) {
+        tiles.push_back(over[i]);
+        cuts.push_back(p | parts << 8 | i << 16);
+      }
+    c->n_cut_tiles = rest;
+    CCM_CUDA_TRY(dev_alloc(c, &c->d_cuts, sizeof(int) * cut_sums_offset((int)cuts.size()) +
+                                              kCutPartBytes * rest * parts));
+    CCM_CUDA_TRY(cudaMemcpyAsync(c->d_cuts, cuts.data(), sizeof(int) * cuts.size(),
+                                 cudaMemcpyHostToDevice, c->stream));
+  }
   c->n_bwd_tiles = (int)tiles.size();
   CCM_CUDA_TRY(dev_alloc(c, &c->d_bwd_tiles, sizeof(int2) * tiles.size()));
   CCM_CUDA_TRY(cudaMemcpyAsync(c->d_bwd_tiles, tiles.data(), sizeof(int2) * tiles.size(),
@@ -505,7 +525,7 @@ void free_all(ccm_context *c) {
   f(c->d_msa); f(c->d_w); f(c->d_out); f(c->d_onehot);
   for (int i = 0; i < 3; ++i) { f(c->d_wperm[i]); f(c->d_r[i]); f(c->d_wdig[i]); f(c->d_rdig[i]); }
   f(c->d_o1); f(c->d_o128); f(c->d_colmax); f(c->d_ac1); f(c->d_ac128); f(c->d_meta);
-  f(c->d_onat); f(c->d_rnat); f(c->d_cmacc);
+  f(c->d_onat); f(c->d_rnat); f(c->d_cmacc); f(c->d_cuts);
   f(c->d_part_f); f(c->d_part_reg); f(c->d_fin_part); f(c->d_fin_done); f(c->d_g1d); f(c->d_bwd_tiles);
   f(c->d_simt_pc); f(c->d_simt_g2); f(c->d_simt_part); f(c->d_simt_g1);
   f(c->d_xh); f(c->d_gh);
@@ -759,7 +779,8 @@ int ccm::create_context(ccm_context **out, const unsigned char *msa, int ncol, i
   CCM_CTX_TRY(cudaMemcpyAsync(c->d_msa, msa, (size_t)ncol * nrow, cudaMemcpyHostToDevice, c->stream));
   CCM_CTX_TRY(dev_alloc(c, &c->d_w, sizeof(float) * nrow));
   CCM_CTX_TRY(cudaMemcpyAsync(c->d_w, c->h_w, sizeof(float) * nrow, cudaMemcpyHostToDevice, c->stream));
-  CCM_CTX_TRY(dev_alloc(c, &c->d_out, sizeof(ccm_result)));
+  // behind it the counters of the sparse backward's cut tiles (BwdArgs::cuts)
+  CCM_CTX_TRY(dev_alloc(c, &c->d_out, kResultBytes));
   CCM_CTX_TRY(cudaMemsetAsync(c->d_out, 0, sizeof(ccm_result), c->stream));
   c->h_out = static_cast<ccm_result *>(pinned_small_alloc(sizeof(ccm_result)));
   if (!c->h_out) return fail(set_error(CCM_ERR_NOMEM, "pinned result record"));

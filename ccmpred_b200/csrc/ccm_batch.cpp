@@ -34,6 +34,8 @@ size_t ccm::context_bytes_estimate(int L, int N, int path) {
     const size_t KP = (QL + 255) / 256 * 256;
     b += 5 * Np * S + 3 * KP * SW + Np * KP + Np * KP / 8 + 8 * (Np / 128) * T * 8;
     b += 4 * (QL + S);
+    // at most one part of a cut backward tile per CTA pair
+    if (i8_cut_parts(1, 8, Np, true) > 1) b += 80 * kCutPartBytes;
   } else if (path == CCM_PATH_TC_I8X3) {
     const size_t S = 256 * (((size_t)L + kGroupCols - 1) / kGroupCols);
     b += 5 * Np * S + 3 * S * S + 8 * (Np / 128) * (S / 256) * 8 + 4 * (QL + S);

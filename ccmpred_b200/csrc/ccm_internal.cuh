@@ -101,9 +101,10 @@ struct I8ScanArgs {
   uint32_t *cmacc;       // column maxima as float bits, zero at the start
   double *part_reg;      // one partial of sum x2^2 per block
   float *g2;
-  ccm_result *out;       // cleared
+  ccm_result *out;       // cleared, with the counters behind it (out_vecs times 16 bytes)
   long long nsp;
   int L, rows_per_block;
+  unsigned out_vecs;     // at most the 256 threads of a block
   int cols;              // elements of a row: 32 L, or 21 L (padding skipped)
   int vec;               // every vector is 16-byte aligned
   float g2_scale;        // g2 = g2_scale * x
@@ -208,6 +209,9 @@ struct BwdArgs {
   int vec;
   uint32_t *cmacc;
   CgSwap sw;
+  // tiles cut along the rows (null: none): per tile part | parts << 8 | number of the cut
+  // tile << 16; behind them the parts' sums.  The parts finished are counted behind fin.out.
+  int *cuts;
   FinalizeArgs fin;
 };
 
@@ -253,6 +257,15 @@ cudaError_t i8_configure_kernels();
 cudaError_t i8_forward_max_pairs(int *pairs);
 cudaError_t i8_backward_max_pairs(int *pairs);
 cudaError_t i8_build_onehot(ccm_context *c);
+// Into how many parts along the rows the sparse path's backward cuts each of the tiles
+// that its last wave leaves over (1: none), for `tiles` tiles on `pairs` CTA pairs.
+int i8_cut_parts(int tiles, int pairs, int Npad, bool sym);
+constexpr size_t kCutPartBytes = 512 * 1024;  // (hi, lo) of a 256 x 256 tile
+constexpr int kMaxCutTiles = 60;
+constexpr int kCutCounters = 16;  // of a cut tile: two CTAs of eight epilogue warps
+constexpr size_t kResultBytes = (sizeof(ccm_result) + 4 * kCutCounters * kMaxCutTiles + 15) & ~15;
+static_assert(kResultBytes <= 16 * 256);
+__host__ __device__ inline int cut_sums_offset(int entries) { return (entries + 63) & ~63; }
 void i8nat_to_groups(const ccm_context *c, const uint8_t *nat, int mats, int mat, uint8_t *dst);
 cudaError_t i8sp_forward_max_pairs(int *pairs);
 // tc_finalize over the loss partials of n_fwd_tiles 128-row forward tiles.
@@ -378,6 +391,8 @@ struct ccm_context {
   // x1 | x128 (2 x Npad x SB bytes) and digits of R (3 x Npad x SB), tiled
   int SB = 0;
   uint8_t *d_onat = nullptr, *d_rnat = nullptr;
+  int *d_cuts = nullptr;            // its tiles cut along the rows (BwdArgs::cuts)
+  int n_cut_tiles = 0;
   uint8_t *d_ac1 = nullptr, *d_ac128 = nullptr, *d_meta = nullptr;
   ccm::I8SpMaps i8sp_maps;
 

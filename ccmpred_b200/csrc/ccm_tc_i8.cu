@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
     }
     return;
   }
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(ccm_result) / 4)
-    reinterpret_cast<uint32_t *>(args.out)[threadIdx.x] = 0u;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < args.out_vecs)
+    reinterpret_cast<uint4 *>(args.out)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   double acc = 0.0;
   if (c < args.cols) {
@@ -1407,6 +1407,10 @@ struct I8BwdSmem {
   static constexpr int kTotal = kTOff + kTBytes + 1024;
 };
 
+// CUT: a last wave of tiles that fills less than half of the pairs is cut along K (the rows):
+// every part is an entry of its own in the tile list, and the epilogue warp that finishes
+// a tile's part last adds the parts' integer sums (exact, so that the gradient is that of
+// the uncut tile bit for bit) and writes the output.
 // NAT: natural slots, K-major operands in the storage of i8nat_offset (the sparse
 // path); else Groups256 slots, row-major Npad x S operands (MN-major).  The MMAs run
 // at the same rate either way.
@@ -1447,7 +1451,7 @@ __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const f
   }
 }
 
-template <bool SYM, bool NAT>
+template <bool SYM, bool NAT, bool CUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8_backward_kernel(const __grid_constant__ I8BwdMaps maps, BwdArgs args) {
   using SM = I8BwdSmem;
@@ -1468,6 +1472,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int n_tiles = args.n_tiles;
   const int k_blocks = args.Npad / kI8BwdBK;
+  // K blocks [first, end) of an entry of the tile list
+  auto cut_of = [&](int tile) { return CUT ? args.cuts[tile] : 0; };
+  auto k_first = [&](int cut) { return CUT ? k_blocks * (cut & 255) / (cut >> 8 & 255) : 0; };
+  auto k_end = [&](int cut) { return CUT ? k_first(cut + 1) : k_blocks; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -1505,7 +1513,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         const int2 pq = args.tiles[tile];
         const int xP = pq.x * kPairM + (int)rank * kBM;
         const int xQ = pq.y * kBN + (int)rank * kHalfN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const int cut = cut_of(tile), kb_end = k_end(cut);
+        for (int kb = k_first(cut); kb < kb_end; ++kb, ++it) {
           const int stage = it % kStages;
           const uint32_t round = it / kStages;
           if (!mbar_wait(&empty[stage], (round & 1) ^ 1)) {
@@ -1557,14 +1566,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       uint32_t it = 0, chunk = 0;
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok && !i8_aborted(abort_flag); tile += npairs) {
-        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += kI8BwdChunkKB, ++chunk) {
+        const int cut = cut_of(tile), kb_end = k_end(cut);
+        for (int kb0 = k_first(cut); kb0 < kb_end && ok; kb0 += kI8BwdChunkKB, ++chunk) {
           if (!mbar_wait(acc_empty, (chunk & 1) ^ 1)) {
             i8_record_error(args.status, kErrBwdTimeout, abort_flag);
             ok = false;
             break;
           }
           tc_fence_after();
-          const int kb1 = min(kb0 + kI8BwdChunkKB, k_blocks);
+          const int kb1 = min(kb0 + kI8BwdChunkKB, kb_end);
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const int stage = it % kStages;
             const uint32_t round = it / kStages;
@@ -1659,9 +1669,93 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         ++chunk;
         return true;
       };
-      ok = take(std::true_type{});
-      for (int kb0 = kI8BwdChunkKB; kb0 < k_blocks && ok; kb0 += kI8BwdChunkKB)
-        ok = take(std::false_type{});
+      // One part of a cut tile: its sums to cut_sums, unless the other parts are there
+      // already; the warp that finishes last adds the parts' integers (exact, in any
+      // order) and goes on to the output.  Nobody waits.  0: error, 1: not last, 2: last.
+      auto take_part = [&](int cut) {
+        const bool w_ok = mbar_wait(acc_full, chunk & 1);
+        if (__any_sync(0xffffffffu, !w_ok)) {
+          if (lane == 0) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+          return 0;
+        }
+        tc_fence_after();
+        const int part = cut & 255, parts = cut >> 8 & 255;
+        const int who = (cut >> 16) * kCutCounters + (int)rank * 8 + (warp - 4);
+        // [cut tile, CTA, warp][part][16-column chunk, hi | lo, 4 columns][lane]
+        uint4 *sums = reinterpret_cast<uint4 *>(args.cuts + cut_sums_offset(args.n_tiles)) +
+                      (long long)who * parts * 64 * 32 + lane;
+        unsigned *done = reinterpret_cast<unsigned *>(args.fin.out + 1) + who;
+        auto seen = [&](bool count) {
+          unsigned n = 0;
+          if (lane == 0) n = count ? atomicAdd(done, 1u) : *reinterpret_cast<volatile unsigned *>(done);
+          return __shfl_sync(0xffffffffu, n, 0);
+        };
+        bool last = seen(false) == (unsigned)parts - 1;
+        if (!last) {
+#pragma unroll 1
+          for (int c = 0; c < kHalfN / 16; ++c) {
+            uint32_t v[2][16];
+            tmem_ld16(t_hi + col0 + c * 16, v[0]);
+            tmem_ld16(t_lo + col0 + c * 16, v[1]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              __stcg(sums + (part * 64 + c * 8 + i) * 32,
+                     make_uint4(v[i >> 2][(i & 3) * 4], v[i >> 2][(i & 3) * 4 + 1],
+                                v[i >> 2][(i & 3) * 4 + 2], v[i >> 2][(i & 3) * 4 + 3]));
+          }
+          __threadfence();
+          __syncwarp();
+          last = seen(true) == (unsigned)parts - 1;
+        }
+        if (last) {
+          __threadfence();
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < kHalfN / 16; ++c) {
+            uint32_t v[2][16];
+            tmem_ld16(t_hi + col0 + c * 16, v[0]);
+            tmem_ld16(t_lo + col0 + c * 16, v[1]);
+            tmem_wait_ld();
+#pragma unroll 1
+            for (int p = 0; p < parts; ++p) {
+              if (p == part) continue;
+              uint4 o[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = __ldcg(sums + (p * 64 + c * 8 + i) * 32);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                v[i >> 2][(i & 3) * 4] += o[i].x;
+                v[i >> 2][(i & 3) * 4 + 1] += o[i].y;
+                v[i >> 2][(i & 3) * 4 + 2] += o[i].z;
+                v[i >> 2][(i & 3) * 4 + 3] += o[i].w;
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) accv[c * 16 + i] = i8_merge_exact(v[0][i], v[1][i]) * r_dec;
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(empty_bar);
+        ++chunk;
+        return last ? 2 : 1;
+      };
+      bool cut_tile = false;
+      if constexpr (CUT) {
+        const int cut = cut_of(tile);
+        cut_tile = (cut >> 8 & 255) > 1;
+        if (cut_tile) {
+          const int got = take_part(cut);
+          ok = got != 0;
+          if (got == 1) continue;
+        }
+      }
+      if (!cut_tile) {
+        ok = take(std::true_type{});
+        for (int kb0 = kI8BwdChunkKB; kb0 < k_blocks && ok; kb0 += kI8BwdChunkKB)
+          ok = take(std::false_type{});
+      }
       if (!ok) break;
       const int2 pq = args.tiles[tile];
       const int s1 = pq.x * kPairM + (int)rank * kBM + q * 32, s2 = pq.y * kBN + half * kHalfN;
@@ -1749,6 +1843,7 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
   }
   sa.cmacc = c->d_cmacc; sa.part_reg = c->d_part_reg; sa.g2 = g2; sa.out = c->d_out;
   sa.nsp = c->nsp; sa.L = L;
+  sa.out_vecs = (int)(sizeof(ccm_result) + 4 * kCutCounters * c->n_cut_tiles + 15) / 16;
   sa.cols = (c->skip_padding ? kQ : kQPad) * L;
   sa.g2_scale = (c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f) * c->lambda_pair;
   auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
@@ -1776,6 +1871,27 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
   return launch_pdl(i8sp_digits_kernel,
                     dim3(gb, (kQ * L + da.rows_per_block - 1) / da.rows_per_block),
                     dim3(kDigThreads), sizeof(int) * kDigRows * dig_row_words(da.gpb), c->stream, da);
+}
+
+// A K block is 768 cycles of MMAs (not symmetric: 384), and cutting a tile in p saves
+// (p - 1) / p of its last wave.  It costs what writing the sums and adding p - 1 of them
+// takes (512 KB per part, L2 to two SMs), measured as 12 k + 6 k p cycles, and 8 k cycles in the
+// next scan, whose L2 these sums occupy.  The measured sides, backward alone: L = 300, 29 of 325
+// tiles left over, p = 2: N = 3000 250 us uncut, 241 cut, N = 5000 396 and 378; L = 253, 9 of
+// 231 tiles, p = 8: N = 2000 149 and 159, N = 3000 199 and 194, N = 7001 445 and 391;
+// L = 150, 17 of 91, p = 4: N = 2000 78 and 89, N = 3500 121 and 108; L = 200, N = 20000,
+// 5 of 153, p = 8: 870 and 710.  Rows beyond one chunk are not cut: their sums leave
+// the integers chunk by chunk.
+int i8_cut_parts(int tiles, int pairs, int Npad, bool sym) {
+  const int k_blocks = Npad / kI8BwdBK, rest = tiles % pairs;
+  if (rest == 0 || rest > kMaxCutTiles || k_blocks > kI8BwdChunkKB) return 1;
+  const int max_parts = pairs / rest < 8 ? pairs / rest : 8;
+  int best = 1, best_gain = 0;
+  for (int p = 2; p <= max_parts; ++p) {
+    const int gain = k_blocks * (sym ? 768 : 384) * (p - 1) / p - 20000 - 6000 * p;
+    if (gain > best_gain) best = p, best_gain = gain;
+  }
+  return best;
 }
 
 cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
@@ -1825,6 +1941,7 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   if (sp) {
     // the sums and g1 are the backward's own (no finalize)
     ba.cmacc = c->d_cmacc;
+    ba.cuts = c->d_cuts;
     ba.vec = (reinterpret_cast<uintptr_t>(g2) & 15) == 0;
     if (trial) {
       ba.sw = trial->sw;
@@ -1834,10 +1951,12 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
     ba.fin.n_part_reg = c->n_part_reg;
   }
   const dim3 bgrid(2 * bpairs);
-  auto bwd = sp && sym ? i8_backward_kernel<true, true>
-             : sp        ? i8_backward_kernel<false, true>
-             : sym       ? i8_backward_kernel<true, false>
-                         : i8_backward_kernel<false, false>;
+  auto bwd = sp && c->d_cuts ? (sym ? i8_backward_kernel<true, true, true>
+                                    : i8_backward_kernel<false, true, true>)
+             : sp            ? (sym ? i8_backward_kernel<true, true, false>
+                                    : i8_backward_kernel<false, true, false>)
+             : sym           ? i8_backward_kernel<true, false, false>
+                             : i8_backward_kernel<false, false, false>;
   e = launch_pdl(bwd, bgrid, dim3(kWgThreads), I8BwdSmem::kTotal, c->stream, c->i8bwd_maps, ba);
   if (e != cudaSuccess) return e;
   prof_mark(c);
@@ -1862,15 +1981,12 @@ cudaError_t i8_configure_kernels() {
       (e = cudaFuncSetAttribute(i8sp_forward_kernel, (cudaFuncAttribute)kMax, I8SpSmem::kTotal)) !=
           cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute(i8_backward_kernel<true, false>, (cudaFuncAttribute)kMax,
-                                I8BwdSmem::kTotal)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8_backward_kernel<false, false>, (cudaFuncAttribute)kMax,
-                                I8BwdSmem::kTotal)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8_backward_kernel<true, true>, (cudaFuncAttribute)kMax,
-                                I8BwdSmem::kTotal)) != cudaSuccess)
-    return e;
-  return cudaFuncSetAttribute(i8_backward_kernel<false, true>, (cudaFuncAttribute)kMax,
-                              I8BwdSmem::kTotal);
+  for (auto bwd : {i8_backward_kernel<true, false, false>, i8_backward_kernel<false, false, false>,
+                   i8_backward_kernel<true, true, false>, i8_backward_kernel<false, true, false>,
+                   i8_backward_kernel<true, true, true>, i8_backward_kernel<false, true, true>})
+    if ((e = cudaFuncSetAttribute(bwd, (cudaFuncAttribute)kMax, I8BwdSmem::kTotal)) != cudaSuccess)
+      return e;
+  return cudaSuccess;
 }
 
 cudaError_t i8_forward_max_pairs(int *pairs) {
@@ -1897,7 +2013,7 @@ cudaError_t i8_backward_max_pairs(int *pairs) {
   cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = I8BwdSmem::kTotal;
   *pairs = 0;
-  return cudaOccupancyMaxActiveClusters(pairs, i8_backward_kernel<true, false>, &cfg);
+  return cudaOccupancyMaxActiveClusters(pairs, i8_backward_kernel<true, false, false>, &cfg);
 }
 
 // One-hot operands for a context of the integer paths (Npad x S bytes each), and
