@@ -193,4 +193,15 @@ __device__ __forceinline__ void bwd_output_natural(float (&acc)[128], float *Tb,
   }
 }
 
+// The record into the pinned copy of a host that waits for this evaluation: no copy
+// behind the last kernel.  The host cleared the status; only an error is written, so that
+// this never covers one that the same kernel records on its own.
+__device__ __forceinline__ void finalize_host(const FinalizeArgs &args, double fx, double data) {
+  args.host->fx = fx;
+  args.host->f_data = data;
+  args.host->reg = fx - data;
+  const int status = *reinterpret_cast<const volatile int *>(&args.out->status);
+  if (status) *reinterpret_cast<volatile int *>(&args.host->status) = status;
+}
+
 }  // namespace ccm

@@ -192,6 +192,7 @@ struct FinalizeArgs {
   int L;
   float lambda_single, lambda_pair;
   ccm_result *out;
+  ccm_result *host;    // the caller's copy in pinned memory, or null (finalize_host)
   double *block_part;  // kFinBlocks x 3 sums
   unsigned *done;      // blocks finished (0 between evaluations)
 };
@@ -352,6 +353,7 @@ struct ccm_context {
   float *h_w = nullptr;           // N (host copy)
   ccm_result *d_out = nullptr;    // result of the last evaluation
   ccm_result *h_out = nullptr;    // pinned host mirror
+  bool host_record = false;       // the next evaluation writes its record there itself
   int *d_status = nullptr;        // == &d_out->status
 
   // tensor-core path

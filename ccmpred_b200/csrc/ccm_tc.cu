@@ -806,6 +806,7 @@ __global__ void __launch_bounds__(kFinThreads) tc_finalize_kernel(FinalizeArgs a
     args.out->fx = fx;
     args.out->f_data = F;
     args.out->reg = fx - F;
+    if (args.host) finalize_host(args, fx, F);
     *args.done = 0u;  // for the next evaluation (also inside a replayed graph)
   }
 }
@@ -882,6 +883,7 @@ FinalizeArgs finalize_args(ccm_context *c, const float *x1, float *d_g, long lon
   za.part_reg = c->d_part_reg; za.n_part_reg = (long long)kQ * c->L;
   za.x1 = x1; za.g1d = c->d_g1d; za.g1 = d_g; za.L = c->L; za.nsp = c->nsp;
   za.lambda_single = c->lambda_single; za.lambda_pair = c->lambda_pair; za.out = c->d_out;
+  za.host = c->host_record ? c->h_out : nullptr;
   za.block_part = c->d_fin_part; za.done = c->d_fin_done;
   return za;
 }

@@ -1448,7 +1448,14 @@ __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const f
     args.out->fx = fx;
     args.out->f_data = F;
     args.out->reg = fx - F;
+    if (args.host) finalize_host(args, fx, F);
   }
+}
+
+// (finalize_host may have written the record already)
+__device__ __forceinline__ void i8_backward_error(const BwdArgs &args, int *abort_flag) {
+  i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+  if (args.fin.host) *reinterpret_cast<volatile int *>(&args.fin.host->status) = kErrBwdTimeout;
 }
 
 template <bool SYM, bool NAT, bool CUT>
@@ -1518,7 +1525,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
           const int stage = it % kStages;
           const uint32_t round = it / kStages;
           if (!mbar_wait(&empty[stage], (round & 1) ^ 1)) {
-            i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+            i8_backward_error(args, abort_flag);
             ok = false;
             break;
           }
@@ -1553,7 +1560,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         const bool w = rank == 0 ? mbar_wait(&full[r % kStages], (r / kStages) & 1)
                                  : mbar_wait(&empty[r % kStages], (r / kStages) & 1);
         if (!w) {
-          i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+          i8_backward_error(args, abort_flag);
           break;
         }
       }
@@ -1569,7 +1576,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         const int cut = cut_of(tile), kb_end = k_end(cut);
         for (int kb0 = k_first(cut); kb0 < kb_end && ok; kb0 += kI8BwdChunkKB, ++chunk) {
           if (!mbar_wait(acc_empty, (chunk & 1) ^ 1)) {
-            i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+            i8_backward_error(args, abort_flag);
             ok = false;
             break;
           }
@@ -1579,7 +1586,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
             const int stage = it % kStages;
             const uint32_t round = it / kStages;
             if (!mbar_wait(&full[stage], round & 1)) {
-              i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+              i8_backward_error(args, abort_flag);
               ok = false;
               break;
             }
@@ -1605,7 +1612,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
         }
       }
       umma_commit_pair(drain, 0x1);
-      if (!mbar_wait(drain, 0)) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+      if (!mbar_wait(drain, 0)) i8_backward_error(args, abort_flag);
     }
   } else if (NAT && warp == 2) {
     // the sums of the loss and regulariser partials, while the MMAs run
@@ -1640,7 +1647,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       auto take = [&](auto first) {
         const bool w_ok = mbar_wait(acc_full, chunk & 1);
         if (__any_sync(0xffffffffu, !w_ok)) {
-          if (lane == 0) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+          if (lane == 0) i8_backward_error(args, abort_flag);
           return false;
         }
         tc_fence_after();
@@ -1675,7 +1682,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       auto take_part = [&](int cut) {
         const bool w_ok = mbar_wait(acc_full, chunk & 1);
         if (__any_sync(0xffffffffu, !w_ok)) {
-          if (lane == 0) i8_record_error(args.status, kErrBwdTimeout, abort_flag);
+          if (lane == 0) i8_backward_error(args, abort_flag);
           return 0;
         }
         tc_fence_after();
