@@ -3,7 +3,11 @@
 //   x[a L + j] = V[j, a];  x[nsp + ((b L + k) 32 + a) L + j] = W[k, j, b, a]
 // W's states are innermost, x's columns: a block takes one k and a run of JT columns j
 // with all 441 state pairs through shared memory (pitch JT + 1 words: no bank conflict),
-// so that both sides are read and written in runs.  Bound by memory: W and x once each.
+// so that both sides are read and written in runs.  Bound by memory (W and x once each,
+// 15 and 12 us at L = 150), which takes many loads in flight and little arithmetic per
+// element: the threads keep their place in a row and step by strides, seven or sixteen
+// loads at a time.  With an index divided out per element and one load in flight packing
+// took 41 and unpacking 48 us at L = 150, here 23 and 17.
 // (As torch operations -- permute, pad, concatenate and their backwards -- this was
 // some twenty launches and three copies of x: 300 of an evaluation's 500 us at L = 150.)
 #include <cuda_runtime.h>
@@ -39,31 +43,70 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(T *V, T *W, T *x, co
     return;
   }
   if (UNPACK && !W) return;
-  T *const w = W + k * st.w[0];
-  // x's side: JT consecutive columns of a row (b, k, a)
-  auto rows = [&](auto f) {
-    const int states = UNPACK ? kQ : kQPad;
-    for (int i = threadIdx.x; i < kQ * states * JT; i += kPackThreads) {
-      const int jj = i % JT, a = i / JT % states, b = i / (JT * states);
-      if (j0 + jj < L) f(x + nsp + (((long long)b * L + k) * kQPad + a) * L + j0 + jj, b, a, jj);
+  // x's side: thread (jj, gr) has column jj of the rows (b, k, a), a = gr, gr + kG, ...;
+  // seven states b at a time
+  constexpr int kG = kPackThreads / JT, kB = 7;
+  const int jj = threadIdx.x % JT, gr = threadIdx.x / JT;
+  T *const px = x + nsp + ((long long)k * kQPad + gr) * L + j0 + jj;
+  const long long bstep = (long long)kQPad * L * L;
+  auto rows = [&](auto move) {
+    if (j0 + jj >= L) return;
+#pragma unroll
+    for (int h = 0; h < kQPad / kG; ++h) {
+      const int a = gr + h * kG;
+      if (UNPACK && a >= kQ) break;
+      T *p = px + (long long)(h * kG) * L;
+      int t = a * (JT + 1) + jj;
+      for (int b = 0; b < kQ; b += kB, p += kB * bstep, t += kB * kQ * (JT + 1)) move(p, t, a < kQ);
     }
   };
-  // W's side: the state pairs of one column
-  auto pairs = [&](auto f) {
-    for (int i = threadIdx.x; i < kQQ * JT; i += kPackThreads) {
-      const int ba = i % kQQ, jj = i / kQQ;
-      if (j0 + jj < L)
-        f(w + (j0 + jj) * st.w[1] + ba / kQ * st.w[2] + ba % kQ * st.w[3], ba * (JT + 1) + jj);
-    }
-  };
+  // W's side: thread has the state pairs threadIdx.x and threadIdx.x + 256 of every
+  // column, eight columns at a time
+  constexpr int kP = (kQQ + kPackThreads - 1) / kPackThreads, kC = 8;
+  long long wp[kP];
+#pragma unroll
+  for (int u = 0; u < kP; ++u) {
+    const int ba = threadIdx.x + u * kPackThreads;
+    wp[u] = ba / kQ * st.w[2] + ba % kQ * st.w[3];
+  }
+  T *pw = W + k * st.w[0] + j0 * st.w[1];
+  auto in = [&](int u, int c) { return threadIdx.x + u * kPackThreads < kQQ && j0 + c < L; };
+  const int t0 = threadIdx.x * (JT + 1);
+  constexpr int kTU = kPackThreads * (JT + 1);
   if (!UNPACK) {
-    pairs([&](const T *p, int t) { tile[t] = *p; });
+    for (int c0 = 0; c0 < JT; c0 += kC) {
+      T v[kP][kC];
+#pragma unroll
+      for (int u = 0; u < kP; ++u)
+#pragma unroll
+        for (int c = 0; c < kC; ++c)
+          v[u][c] = in(u, c0 + c) ? pw[(c0 + c) * st.w[1] + wp[u]] : T(0);
+#pragma unroll
+      for (int u = 0; u < kP; ++u)
+#pragma unroll
+        for (int c = 0; c < kC; ++c)
+          if (in(u, c0 + c)) tile[t0 + u * kTU + c0 + c] = v[u][c];
+    }
     __syncthreads();
-    rows([&](T *p, int b, int a, int jj) { *p = a < kQ ? tile[(b * kQ + a) * (JT + 1) + jj] : T(0); });
+    rows([&](T *p, int t, bool real) {
+#pragma unroll
+      for (int b = 0; b < kB; ++b) p[b * bstep] = real ? tile[t + b * kQ * (JT + 1)] : T(0);
+    });
   } else {
-    rows([&](const T *p, int b, int a, int jj) { tile[(b * kQ + a) * (JT + 1) + jj] = *p; });
+    rows([&](const T *p, int t, bool) {
+      T v[kB];
+#pragma unroll
+      for (int b = 0; b < kB; ++b) v[b] = p[b * bstep];
+#pragma unroll
+      for (int b = 0; b < kB; ++b) tile[t + b * kQ * (JT + 1)] = v[b];
+    });
     __syncthreads();
-    pairs([&](T *p, int t) { *p = s * tile[t]; });
+    for (int c0 = 0; c0 < JT; c0 += kC)
+#pragma unroll
+      for (int u = 0; u < kP; ++u)
+#pragma unroll
+        for (int c = 0; c < kC; ++c)
+          if (in(u, c0 + c)) pw[(c0 + c) * st.w[1] + wp[u]] = s * tile[t0 + u * kTU + c0 + c];
   }
 }
 
