@@ -5,7 +5,8 @@
 // ccm_cg_rules.cuh; here they run on the device.
 //
 // Per line-search trial, on the context's stream:
-//   cg_dir_kernel      s <- -g or -g + beta s when the last decision asks for it
+//   cg_dir_kernel      s <- -g or -g + beta s when the last decision asks for it (whole
+//                      solves on the sparse path: in the evaluation's first kernel)
 //   step + evaluation  x_t = x + alpha s (alpha read from the control record;
 //                      fused into the first pass over x on the tensor-core
 //                      paths), f(x_t), g_t
@@ -13,11 +14,11 @@
 //   cg_control_kernel  one block: the partials summed in a fixed order, then
 //                      one thread applies the rules to the control record and
 //                      sets the conditional nodes' values
-// The trials form the body of a CUDA-graph WHILE node (the line search), and
-// the iterations -- two of them per round, one for each buffer parity, the x
-// and g of one iteration being the trial buffers of the previous one -- the
-// body of an outer WHILE node: without a progress callback the whole solve is
-// one graph launch and the host waits once.  With a progress callback (which
+// Without a progress callback the whole solve is one graph launch and the host waits
+// once: a CUDA-graph WHILE node whose body is one trial.  The x and g of one iteration
+// are the trial buffers of the previous one; on the sparse path the kernels choose
+// them on the device (CgSwap), elsewhere the body holds a trial per buffer parity,
+// each in an IF node of its own, and a guard.  With a progress callback (which
 // the reference calls after every iteration, src/ccmpred.c:50-61) the host
 // launches one line-search graph per iteration and reads the control record
 // back after each.  Vectors stay in float; every dot product and every

@@ -16,8 +16,10 @@
 // Per K element the tensor cores do three 8-bit products (at twice the bf16
 // rate) where the split-bf16 path does two bf16 products: 3/4 of the cycles.
 //
-// One evaluation = colmax (+ the fused CG step), prep (digits of W, g2 <- 2 l2 x,
-// sum x^2), forward, backward, finalize (shared with ccm_tc.cu).
+// One evaluation: on the dense path colmax (+ the fused CG step), prep (digits of W,
+// g2 <- 2 l2 x, sum x^2), forward, backward, finalize (shared with ccm_tc.cu); on the
+// sparse path four launches, scan (colmax, step, g2, sum x^2), digits, forward, backward
+// (with the sums of f and g1).
 #include <cmath>
 #include <type_traits>
 
@@ -280,17 +282,23 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
 
 // i8sp_digits_kernel: the three digits of W in the forward's tiled storage
 // (i8sp_b_offset).  A block takes `gpb` slot groups (9 gpb alignment columns with their
-// 21 states) and a run of K rows, eight rows at a time: a thread's elements are the
+// 21 states) and a run of K rows, ROWS at a time: a thread's elements are the
 // same columns of every row, so that their index arithmetic and encoding factors are
 // computed once; consecutive threads read runs of 9 gpb floats.  The fixed-point
 // integers go through shared memory in slot order (groups 200 words apart, rows an odd
 // multiple of 4 words apart modulo 32: no bank conflict), and 16 consecutive threads
 // write 256 contiguous bytes of a tile.  The first row of blocks also copies the column
 // maxima to `colmax`, which the forward reads: cmacc is cleared by the backward.
-constexpr int kDigThreads = 384, kDigRows = 8, kDigGroups = 8, kDigGroupWords = 200;
+// ROWS: eight, or four where eight leave blocks for less than two per SM
+// (L <= 72: 14.5 instead of 16.3 us for both kernels at L = 50, an evaluation 58.3 instead
+// of 60.0; with more blocks the longer steps win: L = 300 157 us with eight, 171 with four).
+// Loads of the next step in flight during the stores, or registers capped for a third block
+// per SM, spill and cost 5-9 us at L = 300.
+constexpr int kDigThreads = 384, kDigRows = 8, kDigRowsFew = 4, kDigGroups = 8, kDigGroupWords = 200;
 constexpr int dig_row_words(int gpb) { return (gpb * kDigGroupWords + 31) / 32 * 32 + 4; }
+template <int ROWS>
 __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs args) {
-  extern __shared__ __align__(16) int qs[];  // kDigRows rows of dig_row_words(gpb)
+  extern __shared__ __align__(16) int qs[];  // ROWS rows of dig_row_words(gpb)
   griddep_wait();
   griddep_launch();
   constexpr int kE = (kDigGroups * Groups192::kUsed + kDigThreads - 1) / kDigThreads;
@@ -315,14 +323,14 @@ __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs a
     }
   }
   // padding slots of the groups stay zero
-  for (int i = threadIdx.x; i < kDigRows * row_words; i += kDigThreads) qs[i] = 0;
+  for (int i = threadIdx.x; i < ROWS * row_words; i += kDigThreads) qs[i] = 0;
   const int k_rows = kQ * L;
   const float *x2 = args.sw.parity ? args.sw.at_x(1 - *args.sw.parity) + args.nsp : args.x2;
   const int r1 = min((int)(blockIdx.y + 1) * args.rows_per_block, k_rows);
-  for (int r0 = blockIdx.y * args.rows_per_block; r0 < r1; r0 += kDigRows) {
-    float v[kDigRows][kE];
+  for (int r0 = blockIdx.y * args.rows_per_block; r0 < r1; r0 += ROWS) {
+    float v[ROWS][kE];
 #pragma unroll
-    for (int i = 0; i < kDigRows; ++i) {
+    for (int i = 0; i < ROWS; ++i) {
       const int kr = min(r0 + i, r1 - 1);
       const float *row = x2 + ((long long)(kr % kQ) * L + kr / kQ) * kQPad * L;
 #pragma unroll
@@ -330,7 +338,7 @@ __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs a
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kDigRows; ++i)
+    for (int i = 0; i < ROWS; ++i)
 #pragma unroll
       for (int u = 0; u < kE; ++u)
         if (off[u] >= 0) {
@@ -339,9 +347,9 @@ __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs a
         }
     __syncthreads();
     // 16 slots of one row per thread: chunk (group, 32-slot atom), row, half
-    const int chunks = gpb * 6 * 2 * kDigRows;
+    const int chunks = gpb * 6 * 2 * ROWS;
     for (int u = threadIdx.x; u < chunks; u += kDigThreads) {
-      const int hc = u & 1, i = (u >> 1) & (kDigRows - 1), ga = u / (2 * kDigRows);
+      const int hc = u & 1, i = (u >> 1) & (ROWS - 1), ga = u / (2 * ROWS);
       const int g = ga / 6, c = ga % 6 * 32 + hc * 16;
       if (r0 + i >= r1 || t0 + g >= args.T) continue;
       const int *from = qs + i * row_words + g * kDigGroupWords + c;
@@ -1012,8 +1020,12 @@ __global__ void i8sp_onehot_kernel(const uint8_t *__restrict__ msa, uint32_t *__
 // storage above (no TMA swizzle: the images are stored swizzled).
 // One pass per tile: a stage holds everything one block of 128 logical K needs
 // for the three digit products (A x1, A x128, B d0..d2, E; 54 KB), so the one-hot
-// operand and its metadata cross L2 once per tile, not once per digit phase; the
-// kernel is bound by this L2 -> shared-memory operand stream.  The epilogue takes
+// operand and its metadata cross L2 once per tile, not once per digit phase.  Two
+// bounds lie close together (L = 300, N = 5000, 303 us; timing copies): the operand stream
+// alone, with two of the six MMAs, 254 us (all SMs together are at L2's throughput: an L2
+// prefetch makes it slower), and the MMAs alone, with 38 of the 54 KB loaded, 264 us
+// (sparse MMAs issue at 106 cycles each, 96 ideal, and wait for the issuing thread).  A
+// expanded into TMEM by four more warps (36 KB per block) took 304 us.  The epilogue takes
 // the sums out of both accumulators into registers and releases them at once, so the
 // next tile's MMAs overlap the softmax and the R digits.
 // TMEM: hi = [0, 192), lo = [256, 448), metadata slots at 456 and 460.
@@ -1392,7 +1404,7 @@ namespace ccm {
 // (SYM = false: the O^T R products only).  The sums are exact in s32 for up to
 // 32768 rows; longer alignments are cut into K chunks of that length, each merged
 // as (hi * 2^14 + lo) * 2^-21 (exact, one rounding) into FP32 registers.  The
-// output phase is tc_backward's: one atomic add per g2 element.
+// output phase (ccm_bwd_out.cuh) is one atomic add per g2 element.
 constexpr int kI8BwdBK = 32;
 constexpr int kI8BwdChunkKB = 1024;  // 32768 rows: |lo| <= 32768 * 2 * 16383 < 2^31
 
@@ -1407,13 +1419,6 @@ struct I8BwdSmem {
   static constexpr int kTotal = kTOff + kTBytes + 1024;
 };
 
-// CUT: a last wave of tiles that fills less than half of the pairs is cut along K (the rows):
-// every part is an entry of its own in the tile list, and the epilogue warp that finishes
-// a tile's part last adds the parts' integer sums (exact, so that the gradient is that of
-// the uncut tile bit for bit) and writes the output.
-// NAT: natural slots, K-major operands in the storage of i8nat_offset (the sparse
-// path); else Groups256 slots, row-major Npad x S operands (MN-major).  The MMAs run
-// at the same rate either way.
 // fx = sum(loss partials) + lambda1 sum V^2 + 0.5 lambda2 sum x2^2 in FP64, in a fixed
 // order, and the padding of g1 (the backward's output phase writes g1 itself); one warp.
 __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const float *x1, float *g1,
@@ -1458,6 +1463,17 @@ __device__ __forceinline__ void i8_backward_error(const BwdArgs &args, int *abor
   if (args.fin.host) *reinterpret_cast<volatile int *>(&args.fin.host->status) = kErrBwdTimeout;
 }
 
+// CUT: a last wave of tiles that fills less than half of the pairs is cut along K (the rows):
+// every part is an entry of its own in the tile list, and the epilogue warp that finishes
+// a tile's part last adds the parts' integer sums (exact, so that the gradient is that of
+// the uncut tile bit for bit) and writes the output.
+// NAT: natural slots, K-major operands in the storage of i8nat_offset (the sparse
+// path); else Groups256 slots, row-major Npad x S operands (MN-major).  The MMAs run
+// at the same rate either way.
+// Bound on the sparse path: the MMAs, 768 cycles of a K block's six (their issue rate is
+// the peak of kind::i8; at L = 1000 the power cap lowers the clock), then the last wave's
+// fill (i8_cut_parts) and, below N = 2000, the output phase of a pair's last tile.
+// L = 300, N = 5000 380 us, L = 253, N = 7001 391, L = 50, N = 200 23.
 template <bool SYM, bool NAT, bool CUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8_backward_kernel(const __grid_constant__ I8BwdMaps maps, BwdArgs args) {
@@ -1872,12 +1888,14 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
   const int gb = (c->T + kDigGroups - 1) / kDigGroups;  // blocks along the groups, evenly filled
   da.gpb = (c->T + gb - 1) / gb;
   const int row_tiles = (kQ * L + kDigRows - 1) / kDigRows;
+  const bool few = row_tiles * gb <= 2 * 148;
+  const int rows = few ? kDigRowsFew : kDigRows;
   const int per = (row_tiles * gb + 8 * 148 - 1) / (8 * 148);
-  da.rows_per_block = kDigRows * (per < 4 ? per : 4);
+  da.rows_per_block = rows * (per < 4 ? per : 4);
   count_launch(c, 2);
-  return launch_pdl(i8sp_digits_kernel,
+  return launch_pdl(few ? i8sp_digits_kernel<kDigRowsFew> : i8sp_digits_kernel<kDigRows>,
                     dim3(gb, (kQ * L + da.rows_per_block - 1) / da.rows_per_block),
-                    dim3(kDigThreads), sizeof(int) * kDigRows * dig_row_words(da.gpb), c->stream, da);
+                    dim3(kDigThreads), sizeof(int) * rows * dig_row_words(da.gpb), c->stream, da);
 }
 
 // A K block is 768 cycles of MMAs (not symmetric: 384), and cutting a tile in p saves
@@ -1980,8 +1998,10 @@ cudaError_t i8_configure_kernels() {
   // the staged row is S floats: up to L = 2688 (the 227 KB per block, less the
   // kernel's static reduction buffer)
   if ((e = cudaFuncSetAttribute(i8_prep_kernel, (cudaFuncAttribute)kMax, 230000)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(i8sp_digits_kernel, (cudaFuncAttribute)kMax,
-                                (int)sizeof(int) * kDigRows * dig_row_words(kDigGroups))) != cudaSuccess)
+      (e = cudaFuncSetAttribute(i8sp_digits_kernel<kDigRows>, (cudaFuncAttribute)kMax,
+                                (int)sizeof(int) * kDigRows * dig_row_words(kDigGroups))) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(i8sp_digits_kernel<kDigRowsFew>, (cudaFuncAttribute)kMax,
+                                (int)sizeof(int) * kDigRowsFew * dig_row_words(kDigGroups))) != cudaSuccess)
     return e;
   if ((e = cudaFuncSetAttribute(i8_forward_kernel, (cudaFuncAttribute)kMax, I8FwdSmem::kTotal)) !=
           cudaSuccess ||

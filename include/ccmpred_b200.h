@@ -180,7 +180,8 @@ CCM_API int ccm_calculate_weights(const unsigned char *msa, int ncol, int nrow, 
  * stream around every kernel of the next max_evals evaluations;
  * ccm_profile_end synchronises and returns, per kernel position in the
  * launch sequence, the summed device time in ms (tensor-core path: prep,
- * forward, backward, finalize; SIMT path: rows, pairs, single, sym,
+ * forward, backward, finalize -- CCM_PATH_TC_I8SP sums in the backward, its last
+ * interval is the gap between two events; SIMT path: rows, pairs, single, sym,
  * finalize), the number of kernels per evaluation and of evaluations seen. */
 CCM_API int ccm_profile_begin(ccm_context *ctx, int max_evals);
 CCM_API int ccm_profile_end(ccm_context *ctx, double *kernel_ms, int max_kernels, int *n_kernels,
