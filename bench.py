@@ -704,10 +704,10 @@ def main():
         if args.path == "tc_i8sp":
             # forward: 192-slot groups (9 columns) as N, K = 21 L padded to 256, three
             # 8-bit products at the 2:4-sparse rate (four times bf16): 0.75 per element;
-            # backward: the 192-slot groups padded to 256-slot tiles
+            # backward: 21 L + 1 natural slots padded to 256-slot tiles
             SW = 192 * ((L + 8) // 9)
             KP = (21 * L + 255) // 256 * 256
-            TB = (SW + 255) // 256
+            TB = (21 * L + 1 + 255) // 256
             executed = {"tc_forward": 2.0 * Npad * SW * KP * 0.75,
                         "tc_backward": TB * (TB + 1) / 2 * 256 * 256 * 2.0 * Npad * 2 * nsplit}[dom]
         else:
