@@ -169,7 +169,7 @@ __host__ __device__ constexpr long long i8sp_b_offset(int kr, int s, int KB) {
 // blocks steps the single fields), in a solve's trial after the update of s.  It also clears the result record.
 // Rows go in K-row order k * 21 + b backwards, so that the digits kernel's first rows
 // are the ones read last here and are still in L2.  HBM-bound.  Together with the
-// digits kernel 108 us at L = 253, N = 7001 and 151 us at L = 300; the column-maximum,
+// digits kernel 110 us at L = 253, N = 7001 and 144 us at L = 300; the column-maximum,
 // factor and row-per-block digit kernels before them took 226 us (scalar loads where
 // 4 does not divide L) and 165 us.  (The backward writing g2_scale * x2 + C itself, or
 // filling g2 while its MMAs run, saves this kernel 20 us at L = 300 and costs the
@@ -289,12 +289,14 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
 // multiple of 4 words apart modulo 32: no bank conflict), and 16 consecutive threads
 // write 256 contiguous bytes of a tile.  The first row of blocks also copies the column
 // maxima to `colmax`, which the forward reads: cmacc is cleared by the backward.
-// ROWS: eight, or four where eight leave blocks for less than two per SM
-// (L <= 72: 14.5 instead of 16.3 us for both kernels at L = 50, an evaluation 58.3 instead
-// of 60.0; with more blocks the longer steps win: L = 300 157 us with eight, 171 with four).
-// Loads of the next step in flight during the stores, or registers capped for a third block
-// per SM, spill and cost 5-9 us at L = 300.
-constexpr int kDigThreads = 384, kDigRows = 8, kDigRowsFew = 4, kDigGroups = 8, kDigGroupWords = 200;
+// ROWS: eight, or four where eight make less than eight blocks per SM (L <= 89; L = 60
+// 16.2 us for both kernels with four, 18.3 with eight; L = 300 144 with eight, 171 with four).
+// Small blocks, two groups each: the barriers between a step's loads, conversion and
+// stores stop 128 threads, not 384, and eight blocks fill an SM (scan and digits with
+// eight groups and 384 threads a block: 50 us at L = 150, 159 at L = 300; so 43 and 144;
+// one group and 64 threads 46 and 151).  Loads of the next step in flight during the
+// stores, or registers capped for more blocks, spill and cost 5-9 us at L = 300.
+constexpr int kDigThreads = 128, kDigRows = 8, kDigRowsFew = 4, kDigGroups = 2, kDigGroupWords = 200;
 constexpr int dig_row_words(int gpb) { return (gpb * kDigGroupWords + 31) / 32 * 32 + 4; }
 template <int ROWS>
 __global__ void __launch_bounds__(kDigThreads) i8sp_digits_kernel(I8DigitsArgs args) {
@@ -1888,9 +1890,9 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
   const int gb = (c->T + kDigGroups - 1) / kDigGroups;  // blocks along the groups, evenly filled
   da.gpb = (c->T + gb - 1) / gb;
   const int row_tiles = (kQ * L + kDigRows - 1) / kDigRows;
-  const bool few = row_tiles * gb <= 2 * 148;
+  const bool few = row_tiles * gb <= 8 * 148;
   const int rows = few ? kDigRowsFew : kDigRows;
-  const int per = (row_tiles * gb + 8 * 148 - 1) / (8 * 148);
+  const int per = (row_tiles * gb + 16 * 148 - 1) / (16 * 148);  // two waves of blocks
   da.rows_per_block = rows * (per < 4 ? per : 4);
   count_launch(c, 2);
   return launch_pdl(few ? i8sp_digits_kernel<kDigRowsFew> : i8sp_digits_kernel<kDigRows>,

@@ -1,5 +1,5 @@
 """The digits of W on both sides of the rule that takes four rows a step instead of
-eight (L <= 72: every row in one run of blocks), against the FP64 oracle."""
+eight (L <= 89), against the FP64 oracle."""
 import numpy as np
 import pytest
 
@@ -7,7 +7,7 @@ from ccmpred_b200 import Evaluator, nvar_padded, synth
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("L", [2, 9, 63, 72, 73, 112, 113])
+@pytest.mark.parametrize("L", [2, 9, 63, 72, 73, 89, 90, 112, 113])
 def test_digit_rows(gpu, oracle_mod, L):
     import torch
     msa = synth.generate(synth.MSAConfig("rows", L, 40, n_pairs=L // 8, dup_frac=0.2, seed=700 + L))
