@@ -430,11 +430,19 @@ int alloc_tc(ccm_context *c) {
     for (int P = 0; P < blocks; ++P)
       if (c->gradient == CCM_GRADIENT_PARTIAL || P <= Q) tiles.push_back(make_int2(P, Q));
   std::vector<int> cuts;  // outlives the copy below
-  const int parts = sp ? i8_cut_parts((int)tiles.size(), c->bwd_pairs, c->Npad,
-                                      c->gradient != CCM_GRADIENT_PARTIAL) : 1;
+  // (a context with a memory cap, or one whose sums do not fit, goes without: as much
+  // fits under the cap as without the sums)
+  int parts = sp && c->mem_limit == 0 ? i8_cut_parts((int)tiles.size(), c->bwd_pairs, c->Npad,
+                                                     c->gradient != CCM_GRADIENT_PARTIAL) : 1;
+  const int rest = (int)tiles.size() % c->bwd_pairs, whole = (int)tiles.size() - rest;
+  if (parts > 1 && dev_alloc(c, &c->d_cuts, sizeof(int) * cut_sums_offset(whole + rest * parts) +
+                                                kCutPartBytes * rest * parts) != cudaSuccess) {
+    (void)cudaGetLastError();
+    c->d_cuts = nullptr;
+    parts = 1;
+  }
   if (parts > 1) {
     // the tiles left over by whole waves, each as `parts` entries
-    const int rest = (int)tiles.size() % c->bwd_pairs, whole = (int)tiles.size() - rest;
     const std::vector<int2> over(tiles.begin() + whole, tiles.end());
     tiles.resize(whole);
     cuts.assign(whole, 1 << 8);
@@ -444,8 +452,6 @@ int alloc_tc(ccm_context *c) {
         cuts.push_back(p | parts << 8 | i << 16);
       }
     c->n_cut_tiles = rest;
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_cuts, sizeof(int) * cut_sums_offset((int)cuts.size()) +
-                                              kCutPartBytes * rest * parts));
     CCM_CUDA_TRY(cudaMemcpyAsync(c->d_cuts, cuts.data(), sizeof(int) * cuts.size(),
                                  cudaMemcpyHostToDevice, c->stream));
   }

@@ -32,3 +32,18 @@ def test_cut_tiles_are_bit_identical(gpu, L, N, gradient, max_sms):
                 got.append((f, g.cpu().numpy().copy()))
     for f, g in got[1:]:
         assert f == got[0][0] and np.array_equal(g, got[0][1])
+
+
+@pytest.mark.gpu
+def test_memory_cap_goes_without(gpu):
+    """A context with a memory cap keeps to the uncut schedule, with the same bits."""
+    import torch
+    L, N = 12, 9999
+    msa = synth.generate(synth.MSAConfig("cap", L, N, n_pairs=1, dup_frac=0.2, seed=13))
+    x = torch.from_numpy(synth.random_x(L, 14)).cuda()
+    got = []
+    for limit in (0, 40 << 20):  # the eight parts' sums and the operands do not both fit
+        with Evaluator(msa, mem_limit=limit) as ev:
+            g = torch.empty(nvar_padded(L), device="cuda")
+            got.append((ev.evaluate(x, g), g.cpu().numpy()))
+    assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])

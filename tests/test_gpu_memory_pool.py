@@ -11,29 +11,41 @@ from ccmpred_b200 import Evaluator, _lib, calculate_weights, lib, synth
 pytestmark = pytest.mark.gpu
 
 
-def work(L, N, seed):
+def buffers(L, seed):
     import torch
+    x = torch.from_numpy(synth.random_x(L, seed + 1)).cuda()
+    return x, torch.empty_like(x)
+
+
+def work(L, N, seed, x, g):
+    """(Only calls of the library: an operation on the legacy stream, as torch's own are,
+    is refused while another thread's solve captures its graph.)"""
     msa = synth.generate(synth.MSAConfig("pool", L, N, dup_frac=0.3, seed=seed))
     w = calculate_weights(msa, 0.8)
     with Evaluator(msa, weights=w) as ev:
-        x = torch.from_numpy(synth.random_x(L, seed + 1)).cuda()
-        g = torch.empty_like(x)
         f = ev.evaluate(x, g)
         r = ev.minimize(x, max_iterations=3, epsilon=0.0)
-        return f, r.fx, w, g.cpu().numpy(), x.cpu().numpy()
+        return f, r.fx, w
 
 
 @pytest.mark.parametrize("threads", [1, 4])
 def test_threads_share_the_pool(gpu, threads):
+    import torch
     sizes = [(20, 300, 1), (45, 700, 2), (64, 257, 3), (31, 1500, 4)]
-    alone = [work(*s) for s in sizes]
+    alone, first = [], []
+    for L, N, seed in sizes:
+        x, g = buffers(L, seed)
+        alone.append(work(L, N, seed, x, g))
+        first.append((x, g))
     assert lib().ccm_release_memory(0) == _lib.CCM_OK
-    got = [None] * len(sizes)
+    got = [[None, None] for _ in sizes]
+    own = [[buffers(L, seed) for _ in range(2)] for L, _, seed in sizes]
+    torch.cuda.synchronize()
 
     def run(k):
         for i in range(k, len(sizes), threads):
-            for _ in range(2):
-                got[i] = work(*sizes[i])
+            for rep in range(2):
+                got[i][rep] = work(*sizes[i], *own[i][rep])
                 assert lib().ccm_release_memory(0) == _lib.CCM_OK
 
     pool = [threading.Thread(target=run, args=(k,)) for k in range(threads)]
@@ -41,9 +53,12 @@ def test_threads_share_the_pool(gpu, threads):
         t.start()
     for t in pool:
         t.join()
-    for a, b in zip(alone, got):
-        assert a[:2] == b[:2]
-        assert all(np.array_equal(u.view(np.uint32), v.view(np.uint32)) for u, v in zip(a[2:], b[2:]))
+    torch.cuda.synchronize()
+    for a, vectors, both, mine in zip(alone, first, got, own):
+        for b, vecs in zip(both, mine):
+            assert a[:2] == b[:2] and np.array_equal(a[2], b[2])
+            for u, v in zip(vectors, vecs):
+                assert torch.equal(u.view(torch.int32), v.view(torch.int32))
 
 
 def test_release_rejects_a_bad_device(gpu):
