@@ -161,7 +161,8 @@ class Evaluator:
 
     def evaluate(self, x, g) -> float:
         """f at x, gradient written into g.  x, g: torch CUDA tensors (float32, or
-        float64 for the simt_f64 path) or numpy float32 host arrays."""
+        float64 for the simt_f64 path) or numpy float32 host arrays; g may be x itself,
+        but not overlap it in another way."""
         fx = ctypes.c_double(0.0)
         if isinstance(x, np.ndarray):
             assert x.dtype == np.float32 and g.dtype == np.float32

@@ -201,6 +201,7 @@ struct FinalizeArgs {
   ccm_result *out;
   ccm_result *host;    // the caller's copy in pinned memory, or null (finalize_host)
   double *block_part;  // kFinBlocks x 3 sums
+  const double *squares;  // sparse path: sum V^2 by lane, taken before g1 replaces V, or null
   unsigned *done;      // blocks finished (0 between evaluations)
 };
 

@@ -1421,6 +1421,31 @@ struct I8BwdSmem {
   static constexpr int kTotal = kTOff + kTBytes + 1024;
 };
 
+// sum V^2 of the single fields in FP64, in a fixed order, as each lane's part of it.
+__device__ __forceinline__ double i8nat_squares(const float *x1, int ns, int lane) {
+  double s = 0.0;
+  for (int i0 = lane; i0 < ns; i0 += 16 * 32) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = i0 + 32 * u < ns ? x1[i0 + 32 * u] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += (double)v[u] * (double)v[u];
+  }
+  return s;
+}
+
+// An evaluation whose gradient replaces its point (d_g == d_x): the scan leaves x as it is
+// (its g2 is 1 x), and this kernel, between the forward, the last to read x2 and all of V,
+// and the backward, which writes g1, makes g2 of it and takes each lane's sum of V^2.
+__global__ void __launch_bounds__(256) i8sp_in_place_kernel(float *g2, long long n, float g2_scale,
+                                                            const float *x1, int ns,
+                                                            double *squares) {
+  griddep_wait();
+  griddep_launch();
+  if (blockIdx.x == 0 && threadIdx.x < 32) squares[threadIdx.x] = i8nat_squares(x1, ns, threadIdx.x);
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) g2[i] *= g2_scale;
+}
+
 // fx = sum(loss partials) + lambda1 sum V^2 + 0.5 lambda2 sum x2^2 in FP64, in a fixed
 // order, and the padding of g1 (the backward's output phase writes g1 itself); one warp.
 __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const float *x1, float *g1,
@@ -1437,14 +1462,8 @@ __device__ __forceinline__ void i8nat_finalize(const FinalizeArgs &args, const f
     return s;
   };
   const int ns = (int)nsingle_of(args.L);
-  double acc[3] = {sum(args.part_f, args.n_part_f), sum(args.part_reg, args.n_part_reg), 0.0};
-  for (int i0 = lane; i0 < ns; i0 += 16 * 32) {
-    float v[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = i0 + 32 * u < ns ? x1[i0 + 32 * u] : 0.0f;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) acc[2] += (double)v[u] * (double)v[u];
-  }
+  double acc[3] = {sum(args.part_f, args.n_part_f), sum(args.part_reg, args.n_part_reg),
+                   args.squares ? args.squares[lane] : i8nat_squares(x1, ns, lane)};
   for (long long i = ns + lane; i < args.nsp; i += 32) g1[i] = 0.0f;
 #pragma unroll
   for (int k = 0; k < 3; ++k)
@@ -1855,11 +1874,15 @@ static int scan_rows(int L, int col_blocks) {
   return rows < 16 ? 16 : rows > 64 ? 64 : (rows + 7) / 8 * 8;
 }
 
+static float i8_g2_scale(const ccm_context *c) {
+  return (c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f) * c->lambda_pair;
+}
+
 static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2, const float *d_s,
                                      const double *d_alpha, float *d_xt, const CgTrialArgs *trial) {
   const int L = c->L;
   const bool step = d_s != nullptr || trial;
-  const float *xe = step ? d_xt : d_x;
+  const float *x2 = trial ? nullptr : (step ? d_xt : d_x) + c->nsp;
   I8ScanArgs sa{};
   sa.x = d_x; sa.s = const_cast<float *>(d_s); sa.alpha = d_alpha; sa.xt = d_xt;
   if (trial) {
@@ -1870,7 +1893,8 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
   sa.nsp = c->nsp; sa.L = L;
   sa.out_vecs = (int)(sizeof(ccm_result) + 4 * kCutCounters * c->n_cut_tiles + 15) / 16;
   sa.cols = (c->skip_padding ? kQ : kQPad) * L;
-  sa.g2_scale = (c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f) * c->lambda_pair;
+  // (over x itself: see i8sp_in_place_kernel)
+  sa.g2_scale = g2 && g2 == x2 ? 1.0f : i8_g2_scale(c);
   auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
   const CgSwap &w = sa.sw;
   sa.vec = ((bits(d_x) | bits(sa.s) | bits(d_xt) | bits(g2) | bits(w.x[0]) | bits(w.x[1]) |
@@ -1885,7 +1909,7 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
 
   I8DigitsArgs da{};
   for (int i = 0; i < 3; ++i) da.wdig[i] = c->d_wdig[i];
-  da.x2 = trial ? nullptr : xe + c->nsp; da.sw = sa.sw; da.nsp = c->nsp; da.cmacc = c->d_cmacc; da.colmax = c->d_colmax;
+  da.x2 = x2; da.sw = sa.sw; da.nsp = c->nsp; da.cmacc = c->d_cmacc; da.colmax = c->d_colmax;
   da.L = L; da.T = c->T; da.KB = c->KP / 128;
   const int gb = (c->T + kDigGroups - 1) / kDigGroups;  // blocks along the groups, evenly filled
   da.gpb = (c->T + gb - 1) / gb;
@@ -1976,6 +2000,14 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
     }
     ba.fin = finalize_args(c, x1, d_g, 2LL * pair_tiles);
     ba.fin.n_part_reg = c->n_part_reg;
+    if (g2 && g2 == x2) {
+      const long long n = c->nvarp - c->nsp, blocks = (n + 255) / 256;
+      ba.fin.squares = c->d_fin_part;
+      e = launch_pdl(i8sp_in_place_kernel, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), dim3(256),
+                     0, c->stream, g2, n, i8_g2_scale(c), x1, nsingle_of(L), c->d_fin_part);
+      if (e != cudaSuccess) return e;
+      count_launch(c);
+    }
   }
   const dim3 bgrid(2 * bpairs);
   auto bwd = sp && c->d_cuts ? (sym ? i8_backward_kernel<true, true, true>

@@ -135,7 +135,8 @@ CCM_API int ccm_create(ccm_context **ctx, const unsigned char *msa, int ncol, in
 CCM_API int ccm_destroy(ccm_context *ctx);
 
 /* f and g at x; x and g are DEVICE pointers of nvar_padded floats (the
- * conjugrad_gpu convention, src/evaluate_cuda.c:23-74).  g is overwritten.
+ * conjugrad_gpu convention, src/evaluate_cuda.c:23-74).  g is overwritten; it may be x
+ * itself (the gradient then replaces the point), but not overlap x in another way.
  * Blocks until the result is on the host; *fx receives f in FP64. */
 CCM_API int ccm_evaluate(ccm_context *ctx, const float *d_x, float *d_g, long long nvar_padded,
                  double *fx);
