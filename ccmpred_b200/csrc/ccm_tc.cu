@@ -14,6 +14,8 @@
 //
 // Semantics follow src/evaluate_cpu.c:16-166 (see oracle/ccm_oracle.c for the
 // line-by-line restatement used as the checker).
+#include <cfloat>
+
 #include <cuda_bf16.h>
 
 #include "ccm_bwd_out.cuh"
@@ -198,7 +200,8 @@ __device__ __forceinline__ bool aborted(const int *abort_flag) {
 
 // Forward epilogue for one warp: TMEM lane quarter q, column half `half` (tile columns
 // 128 half .. 128 half + 127).  The logits of the half are drained into registers and
-// the accumulator released; then per alignment column the maximum m of the own states,
+// the accumulator released; then per alignment column the maximum m of the own states
+// (from -FLT_MAX: fields of -inf may leave a half without one, whose share is then 0),
 // e = exp(logit - m) and its sum, (m, s) exchanged with the partner warp (same rows,
 // other half), and R = w (P - onehot), P = e exp(m - M) / S, as its bf16 terms.
 // Both halves run the same instructions: element i of half 1 is tile column 128 + i,
@@ -246,7 +249,7 @@ __device__ __forceinline__ bool fwd_epilogue_tile(const FwdArgs &args, uint32_t 
 
   float mx[kGroupCols], tg[kGroupCols], se[kGroupCols];
 #pragma unroll
-  for (int lj = 0; lj < kGroupCols; ++lj) { mx[lj] = -INFINITY; tg[lj] = 0.0f; se[lj] = 0.0f; }
+  for (int lj = 0; lj < kGroupCols; ++lj) { mx[lj] = -FLT_MAX; tg[lj] = 0.0f; se[lj] = 0.0f; }
 #pragma unroll
   for (int i4 = 0; i4 < kFwdHalfN; i4 += 4) {
     const float4 v4 = *reinterpret_cast<const float4 *>(Vs + half * kFwdHalfN + i4);

@@ -20,6 +20,7 @@
 // g2 <- 2 l2 x, sum x^2), forward, backward, finalize (shared with ccm_tc.cu); on the
 // sparse path four launches, scan (colmax, step, g2, sum x^2), digits, forward, backward
 // (with the sums of f and g1).
+#include <cfloat>
 #include <cmath>
 #include <type_traits>
 
@@ -628,7 +629,7 @@ __device__ __forceinline__ void i8_fwd_epilogue_tile(const I8FwdArgs &args, uint
   }
   float mx[kGroupCols], tg[kGroupCols], se[kGroupCols];
 #pragma unroll
-  for (int jj = 0; jj < kGroupCols; ++jj) { mx[jj] = -INFINITY; tg[jj] = 0.0f; se[jj] = 0.0f; }
+  for (int jj = 0; jj < kGroupCols; ++jj) { mx[jj] = -FLT_MAX; tg[jj] = 0.0f; se[jj] = 0.0f; }
   // merge + maxima
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
@@ -1060,7 +1061,8 @@ struct I8SpSmem {
 //          in flight; then both accumulators are released, so that the next tile's
 //          MMAs run during everything below;
 //   A      z = sum * scale + V; per alignment column the maximum m of the own states
-//          and the logit of the observed state;
+//          (from -FLT_MAX: fields of -inf may leave a half without one, whose share is
+//          then 0) and the logit of the observed state;
 //   B      e = exp(z - m), s = sum e; (m, s) exchanged with the partner warp (same
 //          rows, other half): M = max(m, m'), S = s exp(m - M) + s' exp(m' - M) (same
 //          order in both halves), lse = M + log S;
@@ -1129,7 +1131,7 @@ __device__ __forceinline__ bool i8sp_epilogue_tile(const I8FwdArgs &args, uint32
   // A
   float mx[kCols], tg[kCols], se[kCols];
 #pragma unroll
-  for (int lj = 0; lj < kCols; ++lj) { mx[lj] = -INFINITY; tg[lj] = 0.0f; se[lj] = 0.0f; }
+  for (int lj = 0; lj < kCols; ++lj) { mx[lj] = -FLT_MAX; tg[lj] = 0.0f; se[lj] = 0.0f; }
 #pragma unroll
   for (int i4 = 0; i4 < kSpHalf; i4 += 4) {
     const float4 sc = *reinterpret_cast<const float4 *>(tab_scale + half * kSpHalf + i4);
