@@ -177,6 +177,9 @@ __global__ void rw_weights_kernel(const int *__restrict__ counts, float *__restr
 
 cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int idthres,
                             int *d_counts, cudaStream_t stream) {
+  // identities are 0 .. L: a threshold beyond them is as good as one next to them (and
+  // L - idthres stays an int; NaN and what an int does not hold come as INT_MIN)
+  idthres = idthres < -1 ? -1 : idthres > L ? L : idthres;
   const int words = ((L + 31) / 32 + kRwWords - 1) / kRwWords * kRwWords;
   const size_t plane_bytes = sizeof(uint32_t) * 8 * (size_t)N * words;
   uint32_t *planes = nullptr;  // the planes, then the flag of states above 31
