@@ -9,6 +9,7 @@
 // count_i gets +1 for every j != i with ids > idthres and +2 for j == i (the
 // reference's i <= j loop visits the diagonal once and increments w[i] twice).
 // Counts are integers, so the order of the atomic additions does not matter.
+#include <climits>
 #include <cstdio>
 
 #include <cuda_runtime.h>
@@ -180,6 +181,8 @@ cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int 
   // identities are 0 .. L: a threshold beyond them is as good as one next to them (and
   // L - idthres stays an int; NaN and what an int does not hold come as INT_MIN)
   idthres = idthres < -1 ? -1 : idthres > L ? L : idthres;
+  const long long nb = (N + (long long)kRwTile - 1) / kRwTile, tiles = nb * (nb + 1) / 2;
+  if (tiles > INT_MAX) return cudaErrorInvalidConfiguration;  // 4,194,240 rows
   const int words = ((L + 31) / 32 + kRwWords - 1) / kRwWords * kRwWords;
   const size_t plane_bytes = sizeof(uint32_t) * 8 * (size_t)N * words;
   uint32_t *planes = nullptr;  // the planes, then the flag of states above 31
@@ -190,10 +193,8 @@ cudaError_t reweight_counts(int device, const uint8_t *d_msa, int L, int N, int 
   cudaMemsetAsync(d_counts, 0, sizeof(int) * N, stream);
   const long long warps = (long long)N * (words / kRwWords);
   rw_planes_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(d_msa, planes, high, L, N, words);
-  const long long nb = (N + kRwTile - 1) / kRwTile;
   constexpr int kSmem = 2 * 8 * kRwTile * kRwPitch * 4;  // 40 KB for eight planes
-  rw_count_kernel<<<(unsigned)(nb * (nb + 1) / 2), 256, kSmem, stream>>>(planes, high, N, L, words,
-                                                                        idthres, d_counts);
+  rw_count_kernel<<<(unsigned)tiles, 256, kSmem, stream>>>(planes, high, N, L, words, idthres, d_counts);
   cudaFreeAsync(planes, stream);
   return cudaGetLastError();
 }

@@ -1,10 +1,10 @@
-"""Sequence weights at thresholds past what an int holds."""
+"""Sequence weights at thresholds and row counts past what an int, or a grid, holds."""
 import ctypes
 
 import numpy as np
 import pytest
 
-from ccmpred_b200 import _lib, calculate_weights, lib, synth
+from ccmpred_b200 import CcmError, _lib, calculate_weights, lib, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +32,14 @@ def test_thresholds(gpu, threshold):
                                                d_w.data_ptr(), None) == _lib.CCM_OK
     torch.cuda.synchronize()
     assert np.array_equal(d_w.cpu().numpy(), expect)
+
+
+@pytest.mark.parametrize("N", [64 * 65535 + 1, 64 * 92682])
+def test_more_tiles_than_a_grid_holds(gpu, N):
+    """65536 blocks of rows have more tiles of pairs than a grid has blocks; those of 92682
+    are 2^32 + 55607, which as an unsigned number would pass for a few."""
+    with pytest.raises(CcmError) as err:
+        calculate_weights(np.zeros((N, 1), np.uint8))
+    assert err.value.code == _lib.CCM_ERR_CUDA
+    msa = synth.generate(synth.MSAConfig("lim", 10, 70, seed=2))
+    assert np.isfinite(calculate_weights(msa)).all()  # nothing of it is left behind
