@@ -138,6 +138,7 @@ struct I8PrepArgs {
   float lambda_pair;
   float g2_coef;
   int ncols;  // elements of a row that prep reads and writes: 32 L, or 21 L (padding skipped)
+  int vec;    // 4 divides L, and x2 and g2 are 16-byte aligned
 };
 
 struct I8FwdArgs {

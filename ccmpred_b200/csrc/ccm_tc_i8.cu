@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ 
   const float two_l2 = args.g2_coef * args.lambda_pair;
   const int nreal = kQ * L;
   double acc = 0.0;
-  if ((L & 3) == 0) {
+  if (args.vec) {
     const float4 *src = reinterpret_cast<const float4 *>(x2 + base);
     float4 *dst = reinterpret_cast<float4 *>(g2 + base);
     const int n4 = args.ncols / 4, nreal4 = nreal / 4;
@@ -1862,6 +1862,8 @@ static cudaError_t i8_prepare_dense(ccm_context *c, const float *d_x, float *g2,
   pa.g2_coef = c->gradient == CCM_GRADIENT_PARTIAL ? 1.0f : 2.0f;
   pa.inv_L = 1.0f / (float)L;
   pa.ncols = cols;
+  pa.vec = (L & 3) == 0 &&
+           ((reinterpret_cast<uintptr_t>(x2) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
   count_launch(c, 4);
   return launch_pdl(i8_prep_kernel, dim3(kQ * L), dim3(256), sizeof(float) * c->S, c->stream, x2, g2,
                     pa);
