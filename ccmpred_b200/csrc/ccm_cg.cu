@@ -47,12 +47,18 @@ int enqueue_evaluation_step(ccm_context *c, const float *d_x, const float *d_s,
 
 constexpr int kDotBlocks = 592;  // 4 x 148 SMs
 
-// x_t = x + alpha * s  (alpha read from device memory)
+static bool aligned16(const void *a, const void *b = nullptr, const void *c = nullptr) {
+  auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
+  return ((bits(a) | bits(b) | bits(c)) & 15) == 0;
+}
+
+// x_t = x + alpha * s  (alpha read from device memory); vec: all are 16-byte aligned (the
+// caller's x need not be)
 __global__ void cg_step_kernel(const float *__restrict__ x, const float *__restrict__ s,
                                const double *__restrict__ alpha, float *__restrict__ xt,
-                               long long n) {
+                               long long n, int vec) {
   const float a = (float)alpha[0];
-  const long long n4 = n / 4;
+  const long long n4 = vec ? n / 4 : 0;
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   const float4 *s4 = reinterpret_cast<const float4 *>(s);
   float4 *t4 = reinterpret_cast<float4 *>(xt);
@@ -402,8 +408,7 @@ void free_run(CgRun &r) {
 
 void launch_dots(CgRun &r, const float *a, const float *b, const float *c, const CgSwap &sw,
                  double *part) {
-  auto bits = [](const void *p) { return reinterpret_cast<uintptr_t>(p); };
-  const int vec = ((bits(a) | bits(b) | bits(c) | bits(sw.g[0]) | bits(sw.g[1])) & 15) == 0;
+  const int vec = aligned16(a, b, c) && aligned16(sw.g[0], sw.g[1]);
   cg_dots_kernel<<<kDotBlocks, 256, 0, r.c->stream>>>(a, b, c, sw, r.span, vec, part);
 }
 
@@ -434,7 +439,8 @@ int enqueue_trial(CgRun &r, int p, const CgRuleParams &rp, CgHandles h) {
   if (r.fused) {
     rc = enqueue_evaluation_step(c, x, r.s, &r.d_ctl->alpha, xt, gt);
   } else {
-    cg_step_kernel<<<grid_for(r.n), 256, 0, s>>>(x, r.s, &r.d_ctl->alpha, xt, r.n);
+    cg_step_kernel<<<grid_for(r.n), 256, 0, s>>>(x, r.s, &r.d_ctl->alpha, xt, r.n,
+                                                 aligned16(x, r.s, xt));
     rc = enqueue_evaluation(c, xt, gt);
   }
   if (rc != CCM_OK) return rc;
@@ -923,7 +929,7 @@ int ccm::conjugrad_callback_gpu(float *d_x, long long n, ccm_eval_callback eval,
   cudaStream_t s = 0;  // legacy default stream
   const size_t bytes = sizeof(float) * (size_t)n;
   const VecSpan flat{n, 0, 0, 0, 0};  // a foreign evaluation: every element
-  const int vec = (reinterpret_cast<uintptr_t>(d_x) & 15) == 0;
+  const int vec = aligned16(d_x);
   float *xb[2] = {d_x, nullptr}, *gb[2] = {nullptr, nullptr}, *dir = nullptr;
   CgCtl *d_ctl = nullptr;
   double *d_part = nullptr, *d_f = nullptr;
@@ -956,7 +962,7 @@ int ccm::conjugrad_callback_gpu(float *d_x, long long n, ccm_eval_callback eval,
   while (e == cudaSuccess && h->status == kCgRunning) {
     const int p = h->parity, iter0 = h->iter;
     cg_dir_kernel<<<grid_for(n), 256, 0, s>>>(gb[p], dir, d_ctl, flat);
-    cg_step_kernel<<<grid_for(n), 256, 0, s>>>(xb[p], dir, &d_ctl->alpha, xb[1 - p], n);
+    cg_step_kernel<<<grid_for(n), 256, 0, s>>>(xb[p], dir, &d_ctl->alpha, xb[1 - p], n, vec);
     e = evaluate(1 - p);
     if (e != cudaSuccess) break;
     cg_dots_kernel<<<kDotBlocks, 256, 0, s>>>(gb[1 - p], dir, gb[p], CgSwap{}, flat, vec, d_part);
