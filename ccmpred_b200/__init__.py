@@ -120,6 +120,7 @@ class Evaluator:
                  path: str = "tc_i8sp", device: int = 0, stream: Optional[int] = None,
                  gradient: str = "tied", max_sms: int = 0, mem_limit: int = 0):
         self._ctx = ctypes.c_void_p(None)
+        self.device = device
         self.msa = np.ascontiguousarray(msa, dtype=np.uint8)
         self.N, self.L = self.msa.shape
         self.path = path
@@ -150,6 +151,8 @@ class Evaluator:
                                self.L, self.N, wptr, ctypes.byref(opt)))
         if weights is None:
             self.weights = np.ones(self.N, dtype=np.float32)
+        self._stream = self.stream or 0
+        self._own_stream = not stream
 
     @property
     def handle(self) -> ctypes.c_void_p:
@@ -159,8 +162,21 @@ class Evaluator:
     def stream(self) -> int:
         return lib().ccm_stream(self._ctx)
 
+    def _after_torch(self, t) -> None:
+        """The context's stream waits for what torch's current stream has still to do, on x
+        and to the memory that g was given.  (Its own stream and torch's default one, the
+        legacy stream, are ordered by themselves.)"""
+        import torch
+        device = t.get_device()
+        current = torch._C._cuda_getCurrentRawStream(device)
+        if device == self.device and (self._own_stream if current == 0 else current == self._stream):
+            return
+        torch.cuda.ExternalStream(self._stream, device=self.device).wait_stream(
+            torch.cuda.current_stream(t.device))
+
     def evaluate(self, x, g) -> float:
-        """f at x, gradient written into g.  x, g: torch CUDA tensors (float32, or
+        """f at x, gradient written into g, after torch's current stream and complete on
+        return.  x, g: torch CUDA tensors (float32, or
         float64 for the simt_f64 path) or numpy float32 host arrays; g may be x itself,
         but not overlap it in another way."""
         fx = ctypes.c_double(0.0)
@@ -172,6 +188,7 @@ class Evaluator:
                                           x.size, ctypes.byref(fx)))
             return fx.value
         assert x.is_cuda and g.is_cuda and x.is_contiguous() and g.is_contiguous()
+        self._after_torch(x)
         if self.path == "simt_f64":
             check(lib().ccm_evaluate_f64(self._ctx, x.data_ptr(), g.data_ptr(), x.numel(),
                                          ctypes.byref(fx)))
@@ -197,11 +214,14 @@ class Evaluator:
             def _cb(inst, xp, gp, fx, xnorm, gnorm, step, n, kk, ls):
                 return 1 if progress(kk, ls, fx, xnorm, gnorm, step) else 0
             cb = _lib.PROGRESS(_cb)
+        self._after_torch(x)
         check(lib().ccm_conjugrad_gpu(self._ctx, x.data_ptr(), x.numel(), ctypes.byref(p), cb,
                                       None, ctypes.byref(res)))
         return res
 
     def evaluate_async(self, x, g) -> None:
+        """Enqueued on the context's stream and nothing else: the caller orders other
+        streams' work on x and g with it."""
         check(lib().ccm_evaluate_async(self._ctx, x.data_ptr(), g.data_ptr(), x.numel()))
 
     def result(self) -> "_lib.CcmResult":
