@@ -101,6 +101,15 @@ void pool_batch_end(int device) {
   cudaMemPoolTrimTo(pool, kPoolKeep);
 }
 
+size_t pool_unused(int device) {
+  cudaMemPool_t pool = library_pool(device);
+  uint64_t reserved = 0, used = 0;
+  if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
 cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream) {
   cudaMemPool_t pool = library_pool(device);
   if (!pool) return cudaMallocAsync(p, bytes, stream);

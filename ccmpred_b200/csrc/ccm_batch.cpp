@@ -62,6 +62,14 @@ struct WaveItem {
   ccm::CgGraphSolve *gs = nullptr;
 };
 
+// Device bytes that the waves of a batch take by default: 60 % of what is free, to the
+// driver or in the library's own pool.
+size_t wave_budget(int device) {
+  size_t mem_free = 0, mem_total = 0;
+  cudaMemGetInfo(&mem_free, &mem_total);
+  return (mem_free + ccm::pool_unused(device)) / 10 * 6;
+}
+
 // Alignments in waves, each wave ONE graph launch: the contexts and device x of a
 // wave are set up on one stream, then every alignment's whole device-side solve
 // (initial evaluation, the iteration loop in conditional nodes, the final x) and
@@ -75,9 +83,7 @@ int solve_waves(int n, const ccm_msa_desc *msas, const ccm_batch_params *params,
   const int dev = params->device;
   if (cudaSetDevice(dev) != cudaSuccess)
     return set_last_error(CCM_ERR_CUDA, "ccm_solve_batch: cannot select device %d", dev);
-  size_t mem_free = 0, mem_total = 0;
-  cudaMemGetInfo(&mem_free, &mem_total);
-  const size_t budget = params->wave_bytes > 0 ? params->wave_bytes : mem_free / 10 * 6;
+  const size_t budget = params->wave_bytes > 0 ? params->wave_bytes : wave_budget(dev);
   const int wave_max = params->wave_max > 0 ? params->wave_max : 64;
   pool_batch_begin(dev);
   cudaStream_t stream = nullptr;
@@ -223,6 +229,12 @@ void ccm_batch_params_default(ccm_batch_params *p) {
   p->wave_max = 64;
   p->wave_bytes = 0;
   ccm_cg_params_default(&p->cg);
+}
+
+long long ccm_debug_wave_budget(int device) {
+  if (cudaSetDevice(device) != cudaSuccess)
+    return ccm::set_last_error(CCM_ERR_CUDA, "ccm_debug_wave_budget: cannot select device %d", device);
+  return (long long)wave_budget(device);
 }
 
 int ccm_solve_batch(int n, const ccm_msa_desc *msas, const ccm_batch_params *params,

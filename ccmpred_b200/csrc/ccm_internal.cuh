@@ -235,6 +235,8 @@ void prof_mark(ccm_context *c);
 // on its stream and counted against its limit.
 cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream);
 cudaError_t dev_alloc_raw(ccm_context *c, void **p, size_t bytes);
+// Bytes that the pool keeps mapped and nobody uses: the driver counts them as taken.
+size_t pool_unused(int device);
 // While a batch runs, the pool keeps all freed memory mapped.
 void pool_batch_begin(int device);
 void pool_batch_end(int device);

@@ -218,6 +218,8 @@ CCM_API int ccm_debug_set_wait_limit(ccm_context *ctx, long long cycles);
  * (allow = 1, the default).  allow = 0 makes the solve visit every element, for
  * comparisons; results agree up to the summation order of the FP64 dots. */
 CCM_API int ccm_debug_set_cg_skip_padding(ccm_context *ctx, int allow);
+/* Diagnostics for tests: the device bytes that ccm_solve_batch's waves take by default. */
+CCM_API long long ccm_debug_wave_budget(int device);
 
 /* Allocation-free sequence reweighting.  No counterpart in the reference.
  *
