@@ -9,7 +9,9 @@ used by the tests, the benchmark and the ``torch.autograd.Function`` wrapper:
   ``src/evaluate_cuda.c:23``) for device (torch CUDA tensors) or host (numpy)
   buffers in the reference's padded layout;
 * :func:`calculate_weights` -- bit-exact GPU sequence reweighting
-  (``src/reweighting.c:9-58``).
+  (``src/reweighting.c:9-58``);
+* :func:`solve_batch` -- many alignments to convergence;
+* :func:`release_memory` -- the device memory kept between calls, given back.
 """
 from __future__ import annotations
 
@@ -54,6 +56,12 @@ def calculate_weights(msa: np.ndarray, threshold: float = 0.8, device: int = 0) 
                                       ctypes.c_float(threshold),
                                       w.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), device))
     return w
+
+
+def release_memory(device: int = 0) -> None:
+    """Give the device memory that the library keeps for its next calls (up to 4 GB) back:
+    for an allocator beside it, such as torch's, that needs it."""
+    check(lib().ccm_release_memory(device))
 
 
 def solve_batch(msas, workers: int = 8, path: str = "tc_i8sp", threshold: float = 0.8,
