@@ -831,8 +831,10 @@ int ccm::create_context(ccm_context **out, const unsigned char *msa, int ncol, i
   CCM_CTX_TRY(cudaMemcpyAsync(c->d_msa, msa, (size_t)ncol * nrow, cudaMemcpyHostToDevice, c->stream));
   CCM_CTX_TRY(dev_alloc(c, &c->d_w, sizeof(float) * nrow));
   CCM_CTX_TRY(cudaMemcpyAsync(c->d_w, c->h_w, sizeof(float) * nrow, cudaMemcpyHostToDevice, c->stream));
-  // behind it the counters of the sparse backward's cut tiles (BwdArgs::cuts)
-  CCM_CTX_TRY(dev_alloc(c, &c->d_out, kResultBytes));
+  // behind it the counters of the sparse backward's cut tiles (BwdArgs::cuts; without a
+  // memory cap, see alloc_tc)
+  const bool may_cut = c->path == CCM_PATH_TC_I8SP && c->mem_limit == 0;
+  CCM_CTX_TRY(dev_alloc(c, &c->d_out, may_cut ? kResultBytes : sizeof(ccm_result)));
   CCM_CTX_TRY(cudaMemsetAsync(c->d_out, 0, sizeof(ccm_result), c->stream));
   c->h_out = static_cast<ccm_result *>(pinned_small_alloc(sizeof(ccm_result)));
   if (!c->h_out) return fail(set_error(CCM_ERR_NOMEM, "pinned result record"));
