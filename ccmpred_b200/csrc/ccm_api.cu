@@ -1160,6 +1160,13 @@ int ccm_debug_set_wait_limit(ccm_context *c, long long cycles) {
   return CCM_OK;
 }
 
+int ccm_debug_set_backward_wait_limit(ccm_context *c, long long cycles) {
+  if (!c || cycles < 0 || cycles > INT_MAX)
+    return set_error(CCM_ERR_INVALID, "ccm_debug_set_backward_wait_limit: invalid arguments");
+  c->bwd_wait_cycles = (int)cycles;
+  return CCM_OK;
+}
+
 int ccm_debug_set_cg_skip_padding(ccm_context *c, int allow) {
   if (!c) return set_error(CCM_ERR_INVALID, "ccm_debug_set_cg_skip_padding: null context");
   c->cg_skip_padding = allow != 0;

@@ -207,13 +207,12 @@ struct FinalizeArgs {
 };
 
 struct BwdArgs {
-  const float *x2;
   float *g2;
   float *g1d;
   const int2 *tiles;
   int *status;
   int n_tiles, L, S, Npad;
-  float lambda_pair;
+  int acc_wait_cycles;  // integer path: as I8FwdArgs::acc_wait_cycles
   float r_dec;  // integer path: 2^(eR - 21), the inverse of I8FwdArgs::r_enc
   // sparse path: g2 is 16-byte aligned; cmacc is cleared; fin: the sums of f, and g1
   int vec;
@@ -357,6 +356,7 @@ struct ccm_context {
   long long nsingle = 0, nsp = 0, nvarp = 0;
   int r_exp = 0;                   // eR of the integer path's R digits: 2^eR >= max |w|
   long long acc_wait_cycles = 0;   // ccm_debug_set_wait_limit (0: default budget)
+  int bwd_wait_cycles = 0;            // ccm_debug_set_backward_wait_limit
   float lambda_single = 0.01f, lambda_pair = 0.0f;
 
   uint8_t *d_msa = nullptr;       // N x L

@@ -863,9 +863,8 @@ static cudaError_t launch_tc(ccm_context *c, const float *d_x, float *d_g,
   prof_mark(c);
 
   BwdArgs ba{};
-  ba.x2 = x2; ba.g2 = g2; ba.g1d = c->d_g1d; ba.tiles = c->d_bwd_tiles;
+  ba.g2 = g2; ba.g1d = c->d_g1d; ba.tiles = c->d_bwd_tiles;
   ba.n_tiles = c->n_bwd_tiles; ba.status = c->d_status; ba.L = L; ba.S = c->S; ba.Npad = c->Npad;
-  ba.lambda_pair = c->lambda_pair;
   const int bwd_pairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
   e = launch_pdl(c->gradient == CCM_GRADIENT_PARTIAL ? tc_backward_kernel<NSPLIT, false>
                                                      : tc_backward_kernel<NSPLIT, true>,

@@ -1510,7 +1510,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
   uint64_t *acc_full = empty + kStages;
   uint64_t *acc_empty = acc_full + 1;
   uint64_t *drain = acc_empty + 1;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+  // as in the forward: waited on instead of acc_full when a test asks for a wait that runs
+  // out (acc_wait_cycles)
+  uint64_t *never = drain + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(never + 1);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1528,6 +1531,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, 16);
     mbar_init(drain, 1);
+    mbar_init(never, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -1680,11 +1684,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     float *g1 = args.sw.parity ? args.sw.at_g(buf) : args.fin.g1;
     uint32_t chunk = 0;
     bool ok = true;
+    // (as instances of their own, the waits of a test cost an evaluation 0.7 us at L = 50 and
+    // 1.6 at L = 150: more kernels in the module; as an argument nothing)
+    auto acc_ready = [&] {
+      return args.acc_wait_cycles ? mbar_wait(never, 0, args.acc_wait_cycles) : mbar_wait(acc_full, chunk & 1);
+    };
     for (int tile = pair; tile < n_tiles && ok; tile += npairs) {
       float accv[kHalfN];
       // one K chunk: wait for it, merge it into accv (or add it there), release it
       auto take = [&](auto first) {
-        const bool w_ok = mbar_wait(acc_full, chunk & 1);
+        const bool w_ok = acc_ready();
         if (__any_sync(0xffffffffu, !w_ok)) {
           if (lane == 0) i8_backward_error(args, abort_flag);
           return false;
@@ -1719,7 +1728,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
       // already; the warp that finishes last adds the parts' integers (exact, in any
       // order) and goes on to the output.  Nobody waits.  0: error, 1: not last, 2: last.
       auto take_part = [&](int cut) {
-        const bool w_ok = mbar_wait(acc_full, chunk & 1);
+        const bool w_ok = acc_ready();
         if (__any_sync(0xffffffffu, !w_ok)) {
           if (lane == 0) i8_backward_error(args, abort_flag);
           return 0;
@@ -1949,6 +1958,13 @@ int i8_cut_parts(int tiles, int pairs, int Npad, bool sym) {
   return best;
 }
 
+static auto backward_kernel(bool sym, bool sp, bool cut) {
+  return sp && cut ? (sym ? i8_backward_kernel<true, true, true> : i8_backward_kernel<false, true, true>)
+         : sp      ? (sym ? i8_backward_kernel<true, true, false> : i8_backward_kernel<false, true, false>)
+         : sym     ? i8_backward_kernel<true, false, false>
+                   : i8_backward_kernel<false, false, false>;
+}
+
 cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const float *d_s,
                         const double *d_alpha, float *d_xt, const CgTrialArgs *trial) {
   const int L = c->L;
@@ -1987,10 +2003,10 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
   prof_mark(c);
 
   BwdArgs ba{};
-  ba.x2 = x2; ba.g2 = g2; ba.g1d = c->d_g1d; ba.tiles = c->d_bwd_tiles;
+  ba.g2 = g2; ba.g1d = c->d_g1d; ba.tiles = c->d_bwd_tiles;
   ba.n_tiles = c->n_bwd_tiles; ba.status = c->d_status; ba.L = L; ba.S = c->S; ba.Npad = c->Npad;
-  ba.lambda_pair = c->lambda_pair;
   ba.r_dec = pow2_host(c->r_exp - kI8FracBits);
+  ba.acc_wait_cycles = c->bwd_wait_cycles;
   const int bpairs = c->n_bwd_tiles < c->bwd_pairs ? c->n_bwd_tiles : c->bwd_pairs;
   const bool sym = c->gradient != CCM_GRADIENT_PARTIAL;
   if (sp) {
@@ -2014,12 +2030,7 @@ cudaError_t i8_evaluate(ccm_context *c, const float *d_x, float *d_g, const floa
     }
   }
   const dim3 bgrid(2 * bpairs);
-  auto bwd = sp && c->d_cuts ? (sym ? i8_backward_kernel<true, true, true>
-                                    : i8_backward_kernel<false, true, true>)
-             : sp            ? (sym ? i8_backward_kernel<true, true, false>
-                                    : i8_backward_kernel<false, true, false>)
-             : sym           ? i8_backward_kernel<true, false, false>
-                             : i8_backward_kernel<false, false, false>;
+  const auto bwd = backward_kernel(sym, sp, c->d_cuts != nullptr);
   e = launch_pdl(bwd, bgrid, dim3(kWgThreads), I8BwdSmem::kTotal, c->stream, c->i8bwd_maps, ba);
   if (e != cudaSuccess) return e;
   prof_mark(c);
@@ -2046,10 +2057,9 @@ cudaError_t i8_configure_kernels() {
       (e = cudaFuncSetAttribute(i8sp_forward_kernel, (cudaFuncAttribute)kMax, I8SpSmem::kTotal)) !=
           cudaSuccess)
     return e;
-  for (auto bwd : {i8_backward_kernel<true, false, false>, i8_backward_kernel<false, false, false>,
-                   i8_backward_kernel<true, true, false>, i8_backward_kernel<false, true, false>,
-                   i8_backward_kernel<true, true, true>, i8_backward_kernel<false, true, true>})
-    if ((e = cudaFuncSetAttribute(bwd, (cudaFuncAttribute)kMax, I8BwdSmem::kTotal)) != cudaSuccess)
+  for (int i = 0; i < 8; ++i)
+    if ((e = cudaFuncSetAttribute(backward_kernel(i & 1, i & 2, i & 4), (cudaFuncAttribute)kMax,
+                                  I8BwdSmem::kTotal)) != cudaSuccess)
       return e;
   return cudaSuccess;
 }
@@ -2078,7 +2088,7 @@ cudaError_t i8_backward_max_pairs(int *pairs) {
   cfg.blockDim = dim3(kWgThreads, 1, 1);
   cfg.dynamicSmemBytes = I8BwdSmem::kTotal;
   *pairs = 0;
-  return cudaOccupancyMaxActiveClusters(pairs, i8_backward_kernel<true, false, false>, &cfg);
+  return cudaOccupancyMaxActiveClusters(pairs, backward_kernel(true, false, false), &cfg);
 }
 
 // One-hot operands for a context of the integer paths (Npad x S bytes each), and

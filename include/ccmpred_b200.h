@@ -211,6 +211,8 @@ CCM_API long long ccm_debug_copy(ccm_context *ctx, int which, void *dst, long lo
  * normal evaluations; the context stays usable.  No counterpart in the
  * reference (which has no bounded waits). */
 CCM_API int ccm_debug_set_wait_limit(ccm_context *ctx, long long cycles);
+/* The same for the backward kernel's epilogue. */
+CCM_API int ccm_debug_set_backward_wait_limit(ccm_context *ctx, long long cycles);
 
 /* Integer paths: a device-side solve (ccm_conjugrad_gpu, ccm_solve_batch) whose
  * x0 has zero padding states (a in [21, 32) of every coupling row; always so on
