@@ -170,15 +170,22 @@ class Evaluator:
     def stream(self) -> int:
         return lib().ccm_stream(self._ctx)
 
+    @staticmethod
+    def _current_stream(device: int) -> int:
+        """Handle of torch's current stream; looked up in torch at the first call."""
+        from torch._C import _cuda_getCurrentRawStream
+        Evaluator._current_stream = staticmethod(_cuda_getCurrentRawStream)
+        return _cuda_getCurrentRawStream(device)
+
     def _after_torch(self, t) -> None:
         """The context's stream waits for what torch's current stream has still to do, on x
         and to the memory that g was given.  (Its own stream and torch's default one, the
         legacy stream, are ordered by themselves.)"""
-        import torch
         device = t.get_device()
-        current = torch._C._cuda_getCurrentRawStream(device)
+        current = self._current_stream(device)
         if device == self.device and (self._own_stream if current == 0 else current == self._stream):
             return
+        import torch
         torch.cuda.ExternalStream(self._stream, device=self.device).wait_stream(
             torch.cuda.current_stream(t.device))
 
