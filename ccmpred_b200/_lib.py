@@ -153,6 +153,8 @@ SIGNATURES = {
     "ccm_launch_count": (ctypes.c_longlong, [_vp]),
     "ccm_debug_set_wait_limit": (ctypes.c_int, [_vp, ctypes.c_longlong]),
     "ccm_debug_set_backward_wait_limit": (ctypes.c_int, [_vp, ctypes.c_longlong]),
+    "ccm_debug_cut_tiles": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_int)]),
+    "ccm_debug_fail_allocation": (ctypes.c_int, [ctypes.c_int]),
     "ccm_debug_set_cg_skip_padding": (ctypes.c_int, [_vp, ctypes.c_int]),
     "ccm_debug_wave_budget": (ctypes.c_longlong, [ctypes.c_int]),
     "ccm_host_copy_bytes": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_longlong),

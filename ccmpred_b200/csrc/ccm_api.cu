@@ -123,7 +123,11 @@ cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream) 
   return e;
 }
 
+// ccm_debug_fail_allocation: counted down to the allocation that fails, on this thread
+static thread_local int fail_allocation = 0;
+
 cudaError_t dev_alloc_raw(ccm_context *c, void **p, size_t bytes) {
+  if (fail_allocation > 0 && --fail_allocation == 0) return cudaErrorMemoryAllocation;
   // the cap of ccm_options.mem_limit: the bytes this context holds
   if (c->mem_limit > 0 && c->mem_used + bytes > c->mem_limit) return cudaErrorMemoryAllocation;
   const cudaError_t e = pool_alloc(c->device, p, bytes, c->stream);
@@ -461,6 +465,7 @@ int alloc_tc(ccm_context *c) {
         cuts.push_back(p | parts << 8 | i << 16);
       }
     c->n_cut_tiles = rest;
+    c->n_cut_parts = parts;
     CCM_CUDA_TRY(cudaMemcpyAsync(c->d_cuts, cuts.data(), sizeof(int) * cuts.size(),
                                  cudaMemcpyHostToDevice, c->stream));
   }
@@ -1165,6 +1170,18 @@ int ccm_debug_set_backward_wait_limit(ccm_context *c, long long cycles) {
     return set_error(CCM_ERR_INVALID, "ccm_debug_set_backward_wait_limit: invalid arguments");
   c->bwd_wait_cycles = (int)cycles;
   return CCM_OK;
+}
+
+int ccm_debug_cut_tiles(const ccm_context *c, int *parts) {
+  if (!c) return set_error(CCM_ERR_INVALID, "ccm_debug_cut_tiles: null context");
+  if (parts) *parts = c->n_cut_parts;
+  return c->n_cut_tiles;
+}
+
+int ccm_debug_fail_allocation(int nth) {
+  const int left = fail_allocation;
+  fail_allocation = nth;
+  return left;
 }
 
 int ccm_debug_set_cg_skip_padding(ccm_context *c, int allow) {

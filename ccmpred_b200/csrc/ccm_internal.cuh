@@ -405,7 +405,7 @@ struct ccm_context {
   int SB = 0;
   uint8_t *d_onat = nullptr, *d_rnat = nullptr;
   int *d_cuts = nullptr;            // its tiles cut along the rows (BwdArgs::cuts)
-  int n_cut_tiles = 0;
+  int n_cut_tiles = 0, n_cut_parts = 1;
   uint8_t *d_ac1 = nullptr, *d_ac128 = nullptr, *d_meta = nullptr;
   ccm::I8SpMaps i8sp_maps;
 

@@ -214,6 +214,13 @@ CCM_API int ccm_debug_set_wait_limit(ccm_context *ctx, long long cycles);
 /* The same for the backward kernel's epilogue. */
 CCM_API int ccm_debug_set_backward_wait_limit(ccm_context *ctx, long long cycles);
 
+/* Diagnostics for tests.  The number of the backward's tiles that are cut along the rows
+ * (0: none), each into *parts; and a failing device allocation: the nth that a context
+ * makes from now on, on the calling thread, is refused as if the device were full (0:
+ * none).  The latter returns how many were left to go. */
+CCM_API int ccm_debug_cut_tiles(const ccm_context *ctx, int *parts);
+CCM_API int ccm_debug_fail_allocation(int nth);
+
 /* Integer paths: a device-side solve (ccm_conjugrad_gpu, ccm_solve_batch) whose
  * x0 has zero padding states (a in [21, 32) of every coupling row; always so on
  * the reference's CLI path) keeps them zero and skips them in every vector pass
