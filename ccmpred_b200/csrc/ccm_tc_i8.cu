@@ -164,10 +164,11 @@ __host__ __device__ constexpr long long i8sp_b_offset(int kr, int s, int KB) {
 //
 // i8sp_scan_kernel, one pass over x (row blocks of its 21 L coupling rows, four columns
 // per thread, eight rows of loads in flight): column maxima of |W| into cmacc (float
-// bits, atomicMax; zero between evaluations), sum x^2 partials (in FP64; where 4 divides
-// L, four squares in float and their sum in FP64), the regulariser gradient g2 <- g2_scale * x2 (the backward adds C to
-// it), and, STEP, the CG trial step v = fmaf(alpha, s, x) into xt (the last row of
-// blocks steps the single fields), in a solve's trial after the update of s.  It also clears the result record.
+// bits, atomicMax; zero between evaluations), sum x^2 partials (FP64 squares: float ones
+// of four columns at a time are no faster), the regulariser gradient g2 <- g2_scale * x2
+// (the backward adds C to it), and, STEP, the CG trial step v = fmaf(alpha, s, x) into xt
+// (the last row of blocks steps the single fields), in a solve's trial after the update
+// of s.  It also clears the result record.
 // Rows go in K-row order k * 21 + b backwards, so that the digits kernel's first rows
 // are the ones read last here and are still in L2.  HBM-bound.  Together with the
 // digits kernel 110 us at L = 253, N = 7001 and 144 us at L = 300; the column-maximum,
@@ -253,11 +254,8 @@ __global__ void __launch_bounds__(256) i8sp_scan_kernel(I8ScanArgs args) {
                              fmaf(alpha, sv[u].z, v[u].z), fmaf(alpha, sv[u].w, v[u].w));
           store(xt + args.nsp + c + at[u], v[u]);
         }
-        if ((L & 3) == 0)
-          acc += (double)fmaf(v[u].w, v[u].w, fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
-        else
-          acc += ((double)v[u].x * v[u].x + (double)v[u].y * v[u].y) +
-                 ((double)v[u].z * v[u].z + (double)v[u].w * v[u].w);
+        acc += ((double)v[u].x * v[u].x + (double)v[u].y * v[u].y) +
+               ((double)v[u].z * v[u].z + (double)v[u].w * v[u].w);
         m[0] = fmaxf(m[0], fabsf(v[u].x));
         m[1] = fmaxf(m[1], fabsf(v[u].y));
         m[2] = fmaxf(m[2], fabsf(v[u].z));
@@ -412,9 +410,8 @@ __global__ void __launch_bounds__(256) i8_prep_kernel(const float *__restrict__ 
       for (int u = 0; u < kU; ++u) {
         const int i = i0 + u * blockDim.x;
         if (i < n4) {
-          // four squares in float, their sum added in FP64
-          acc += (double)fmaf(v[u].w, v[u].w,
-                              fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
+          acc += ((double)v[u].x * v[u].x + (double)v[u].y * v[u].y) +
+                 ((double)v[u].z * v[u].z + (double)v[u].w * v[u].w);
           if (i < nreal4) {
             // c = 4i = a L + j, j a multiple of 4: the four elements share a, and
             // j .. j+3 stay inside the row's column range
