@@ -68,6 +68,11 @@ def _strides(t: torch.Tensor):
     return (ctypes.c_longlong * t.dim())(*t.stride())
 
 
+def _target(t, dims: int):
+    """Pointer and strides of a gradient, or of none."""
+    return (None, (ctypes.c_longlong * dims)()) if t is None else (t.data_ptr(), _strides(t))
+
+
 def _plain(t: torch.Tensor) -> bool:
     """A dense CUDA tensor with memory of its own (not one of a function transform)."""
     if not t.is_cuda or t.layout != torch.strided or t.is_conj() or t.is_neg():
@@ -115,13 +120,12 @@ class PseudoLikelihoodVWFunction(torch.autograd.Function):
                 or grad_out.dtype != g.dtype or g.device.index != torch.cuda.current_device()):
             dV, dW = unpack(grad_out * g, L)  # differentiable, and open to transforms
             return dV if need_v else None, dW if need_w else None, None
-        dV = torch.empty((L, Q - 1), dtype=g.dtype, device=g.device)
-        dW = torch.empty((L, L, Q, Q), dtype=g.dtype, device=g.device)
+        dV = torch.empty((L, Q - 1), dtype=g.dtype, device=g.device) if need_v else None
+        dW = torch.empty((L, L, Q, Q), dtype=g.dtype, device=g.device) if need_w else None
         check(lib().ccm_unpack_gradient(g.data_ptr(), grad_out.data_ptr(), L, g.element_size(),
-                                        dV.data_ptr() if need_v else None, _strides(dV),
-                                        dW.data_ptr() if need_w else None, _strides(dW),
+                                        *_target(dV, 2), *_target(dW, 4),
                                         torch.cuda.current_stream().cuda_stream))
-        return dV if need_v else None, dW if need_w else None, None
+        return dV, dW, None
 
 
 def pseudo_likelihood(V: torch.Tensor, W: torch.Tensor, evaluator: Evaluator) -> torch.Tensor:
