@@ -5,7 +5,8 @@ several alignments of that size run at once.
 The paths differ in how an alignment maps onto the tensor cores:
 
 * ``tc_i8sp``: 256-row x 192-slot forward tiles (9 alignment columns), 2:4-sparse
-  8-bit MMAs; 256 x 256 backward tiles over 192-slot groups;
+  8-bit MMAs; 256 x 256 backward tiles over 21 L + 1 natural slots, those of a poorly
+  filled last wave cut along the rows;
 * ``tc_i8x3``: 256 x 256 dense 8-bit tiles (12 columns per tile);
 * ``tc_bf16x2``: 256 x 256 bf16 tiles, two split terms;
 * ``simt_f32``: no tensor cores (CUDA-core kernels, no tile padding).

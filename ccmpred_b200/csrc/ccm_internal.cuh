@@ -130,7 +130,6 @@ struct I8DigitsArgs {
 
 struct I8PrepArgs {
   int8_t *wdig[3];
-  const uint32_t *colmax;  // per coupling column (a*L + j): max |W| as float bits
   const float *enc;        // per slot: the digit encoding factor 2^(21 - e), 0 for padding
   double *part_reg;
   int L, S;
@@ -272,7 +271,7 @@ cudaError_t i8_build_onehot(ccm_context *c);
 // that its last wave leaves over (1: none), for `tiles` tiles on `pairs` CTA pairs.
 int i8_cut_parts(int tiles, int pairs, int Npad, bool sym);
 constexpr size_t kCutPartBytes = 512 * 1024;  // (hi, lo) of a 256 x 256 tile
-constexpr int kMaxCutTiles = 60;
+constexpr int kMaxCutTiles = 60;  // (half of the CTA pairs at most, 37 of 74)
 constexpr int kCutCounters = 16;  // of a cut tile: two CTAs of eight epilogue warps
 constexpr size_t kResultBytes = (sizeof(ccm_result) + 4 * kCutCounters * kMaxCutTiles + 15) & ~15;
 static_assert(kResultBytes <= 16 * 256);

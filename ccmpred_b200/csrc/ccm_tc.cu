@@ -521,7 +521,7 @@ constexpr int kBwdBufs = 512 / kBwdBN;  // TMEM accumulators of kBwdBN columns
 // (round-to-nearest).  The tensor-core accumulator then never sums more than
 // one chunk, which keeps its rounding error from growing with N.
 constexpr int kBwdChunkKB = 40;
-// warp 0 TMA, warp 1 MMA (leader CTA), warps 2-9 epilogue (two warps per TMEM
+// warp 0 TMA, warp 1 MMA (leader CTA), warps 4-11 epilogue (two warps per TMEM
 // lane quarter, one per half of the 256 columns)
 
 template <int NSPLIT>

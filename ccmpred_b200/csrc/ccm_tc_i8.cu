@@ -1483,7 +1483,7 @@ __device__ __forceinline__ void i8_backward_error(const BwdArgs &args, int *abor
   if (args.fin.host) *reinterpret_cast<volatile int *>(&args.fin.host->status) = kErrBwdTimeout;
 }
 
-// CUT: a last wave of tiles that fills less than half of the pairs is cut along K (the rows):
+// CUT: a last wave of tiles that fills at most half of the pairs is cut along K (the rows):
 // every part is an entry of its own in the tile list, and the epilogue warp that finishes
 // a tile's part last adds the parts' integer sums (exact, so that the gradient is that of
 // the uncut tile bit for bit) and writes the output.
@@ -1493,7 +1493,7 @@ __device__ __forceinline__ void i8_backward_error(const BwdArgs &args, int *abor
 // Bound on the sparse path: the MMAs, 768 cycles of a K block's six (their issue rate is
 // the peak of kind::i8; at L = 1000 the power cap lowers the clock), then the last wave's
 // fill (i8_cut_parts) and, below N = 2000, the output phase of a pair's last tile.
-// L = 300, N = 5000 380 us, L = 253, N = 7001 391, L = 50, N = 200 23.
+// L = 300, N = 5000 375 us, L = 253, N = 7001 374, L = 50, N = 200 23.
 template <bool SYM, bool NAT, bool CUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWgThreads, 1)
     i8_backward_kernel(const __grid_constant__ I8BwdMaps maps, BwdArgs args) {
@@ -1861,7 +1861,6 @@ static cudaError_t i8_prepare_dense(ccm_context *c, const float *d_x, float *g2,
   if (e != cudaSuccess) return e;
   I8PrepArgs pa{};
   for (int i = 0; i < 3; ++i) pa.wdig[i] = c->d_wdig[i];
-  pa.colmax = c->d_colmax;
   pa.enc = enc;
   pa.part_reg = c->d_part_reg;
   pa.L = L; pa.S = c->S; pa.lambda_pair = c->lambda_pair;
@@ -1937,12 +1936,13 @@ static cudaError_t i8_prepare_sparse(ccm_context *c, const float *d_x, float *g2
 // A K block is 768 cycles of MMAs (not symmetric: 384), and cutting a tile in p saves
 // (p - 1) / p of its last wave.  It costs what writing the sums and adding p - 1 of them
 // takes (512 KB per part, L2 to two SMs), measured as 12 k + 6 k p cycles, and 8 k cycles in the
-// next scan, whose L2 these sums occupy.  The measured sides, backward alone: L = 300, 29 of 325
-// tiles left over, p = 2: N = 3000 250 us uncut, 241 cut, N = 5000 396 and 378; L = 253, 9 of
-// 231 tiles, p = 8: N = 2000 149 and 159, N = 3000 199 and 194, N = 7001 445 and 391;
-// L = 150, 17 of 91, p = 4: N = 2000 78 and 89, N = 3500 121 and 108; L = 200, N = 20000,
-// 5 of 153, p = 8: 870 and 710.  Rows beyond one chunk are not cut: their sums leave
-// the integers chunk by chunk.
+// next scan, whose L2 these sums occupy.  The measured sides, backward alone, uncut and
+// cut: L = 300, 29 of 325 tiles left over, p = 2: N = 3000 246 and 239 us, N = 5000 391 and
+// 375; L = 253, 9 of 231 tiles: N = 3000, p = 4 200 and 188, N = 7001, p = 5 417 and 374
+// (N = 2000 149, and 159 in eight parts: left whole); L = 150, 17 of 91, p = 4: N = 3500 122
+// and 108 (N = 2000 78 and 89: left whole); L = 200, N = 20000, 5 of 153, p = 8: 843 and
+// 698.  More than half as many tiles as pairs are never cut: a part each is a pair each.
+// Rows beyond one chunk are not cut: their sums leave the integers chunk by chunk.
 int i8_cut_parts(int tiles, int pairs, int Npad, bool sym) {
   const int k_blocks = Npad / kI8BwdBK, rest = tiles % pairs;
   if (rest == 0 || rest > kMaxCutTiles || k_blocks > kI8BwdChunkKB) return 1;
