@@ -109,6 +109,8 @@ class PseudoLikelihoodVWFunction(torch.autograd.Function):
         f = evaluator.evaluate(x, g)
         ctx.save_for_backward(g)
         ctx.L = evaluator.L
+        if V.dtype == torch.float32:
+            f = ctypes.c_float(f).value  # infinite past its range, where full() would raise
         return torch.full((), f, dtype=V.dtype, device=V.device)
 
     @staticmethod
