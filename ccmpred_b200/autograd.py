@@ -118,7 +118,9 @@ class PseudoLikelihoodVWFunction(torch.autograd.Function):
         (g,) = ctx.saved_tensors
         L = ctx.L
         need_v, need_w, _ = ctx.needs_input_grad
+        # (g may have been through saved-tensor hooks)
         if (torch.is_grad_enabled() or not _plain(grad_out) or not _plain(g)
+                or not g.is_contiguous() or g.shape != (nvar_padded(L),)
                 or grad_out.dtype != g.dtype or g.device.index != torch.cuda.current_device()):
             dV, dW = unpack(grad_out * g, L)  # differentiable, and open to transforms
             return dV if need_v else None, dW if need_w else None, None
