@@ -1003,10 +1003,11 @@ int ccm_evaluate_host(ccm_context *c, const float *x, float *g, long long nvar, 
   if (nvar != c->nvarp)
     return set_error(CCM_ERR_INVALID, "ccm_evaluate_host: nvar %lld != nvar_padded %lld", nvar, c->nvarp);
   const size_t bytes = sizeof(float) * (size_t)nvar;
-  if (!c->d_xh) {
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_xh, bytes));
-    CCM_CUDA_TRY(dev_alloc(c, &c->d_gh, bytes));
+  if (!c->d_gh) {
+    // both or neither: what a failed call leaves is taken up by the next one
+    if (!c->d_xh) CCM_CUDA_TRY(dev_alloc(c, &c->d_xh, bytes));
     CCM_CUDA_TRY(cudaMemsetAsync(c->d_xh, 0, bytes, c->stream));
+    CCM_CUDA_TRY(dev_alloc(c, &c->d_gh, bytes));
     c->xh_pad_dirty = false;
   }
   const int L = c->L;
