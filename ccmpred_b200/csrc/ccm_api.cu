@@ -112,14 +112,15 @@ size_t pool_unused(int device) {
 
 cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t stream) {
   cudaMemPool_t pool = library_pool(device);
-  if (!pool) return cudaMallocAsync(p, bytes, stream);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
-  if (e == cudaErrorMemoryAllocation) {
+  cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream)
+                       : cudaMallocAsync(p, bytes, stream);
+  if (pool && e == cudaErrorMemoryAllocation) {
     // kept blocks of other sizes may stand in the way
-    (void)cudaGetLastError();
     cudaMemPoolTrimTo(pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
   }
+  // reported by the status alone: a failed allocation must not surface in a later launch check
+  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
   return e;
 }
 
